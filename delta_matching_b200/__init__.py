@@ -18,6 +18,7 @@ import os as _os
 
 import torch
 
+from . import _lib
 from .attn import blocks, dm_attn_func_bhnd, dm_attn_debug
 
 __version__ = "0.1.0"
@@ -42,6 +43,10 @@ def dm_attn_func(q, k, v, softmax_scale=None, causal=False, mode="matched", nume
     numerics: "sm100-mx" (the contract; "sm100-mx-d256" names it at head_dim 256) or another arm of the reference
     emulation's preset table that the kernels implement: "sm100-mx-ds32" / "sm100-mx-d256-ds32" (dS scaled per
     32 x 32 block) and "sm100-mx-nonorm" (matched delta without the division by sum P); see NUMERICS_ARMS."""
+    if not torch.compiler.is_compiling():
+        o = (_lib._NATIVE or _lib.native_attn())(q, k, v, softmax_scale, causal, mode, numerics, False)
+        if o is not None:
+            return o
     for name, t in (("q", q), ("k", k), ("v", v)):
         if not isinstance(t, torch.Tensor) or t.dim() != 4:
             raise ValueError(f"delta_matching: {name} must be a 4-D tensor (batch, seqlen, nheads, headdim)")

@@ -42,6 +42,10 @@ SIGNATURES = {
     "dm_bwd_workspace_bytes": (_L, [_I, _I, _I, _I]),
     "dm_bwd_ws": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                        _P, _L, _L, _L, _P, _L, _L, _L, _P, _L, _L, _L, _P, _L, _I, _P, _P]),
+    "dm_attn_fwd": (_I, [_P, _L, _L, _L, _P, _L, _L, _L, _P, _L, _L, _L, _I, _I, _I, _I, _I, _I,
+                         _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "dm_attn_bwd": (_I, [_P, _L, _L, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
+                         _P, _P, _P, _P, _L, _I, _P, _P]),
     "dm_dbg_mma_tile": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P]),
     "dm_dbg_wait_expiry": (_I, [_P, _P, _P, ctypes.c_longlong, _P, _P]),
     "dm_launch_count": (ctypes.c_longlong, []),
@@ -100,3 +104,37 @@ def check(rc: int) -> None:
     reference, csrc/delta_matching_api.cpp:73-98 via TORCH_CHECK)."""
     if rc != 0:
         raise RuntimeError(last_error() or f"delta_matching_b200: library call failed with code {rc}")
+
+
+_NATIVE = None
+
+
+def native_attn():
+    """The native eager route (csrc/dm_torch.cpp): attn(q, k, v, softmax_scale, causal, mode, numerics, head_major) -> o, or
+    None when the Python route has to take the call.  Bound once to the entry points of lib() and to the op layer's status
+    word and workspace plan.  Like the kernel library it has no substitute: a GPU machine without it raises."""
+    global _NATIVE
+    if _NATIVE is None:
+        from . import ops
+        import torch
+        if ops._DEBUG or not torch.cuda.is_available():        # DM_DEBUG checks behind every op; no GPU, no CUDA tensors
+            return _decline
+        L = lib()
+        with _LOCK:
+            if _NATIVE is None:
+                try:
+                    from . import _dm_native
+                except ImportError as e:
+                    raise RuntimeError("delta_matching_b200: _dm_native.so is not built or does not load: run `python -m "
+                                       f"delta_matching_b200.build` in the checkout ({e})") from e
+                addr = lambda name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value
+                _dm_native.bind(addr("dm_attn_fwd"), addr("dm_attn_bwd"), addr("dm_last_error"), addr("dm_bwd_workspace_bytes"),
+                                addr("dm_quant_qkv_workspace_bytes"),
+                                lambda idx: ops.status_word(torch.device("cuda", idx)).data_ptr(), ops._raise_if_set,
+                                lambda *a: ops.bwd_fp8(*a[:11], ds32=a[11]), ops._SMALL_WS, ops._MAX_WS_TILES)
+                _NATIVE = _dm_native.attn
+    return _NATIVE
+
+
+def _decline(*_):
+    return None

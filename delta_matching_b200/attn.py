@@ -1,5 +1,9 @@
 """The autograd route and the input contract.
 
+Eager calls on plain CUDA tensors run in C++ (csrc/dm_torch.cpp: the same checks, the same kernels, one call of the C ABI per
+pass): at short sequences the host time of the Python route below is several times the kernels' own.  The Python route
+serves tracing compilers, tensor subclasses and function transforms, and raises the contract's exceptions.
+
 `dm_attn_func_bhnd(q, k, v, causal, softmax_scale, delta_mode)` on (B, H, N, D) inputs returns (B, N, H, D), as
 delta_matching/attn.py:121-127 does.  Forward: producers (codes, scales, K mean) then the forward kernel.  Backward: the
 dO producer (with the stale delta rowsum(dO * O) when delta_mode == "stale"), the matched delta from pass 0 of the
@@ -11,7 +15,7 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from . import torch_ops as _torch_ops  # noqa: F401  (registers torch.ops.delta_matching_b200.*)
 
 _OPS = torch.ops.delta_matching_b200
@@ -84,7 +88,7 @@ def _is_sm100(index: int) -> bool:
 class _DMAttn(torch.autograd.Function):
     """Forward and backward as calls of the registered ops (delta_matching_b200/torch_ops.py), the way the reference's
     autograd function calls torch.ops.delta_matching (delta_matching/attn.py:37-118): a tracing compiler records five
-    opaque ops instead of breaking its graph here; eager calls skip the dispatcher and run the same functions directly."""
+    opaque ops instead of breaking its graph here; other calls skip the dispatcher and run the same functions directly."""
 
     @staticmethod
     def forward(ctx, q, k, v, causal, delta_mode, ds32, norm):
@@ -130,6 +134,10 @@ def dm_attn_func_bhnd(q, k, v, causal=True, softmax_scale=None, delta_mode="stal
     torch.compile without a graph break (the kernels are registered ops with fake implementations) and under CUDA-graph
     capture after a warm-up call.  numerics: the reference's Blackwell contract "sm100-mx" or one of the arms of
     ops.NUMERICS (the same forward; the backward's dS block or the matched delta's normalisation differ)."""
+    if not torch.compiler.is_compiling():
+        o = (_lib._NATIVE or _lib.native_attn())(q, k, v, softmax_scale, causal, delta_mode, numerics, True)
+        if o is not None:
+            return o
     _check_inputs(q, k, v, causal, softmax_scale, delta_mode)
     ds32, norm = _numerics(numerics, q.shape[-1])
     return _DMAttn.apply(q, k, v, causal, delta_mode, ds32, norm)

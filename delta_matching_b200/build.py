@@ -1,4 +1,5 @@
-"""Build the CUDA library in-tree: nvcc for sm_100a only, one shared object `libdm_b200.so` next to this file.
+"""Build the CUDA library in-tree: nvcc for sm_100a only, one shared object `libdm_b200.so` next to this file, and the
+Python extension `_dm_native.so` (csrc/dm_torch.cpp: the eager route of the attention functions against torch's C++ API).
 
     python -m delta_matching_b200.build [--force] [--verbose]
 
@@ -18,6 +19,8 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libdm_b200.so")
 SOURCES = ("dm_abi.cu", "dm_quant.cu", "dm_fwd.cu", "dm_delta.cu", "dm_bwd.cu", "dm_bwd_p2.cu", "dm_probe.cu", "dm_static_scratch.cu")
+NATIVE = os.path.join(HERE, "_dm_native.so")
+NATIVE_SOURCE = "dm_torch.cpp"
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
@@ -31,7 +34,7 @@ def _nvcc() -> str:
 def source_files():
     out = []
     for f in sorted(os.listdir(CSRC)):
-        if f.endswith((".cu", ".cuh", ".h")):
+        if f.endswith((".cu", ".cuh", ".h", ".cpp")):
             out.append(os.path.join(CSRC, f))
     out.append(os.path.join(os.path.dirname(HERE), "include", "dm_b200.h"))
     return out
@@ -47,6 +50,24 @@ def code_sha() -> str:
     return h.hexdigest()[:12]
 
 
+def _build_native(verbose: bool) -> None:
+    """g++ against the installed torch's headers; the module finds torch's libraries already loaded (it is imported behind
+    torch) and takes the kernel library's entry points as addresses, so it links neither by path."""
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    inc = [f for d in (*cpp_extension.include_paths(), sysconfig.get_path("include"), "/usr/local/cuda/include") for f in ("-isystem", d)]
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, os.path.join(CSRC, NATIVE_SOURCE), "-o", NATIVE,
+           f"-L{lib_dir}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {NATIVE_SOURCE}:\n{r.stdout}\n{r.stderr[-6000:]}")
+    if verbose:
+        sys.stderr.write(r.stderr)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile and link (skipped when the library is newer than a stamp of the sources' hash)."""
     obj_dir = OBJ
@@ -54,7 +75,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(obj_dir, exist_ok=True)
     stamp = os.path.join(obj_dir, "stamp.txt")
     sha = code_sha()
-    if not force and os.path.isfile(lib) and os.path.isfile(stamp) and open(stamp).read().strip() == sha:
+    if not force and os.path.isfile(lib) and os.path.isfile(NATIVE) and os.path.isfile(stamp) and open(stamp).read().strip() == sha:
         return lib
     srcs = list(SOURCES)
     nvcc = _nvcc()
@@ -73,8 +94,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        native = ex.submit(_build_native, verbose)
         objs = list(ex.map(compile_one, srcs))
+        native.result()
     r = subprocess.run([nvcc, "-shared", "-o", lib, *objs, "-lcudart"], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")

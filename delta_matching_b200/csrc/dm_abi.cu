@@ -153,7 +153,25 @@ int dm_kmean(const void* k, int64_t k_sb, int64_t k_sh, int64_t k_sn, int B, int
   return e == cudaSuccess ? 0 : cuda_fail(e, "k-mean launch");
 }
 
-// checks the arguments of one quantiser call and fills its parameter block
+// parameter block of one quantiser call
+static dm::QuantParams make_quant(const void* x, int64_t x_sb, int64_t x_sh, int64_t x_sn, const float* mean, float prescale,
+                                  const void* o, int64_t o_sb, int64_t o_sh, int64_t o_sn, int B, int N, int H, int D,
+                                  void* codes, float* scales, float* delta) {
+  dm::QuantParams p{};
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.sb = x_sb; p.sh = x_sh; p.sn = x_sn;
+  p.mean = mean;
+  p.o = static_cast<const __nv_bfloat16*>(o);
+  p.o_sb = o_sb; p.o_sh = o_sh; p.o_sn = o_sn;
+  p.prescale = prescale;
+  p.codes = static_cast<uint8_t*>(codes);
+  p.scales = scales;
+  p.delta = (o != nullptr) ? delta : nullptr;
+  p.B = B; p.H = H; p.N = N; p.D = D;
+  return p;
+}
+
+// the same behind the checks of its arguments
 static int quant_params(dm::QuantParams& p, const void* x, int64_t x_sb, int64_t x_sh, int64_t x_sn, const float* mean,
                         float prescale, const void* o, int64_t o_sb, int64_t o_sh, int64_t o_sn, int B, int N, int H, int D,
                         void* codes, float* scales, float* delta) {
@@ -168,17 +186,7 @@ static int quant_params(dm::QuantParams& p, const void* x, int64_t x_sb, int64_t
     DM_TRY(check_device_ptr(delta, "delta"));
     DM_TRY(check_strides("o", o_sb, o_sh, o_sn));
   }
-  p = dm::QuantParams{};
-  p.x = static_cast<const __nv_bfloat16*>(x);
-  p.sb = x_sb; p.sh = x_sh; p.sn = x_sn;
-  p.mean = mean;
-  p.o = static_cast<const __nv_bfloat16*>(o);
-  p.o_sb = o_sb; p.o_sh = o_sh; p.o_sn = o_sn;
-  p.prescale = prescale;
-  p.codes = static_cast<uint8_t*>(codes);
-  p.scales = scales;
-  p.delta = (o != nullptr) ? delta : nullptr;
-  p.B = B; p.H = H; p.N = N; p.D = D;
+  p = make_quant(x, x_sb, x_sh, x_sn, mean, prescale, o, o_sb, o_sh, o_sn, B, N, H, D, codes, scales, delta);
   return 0;
 }
 
@@ -216,6 +224,87 @@ int dm_quant_do(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn,
                 const void* o, int64_t o_sb, int64_t o_sh, int64_t o_sn,
                 int B, int N, int H, int D, void* do8, float* dos, float* delta, void* stream) {
   return dm_quant_rows(d_o, do_sb, do_sh, do_sn, nullptr, 1.0f, o, o_sb, o_sh, o_sn, B, N, H, D, do8, dos, delta, stream);
+}
+
+// ------------------------------------------------------------------------------------------------ whole passes
+// dm_attn_fwd / dm_attn_bwd launch what a forward or a backward of the attention layer needs in one call.  The separate
+// entry points above and below look every pointer up in the driver (cudaPointerGetAttributes, some 0.3 us each, about
+// forty of them in a training step) and encode the tensor maps once per kernel; here the caller vouches for its buffers and
+// every map is encoded once per pass.
+int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
+                const void* k, int64_t k_sb, int64_t k_sh, int64_t k_sn,
+                const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                int B, int N, int H, int Hk, int D, int causal,
+                void* q8, void* k8, void* v8, float* qs, float* ks, float* vs, float* kmean, void* workspace,
+                void* o, float* lse, int* status, void* stream) {
+  DM_TRY(check_shape(B, N, H, Hk, D));
+  DM_TRY(check_sm100());
+  DM_TRY(check_strides("q", q_sb, q_sh, q_sn));
+  DM_TRY(check_strides("k", k_sb, k_sh, k_sn));
+  DM_TRY(check_strides("v", v_sb, v_sh, v_sn));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const float sm = static_cast<float>(1.0 / sqrt(static_cast<double>(D)));
+  const dm::QuantParams pq = make_quant(q, q_sb, q_sh, q_sn, nullptr, sm, nullptr, 0, 0, 0, B, N, H, D, q8, qs, nullptr);
+  const dm::QuantParams pk = make_quant(k, k_sb, k_sh, k_sn, kmean, 1.0f, nullptr, 0, 0, 0, B, N, Hk, D, k8, ks, nullptr);
+  const dm::QuantParams pv = make_quant(v, v_sb, v_sh, v_sn, nullptr, 1.0f, nullptr, 0, 0, 0, B, N, Hk, D, v8, vs, nullptr);
+  const dm::KMeanParams pm{static_cast<const __nv_bfloat16*>(k), k_sb, k_sh, k_sn, static_cast<float*>(workspace), kmean, B, Hk, N, D};
+  cudaError_t e = dm::launch_quant_qkv(pq, pk, pv, pm, st);
+  if (e != cudaSuccess) return cuda_fail(e, "producer launch");
+  CUtensorMap tq, tk, tv;
+  DM_TRY(make_code_map(&tq, q8, static_cast<uint64_t>(B) * H * N, D));
+  DM_TRY(make_code_map(&tk, k8, static_cast<uint64_t>(B) * Hk * N, D));
+  DM_TRY(make_code_map(&tv, v8, static_cast<uint64_t>(B) * Hk * N, D));
+  const dm::FwdParams p{qs, ks, vs, static_cast<__nv_bfloat16*>(o), static_cast<int64_t>(N) * H * D, static_cast<int64_t>(H) * D, D,
+                        lse, B, H, Hk, N, causal ? 1 : 0, status, 0};
+  e = dm::launch_fwd(D, tq, tk, tv, p, st);
+  return e == cudaSuccess ? 0 : cuda_fail(e, "forward launch");
+}
+
+int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, const void* o,
+                const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
+                const float* lse, void* do8, float* dos, float* delta, int B, int N, int H, int Hk, int D, int causal,
+                void* dq, void* dk, void* dv, void* workspace, int64_t workspace_bytes, int flags, int* status, void* stream) {
+  DM_TRY(check_shape(B, N, H, Hk, D));
+  DM_TRY(check_sm100());
+  DM_TRY(check_strides("d_o", do_sb, do_sh, do_sn));
+  const bool kernels = (flags & DM_ATTN_DELTA_ONLY) == 0;
+  const int64_t need = dm_bwd_workspace_bytes(B, N, H, D);
+  const uint64_t tiles = static_cast<uint64_t>(B) * H * (N / 128) * (N / 128);
+  if (kernels && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
+    return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed (16-byte aligned)", (long long)workspace_bytes, (long long)need);
+  if (kernels && tiles * 128 >= (1ull << 31))
+    return fail(DM_ERR_ARG, "delta_matching: B * H * (N / 128)^2 = %llu tiles exceed one workspace (split the heads)", (unsigned long long)tiles);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int64_t hd = static_cast<int64_t>(H) * D, kd = static_cast<int64_t>(Hk) * D;
+  const dm::QuantParams pd = make_quant(d_o, do_sb, do_sh, do_sn, nullptr, 1.0f, o, N * hd, D, hd, B, N, H, D, do8, dos, delta);
+  cudaError_t e = dm::launch_quant(pd, st);
+  if (e != cudaSuccess) return cuda_fail(e, "quantiser launch");
+  CUtensorMap tq, tk, tv, td, tds;
+  DM_TRY(make_code_map(&tq, q8, static_cast<uint64_t>(B) * H * N, D));
+  DM_TRY(make_code_map(&tk, k8, static_cast<uint64_t>(B) * Hk * N, D));
+  DM_TRY(make_code_map(&tv, v8, static_cast<uint64_t>(B) * Hk * N, D));
+  DM_TRY(make_code_map(&td, do8, static_cast<uint64_t>(B) * H * N, D));
+  if (o == nullptr) {
+    const dm::DeltaParams p{qs, ks, vs, dos, lse, delta, B, H, Hk, N, causal ? 1 : 0, status, (flags & DM_ATTN_DELTA_SUM) ? 0 : 1};
+    e = dm::launch_delta(D, tq, tk, tv, td, p, st);
+    if (e != cudaSuccess) return cuda_fail(e, "matched-delta launch");
+  }
+  if (!kernels) return 0;
+  dm::BwdParams p{};
+  p.qs = qs; p.ks = ks; p.vs = vs; p.dos = dos; p.lse = lse; p.delta = delta;
+  p.dq = static_cast<__nv_bfloat16*>(dq); p.dq_sb = N * hd; p.dq_sn = hd; p.dq_sh = D;
+  p.dk = static_cast<__nv_bfloat16*>(dk); p.dk_sb = N * kd; p.dk_sn = kd; p.dk_sh = D;
+  p.dv = static_cast<__nv_bfloat16*>(dv); p.dv_sb = N * kd; p.dv_sn = kd; p.dv_sh = D;
+  p.sm_scale = static_cast<float>(1.0 / sqrt(static_cast<double>(D)));
+  p.B = B; p.H = H; p.Hk = Hk; p.N = N; p.causal = causal ? 1 : 0; p.status = status;
+  p.ds32 = (flags & DM_DS_BLOCK32) ? 1 : 0;
+  p.ds_codes = static_cast<uint8_t*>(workspace);
+  p.ds_words = p.ds_codes + tiles * 16384;
+  DM_TRY(make_code_map(&tds, workspace, tiles * 128, 128));
+  e = dm::launch_bwd_dkdv(D, tq, tk, tv, td, &tds, p, st);
+  if (e != cudaSuccess) return cuda_fail(e, "backward dK/dV launch");
+  e = dm::launch_bwd_dq_p2(D, tds, tk, p, st);
+  return e == cudaSuccess ? 0 : cuda_fail(e, "backward dQ launch");
 }
 
 static int fwd_impl(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,

@@ -155,6 +155,30 @@ int dm_bwd_ws(const void* q8, const void* k8, const void* v8, const void* do8,
               void* dv, int64_t dv_sb, int64_t dv_sn, int64_t dv_sh,
               void* workspace, int64_t workspace_bytes, int parts, int* status, void* stream);
 
+/* Whole passes: everything a forward, or a backward, of the attention layer launches, in one call (what the native PyTorch
+ * path uses).  The kernels and their results are those of the separate entry points.  The caller vouches for the
+ * pointers (device memory of the current device, 16-byte aligned): only shapes and strides are checked here.
+ *
+ * dm_attn_fwd = dm_quant_qkv, dm_fwd.  q, k, v by element strides for (batch, head, token); o is contiguous (B, N, H, D).
+ * kmean (B, Hk, D) fp32 and workspace (dm_quant_qkv_workspace_bytes) are scratch. */
+int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
+                const void* k, int64_t k_sb, int64_t k_sh, int64_t k_sn,
+                const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                int B, int N, int H, int Hk, int D, int causal,
+                void* q8, void* k8, void* v8, float* qs, float* ks, float* vs, float* kmean, void* workspace,
+                void* o, float* lse, int* status, void* stream);
+
+/* dm_attn_bwd = dm_quant_do, dm_delta, dm_bwd_ws with parts = 3.  o == NULL: the matched delta (dm_delta, or dm_delta_sum with
+ * DM_ATTN_DELTA_SUM); o = the forward's contiguous (B, N, H, D) output: the stale delta.  do8, dos, delta are filled here;
+ * dq, dk, dv are contiguous token-major.  flags: DM_DS_BLOCK32, DM_ATTN_DELTA_SUM, DM_ATTN_DELTA_ONLY (stop behind
+ * do8, dos and delta: for callers that split the rest over several dm_bwd_ws calls; dq, dk, dv and workspace are unused). */
+#define DM_ATTN_DELTA_SUM 8
+#define DM_ATTN_DELTA_ONLY 16
+int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, const void* o,
+                const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
+                const float* lse, void* do8, float* dos, float* delta, int B, int N, int H, int Hk, int D, int causal,
+                void* dq, void* dk, void* dv, void* workspace, int64_t workspace_bytes, int flags, int* status, void* stream);
+
 /* One 128 x 128 x (32 * nk) e4m3 tile product through the operand paths the kernels use (unit-test hook; the
  * reference has per-kernel debug ops instead, csrc/delta_matching_api.cpp:611-661).  a, b: 128 x 128 e4m3 row-major
  * device buffers; sfa / sfb: 128 x 4 uint32 scale words (block-scaled runs only); out: 128 x 128 fp32. */
