@@ -49,6 +49,12 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
   lo = __fadd_rn(lo, err);
 }
 
+// Maximum over the warp of a non-negative value: non-negative floats order like their bit patterns, so one integer
+// redux.sync does the work of a five-step shuffle butterfly.
+__device__ __forceinline__ float warp_max(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
 // ---------------------------------------------------------------------------------------------- persistent schedule
 // Work items are numbered heaviest first.  Round k hands items k * n_ctas ... k * n_ctas + n_ctas - 1 to the CTAs in
 // ascending CTA order when k is even and in descending order when k is odd, so that the totals of the CTAs stay close to
