@@ -110,6 +110,7 @@ bwd_dq_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dep_wait();
 
   if (warp == 4) {
     if (elect_one()) {
@@ -387,6 +388,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dep_wait();
 
   if (warp == 16) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -634,9 +636,8 @@ static cudaError_t launch_dq_serial_t(const CUtensorMap& tq, const CUtensorMap& 
   cudaError_t e = set_smem(bwd_dq_serial_kernel<D>, C::kSmemBytes, done);
   if (e != cudaSuccess) return e;
   dim3 grid(p.N / 128, p.B * p.H);
-  bwd_dq_serial_kernel<D><<<grid, 192, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(bwd_dq_serial_kernel<D>, grid, 192, C::kSmemBytes, stream, tq, tk, tv, tdo, p);
 }
 
 cudaError_t launch_bwd_dq(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
@@ -651,9 +652,8 @@ cudaError_t launch_bwd_dq(int D, const CUtensorMap& tq, const CUtensorMap& tk, c
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int n_items = (p.N / 128) * p.B * p.H;
-  bwd_dq_kernel<<<n_items < sms ? n_items : sms, DqCfg::kThreads, DqCfg::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(bwd_dq_kernel, n_items < sms ? n_items : sms, DqCfg::kThreads, DqCfg::kSmemBytes, stream, tq, tk, tv, tdo, p);
 }
 
 }  // namespace dm

@@ -137,6 +137,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   constexpr uint32_t tmem = 0;                         // 512 columns are all there are: the allocation starts at column 0
+  grid_dep_wait();
 
   if (warp == C::kComputeWarps + 1) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -510,9 +511,8 @@ static cudaError_t launch_kv_t(const CUtensorMap& tq, const CUtensorMap& tk, con
     done[dev] = true;
   }
   dim3 grid(p.B * p.Hk, p.N / 128);
-  bwd_dkdv_kernel<D, DV, DK, DS32, G><<<grid, C::kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, tds, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(bwd_dkdv_kernel<D, DV, DK, DS32, G>, grid, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
 }
 
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,

@@ -89,6 +89,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dep_wait();
 
   if (warp == 8) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -277,9 +278,8 @@ static cudaError_t launch_p2_t(const CUtensorMap& tds, const CUtensorMap& tk, co
   }
   const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
   const int items = (p.N / 128) * p.B * p.H;
-  bwd_dq_p2_kernel<D><<<items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream>>>(tds, tk, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(bwd_dq_p2_kernel<D>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, p);
 }
 
 cudaError_t launch_bwd_dq_p2(int D, const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream) {

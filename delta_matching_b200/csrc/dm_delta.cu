@@ -103,6 +103,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dep_wait();
 
   if (warp == 16) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -313,9 +314,8 @@ static cudaError_t launch_delta_t(const CUtensorMap& tq, const CUtensorMap& tk, 
   }
   const int n_items = (p.N / 128) * p.B * p.H;
   const int ctas = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
-  delta_kernel<D><<<n_items < ctas ? n_items : ctas, C::kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(delta_kernel<D>, n_items < ctas ? n_items : ctas, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, p);
 }
 
 cudaError_t launch_delta(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,

@@ -112,6 +112,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dep_wait();
   // Barrier and phase of running tile g.  With two S buffers the S / P / PV barriers exist once per buffer and tile g is
   // phase g / 2 of its buffer's barrier: a waiter is then never more than one phase away from the barrier it tests (with
   // one barrier for both buffers the softmax warps, which run a tile ahead of the PV chains, could test the phase bit of
@@ -414,9 +415,8 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
   const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
   const int items = (p.N / 128) * p.B * p.H;
   const int ctas = sms * ((D == 128) ? 2 : 1);              // co-resident CTAs: 256 of the 512 TMEM columns each at D = 128
-  fwd_kernel<D, kOrdered><<<items < ctas ? items : ctas, 192, C::kSmemBytes, stream>>>(tq, tk, tv, p);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(fwd_kernel<D, kOrdered>, items < ctas ? items : ctas, 192, C::kSmemBytes, stream, tq, tk, tv, p);
 }
 
 

@@ -60,11 +60,13 @@ __device__ __forceinline__ void kmean_block(const KMeanParams& p, int chunk, int
 template <int D>
 __global__ void __launch_bounds__(128) kmean_partial_kernel(const KMeanParams p) {
   __shared__ float red[KMeanTile<D>::kRpp][D];
+  grid_dep_wait();
   kmean_block<D>(p, blockIdx.x, blockIdx.y, red);
 }
 
 // Stage 2: one CTA per (batch, kv head): serial fold of the chunk sums in chunk order, divided by N.
 __global__ void kmean_fold_kernel(const KMeanParams p) {
+  grid_dep_wait();
   const int bh = blockIdx.x;
   const int nchunk = p.N / 64;
   for (int c = threadIdx.x; c < p.D; c += blockDim.x) {
@@ -85,11 +87,10 @@ __global__ void kmean_fold_kernel(const KMeanParams p) {
 
 cudaError_t launch_kmean(const KMeanParams& p, cudaStream_t stream) {
   dim3 grid(p.N / 64, p.B * p.Hk);
-  if (p.D == 128) kmean_partial_kernel<128><<<grid, 128, 0, stream>>>(p);
-  else kmean_partial_kernel<256><<<grid, 128, 0, stream>>>(p);
-  kmean_fold_kernel<<<p.B * p.Hk, 128, 0, stream>>>(p);
+  cudaError_t e = launch_chained(p.D == 128 ? kmean_partial_kernel<128> : kmean_partial_kernel<256>, grid, 128, 0, stream, p);
+  if (e == cudaSuccess) e = launch_chained(kmean_fold_kernel, p.B * p.Hk, 128, 0, stream, p);
   count_launch(2);
-  return cudaGetLastError();
+  return e;
 }
 
 // ------------------------------------------------------------------------------------------------ quantiser
@@ -171,6 +172,7 @@ __device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int b
 template <int D, bool kMean, bool kStale>
 __global__ void __launch_bounds__(128) quant_kernel(const QuantParams p) {
   __shared__ float wmax[4];
+  grid_dep_wait();
   quant_block<D, kMean, kStale>(p, blockIdx.x, blockIdx.y, wmax);
 }
 
@@ -181,6 +183,7 @@ template <int D>
 __global__ void __launch_bounds__(128) quant_qv_kmean_kernel(const QuantParams pq, const QuantParams pv, const KMeanParams pk) {
   __shared__ float wmax[4];
   __shared__ float red[KMeanTile<D>::kRpp][D];
+  grid_dep_wait();
   const int n_km = (pk.N / 64) * pk.B * pk.Hk;
   const int n_q = (pq.N / 32) * pq.B * pq.H;
   int i = static_cast<int>(blockIdx.x);
@@ -199,11 +202,10 @@ cudaError_t launch_quant_qkv(const QuantParams& pq, const QuantParams& pk, const
   const long long blocks = static_cast<long long>(pm.N / 64) * pm.B * pm.Hk + static_cast<long long>(pq.N / 32) * pq.B * pq.H +
                            static_cast<long long>(pv.N / 32) * pv.B * pv.H;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
-  if (pq.D == 128) quant_qv_kmean_kernel<128><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(pq, pv, pm);
-  else quant_qv_kmean_kernel<256><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(pq, pv, pm);
-  kmean_fold_kernel<<<pm.B * pm.Hk, 128, 0, stream>>>(pm);
+  cudaError_t e = launch_chained(pq.D == 128 ? quant_qv_kmean_kernel<128> : quant_qv_kmean_kernel<256>, static_cast<unsigned>(blocks), 128,
+                                 0, stream, pq, pv, pm);
+  if (e == cudaSuccess) e = launch_chained(kmean_fold_kernel, pm.B * pm.Hk, 128, 0, stream, pm);
   count_launch(2);
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_quant(pk, stream);                      // K, centred by the mean that the fold has just written
 }
@@ -211,17 +213,10 @@ cudaError_t launch_quant_qkv(const QuantParams& pq, const QuantParams& pk, const
 cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream) {
   dim3 grid(p.N / 32, p.B * p.H);
   const bool mean = p.mean != nullptr, stale = p.o != nullptr;
-  if (p.D == 128) {
-    if (stale) quant_kernel<128, false, true><<<grid, 128, 0, stream>>>(p);
-    else if (mean) quant_kernel<128, true, false><<<grid, 128, 0, stream>>>(p);
-    else quant_kernel<128, false, false><<<grid, 128, 0, stream>>>(p);
-  } else {
-    if (stale) quant_kernel<256, false, true><<<grid, 128, 0, stream>>>(p);
-    else if (mean) quant_kernel<256, true, false><<<grid, 128, 0, stream>>>(p);
-    else quant_kernel<256, false, false><<<grid, 128, 0, stream>>>(p);
-  }
+  auto* kernel = p.D == 128 ? (stale ? quant_kernel<128, false, true> : mean ? quant_kernel<128, true, false> : quant_kernel<128, false, false>)
+                            : (stale ? quant_kernel<256, false, true> : mean ? quant_kernel<256, true, false> : quant_kernel<256, false, false>);
   count_launch();
-  return cudaGetLastError();
+  return launch_chained(kernel, grid, 128, 0, stream, p);
 }
 
 }  // namespace dm
