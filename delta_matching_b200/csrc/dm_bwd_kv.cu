@@ -29,12 +29,12 @@ namespace dm {
 // With sixteen warps on 32 queries each and one 128-column region that S^T and dP^T shared (what this kernel did before), every
 // link of the chain was exposed and the fixed work of a warp per tile was done sixteen times.
 //
-// Head_dim 256: one accumulator fills 256 columns, so the kernel runs twice: a DV launch (S^T, P^T codes, dV; the columns of dP^T
-// are a second S^T buffer, and the words lie beside the codes) and a DK launch (S^T, dP^T, dS codes, dK and the dS tiles for
+// Head_dim 256: one accumulator fills 256 columns, so a key tile is two CTAs: a DV role (S^T, P^T codes, dV; the columns of dP^T
+// are a second S^T buffer, and the words lie beside the codes) and a DK role (S^T, dP^T, dS codes, dK and the dS tiles for
 // the workspace), each with the other half of the work compiled out.
 template <int D, bool DV, bool DK, int G>
 struct KvCfg {
-  static_assert(D == 128 ? (DV && DK) : (D == 256 && DV != DK), "128: both accumulators; 256: one per launch");
+  static_assert(D == 128 ? (DV && DK) : (D == 256 && DV != DK), "128: both accumulators; 256: one per role");
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
   static constexpr int kCodeBytes = 128 * 128;         // dS^T code tile (does not depend on head_dim)
@@ -50,7 +50,7 @@ struct KvCfg {
   static constexpr int kColOne = 8 * kCh + 8;         // 4 columns of 0x7F7F7F7F (written by h = 0)
   static constexpr int kColDv = 256, kColDk = (D == 128) ? 384 : 256;
   static constexpr int kSmemK = 0;
-  static constexpr int kSmemV = kTileBytes;                          // a DV launch has no V tile
+  static constexpr int kSmemV = kTileBytes;                          // the DV role has no V tile
   static constexpr int kSmemQ = DK ? 2 * kTileBytes : kTileBytes;    // [kStages]
   static constexpr int kSmemDo = kSmemQ + kStages * kTileBytes;      // [kStages]
   static constexpr int kSmemWs = kSmemDo + kStages * kTileBytes;     // two staging tiles of dS^T codes
@@ -80,17 +80,15 @@ __device__ __forceinline__ void store_bf16_row32(const uint32_t (&r)[32], __nv_b
 // DS32: the dS scale is taken per (32 queries x 32 keys), which is one 32-column block of one warp, instead of the contract's
 // (128 queries x 32 keys), for which the two warps of a key quadrant exchange their maxima.
 template <int D, bool DV, bool DK, bool DS32, int G>
-__global__ void __launch_bounds__(KvCfg<D, DV, DK, G>::kThreads, 1)
-bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
+__device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
+                                          const CUtensorMap& tm_do, const CUtensorMap& tm_ds, const BwdParams& p) {
   using C = KvCfg<D, DV, DK, G>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemBar);
   uint64_t* bar_kv = bars + 0;       // K and V landed
-  uint64_t* bar_s = bars + 1;        // [2] S^T landed (MMA commit); the second one: the second buffer of a DV launch
+  uint64_t* bar_s = bars + 1;        // [2] S^T landed (MMA commit); the second one: the second buffer of the DV role
   uint64_t* bar_dp = bars + 3;       // dP^T landed
-  uint64_t* bar_p = bars + 4;        // P^T codes and words written (DK launch: S^T in registers); one arrival per compute warp
+  uint64_t* bar_p = bars + 4;        // P^T codes and words written (DK role: S^T in registers); one arrival per compute warp
   uint64_t* bar_k = bars + 5;        // dS^T codes and words written
   uint64_t* bar_done = bars + 6;     // the tile's chains done (MMA commit): columns and staging tile are free
   uint64_t* full_q = bars + 8;       // [kStages] Q and the vectors landed
@@ -222,7 +220,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                       words + h, ones, !first || (ks > 0));
       }
     };
-    // S^T of tile i: into the one S^T region, or alternating (DV launch)
+    // S^T of tile i: into the one S^T region, or alternating (DV role)
     auto issue_s = [&](int i) -> bool {
       if (!landed(full_q, i)) return false;
       tc_fence_after();
@@ -367,7 +365,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             xv |= sb_mul(psb, scale_to_sb(c ? dos2.y : dos2.x)) << (8 * c);
           }
         }
-        if (!DK) {                                       // DV launch: the words go beside the codes, and that is the tile
+        if (!DK) {                                       // DV role: the words go beside the codes, and that is the tile
           tmem_st4(t_s + C::kColXv, xv, xv, xv, xv);
           if (half == 0) tmem_st4(t_s + C::kColOne, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
           tmem_wait_st();
@@ -466,7 +464,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         ws_tile += qt0 * n_t;
       }
     }
-    // (a DV launch's last codes may be written before the chains of the tile before are done: both phases by name)
+    // (the DV role's last codes may be written before the chains of the tile before are done: both phases by name)
     if (!DK && ok && n_it > 1) ok = wait_warp(bar_done, n_it & 1, abort_flag);
     if (ok) ok = wait_warp(bar_done, (n_it - 1) & 1, abort_flag);
     if (!ok) {
@@ -498,35 +496,51 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == C::kComputeWarps) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-template <int D, bool DV, bool DK, bool DS32, int G>
+constexpr int kKvGroups = 2;       // compute warpgroups (8 warps): with four, each warp's fixed work per tile is done sixteen times
+                                   // (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256 the two are equal
+
+template <int D, bool DS32>
+struct KvLaunch {
+  using Dk = KvCfg<D, D == 128, true, kKvGroups>;
+  using Dv = KvCfg<D, true, D == 128, kKvGroups>;
+  static constexpr int kThreads = Dk::kThreads;
+  static constexpr int kSmemBytes = Dk::kSmemBytes > Dv::kSmemBytes ? Dk::kSmemBytes : Dv::kSmemBytes;
+};
+
+// Head_dim 256: both roles in one grid, the longer one (dK) first: a short call's dV CTAs run beside its dK CTAs.
+template <int D, bool DS32>
+__global__ void __launch_bounds__(KvLaunch<D, DS32>::kThreads, 1)
+bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
+  if constexpr (D == 128) dkdv_tile<128, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+  else if (blockIdx.z == 0) dkdv_tile<256, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+  else dkdv_tile<256, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+}
+
+template <int D, bool DS32>
 static cudaError_t launch_kv_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                                const CUtensorMap& tds, const BwdParams& p, cudaStream_t stream) {
-  using C = KvCfg<D, DV, DK, G>;
+  using L = KvLaunch<D, DS32>;
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, DV, DK, DS32, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) return e;
     done[dev] = true;
   }
-  dim3 grid(p.B * p.Hk, p.N / 128);
+  const dim3 grid(p.B * p.Hk, p.N / 128, D == 128 ? 1 : 2);
   count_launch();
-  return launch_chained(bwd_dkdv_kernel<D, DV, DK, DS32, G>, grid, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
+  return launch_chained(bwd_dkdv_kernel<D, DS32>, grid, L::kThreads, L::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
 }
 
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const CUtensorMap& tdo, const CUtensorMap* tds_or_null, const BwdParams& p,
                             cudaStream_t stream) {
   const CUtensorMap& tds = (tds_or_null != nullptr) ? *tds_or_null : tq;     // unused by the kernel without a workspace
-  if (D == 128) {
-    return p.ds32 ? launch_kv_t<128, true, true, true, 2>(tq, tk, tv, tdo, tds, p, stream)
-                  : launch_kv_t<128, true, true, false, 2>(tq, tk, tv, tdo, tds, p, stream);
-  }
-  cudaError_t e = launch_kv_t<256, true, false, false, 4>(tq, tk, tv, tdo, tds, p, stream);
-  if (e != cudaSuccess) return e;
-  return p.ds32 ? launch_kv_t<256, false, true, true, 2>(tq, tk, tv, tdo, tds, p, stream)
-                : launch_kv_t<256, false, true, false, 2>(tq, tk, tv, tdo, tds, p, stream);
+  if (D == 128) return (p.ds32 ? launch_kv_t<128, true> : launch_kv_t<128, false>)(tq, tk, tv, tdo, tds, p, stream);
+  return (p.ds32 ? launch_kv_t<256, true> : launch_kv_t<256, false>)(tq, tk, tv, tdo, tds, p, stream);
 }
 
 }  // namespace dm
