@@ -127,7 +127,7 @@ bwd_dq_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int st = it % C::kStages;
         if (it >= C::kStages) {
           if (!wait_or_abort(empty + st, ((it / C::kStages) - 1) & 1, abort_flag)) {
-            raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+            raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDq);
             break;
           }
         }
@@ -177,7 +177,7 @@ bwd_dq_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tc_commit(empty + st);
         tc_commit(bar_done);
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDq);
     }
   } else {
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
@@ -270,7 +270,7 @@ bwd_dq_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
     if (ok) ok = wait_warp(bar_done, (n_it - 1) & 1, abort_flag);
     if (!ok) {
-      raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+      raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDq);
     } else {
       tc_fence_after();
       __nv_bfloat16* dst = p.dq + static_cast<int64_t>(b) * p.dq_sb + static_cast<int64_t>(row) * p.dq_sn +
@@ -416,7 +416,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           tma_load_2d(sV + st * C::kTileBytes, &tm_v, full + st, 0, row);
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDq);
     }
   } else if (warp == 17) {
     // ------------------------------------------------------------------------------------------ MMA issuer
@@ -478,7 +478,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (cur.item < n_items) dq_walk_set(cur, p, n_t, bh_count);
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDq);
     }
   } else {
     // ------------------------------------------------------------------------------------------ compute groups
@@ -608,7 +608,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDq);
   }
   tc_fence_before();
   __syncthreads();
@@ -648,9 +648,7 @@ cudaError_t launch_bwd_dq(int D, const CUtensorMap& tq, const CUtensorMap& tk, c
   static bool done[64] = {};
   cudaError_t e = set_smem(bwd_dq_kernel, DqCfg::kSmemBytes, done);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int n_items = (p.N / 128) * p.B * p.H;
   count_launch();
   return launch_chained(bwd_dq_kernel, n_items < sms ? n_items : sms, DqCfg::kThreads, DqCfg::kSmemBytes, stream, tq, tk, tv, tdo, p);

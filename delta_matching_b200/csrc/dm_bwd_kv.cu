@@ -29,12 +29,12 @@ namespace dm {
 // With sixteen warps on 32 queries each and one 128-column region that S^T and dP^T shared (what this kernel did before), every
 // link of the chain was exposed and the fixed work of a warp per tile was done sixteen times.
 //
-// Head_dim 256: one accumulator fills 256 columns, so a key tile is two CTAs: a DV role (S^T, P^T codes, dV; the columns of dP^T
+// Head_dim 256: one accumulator fills 256 columns, so a key tile is two CTAs (and so it is in small grids at head_dim 128): a DV role (S^T, P^T codes, dV; the columns of dP^T
 // are a second S^T buffer, and the words lie beside the codes) and a DK role (S^T, dP^T, dS codes, dK and the dS tiles for
 // the workspace), each with the other half of the work compiled out.
 template <int D, bool DV, bool DK, int G>
 struct KvCfg {
-  static_assert(D == 128 ? (DV && DK) : (D == 256 && DV != DK), "128: both accumulators; 256: one per role");
+  static_assert((D == 128 || D == 256) && (DV || DK) && !(D == 256 && DV && DK), "two accumulators of 256 columns fill the TMEM");
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
   static constexpr int kCodeBytes = 128 * 128;         // dS^T code tile (does not depend on head_dim)
@@ -48,7 +48,7 @@ struct KvCfg {
   static constexpr int kColXv = 8 * kCh;          // 64 h + 16: 4 columns of the dV scale word of half h (byte c = block 2 h + c)
   static constexpr int kColXk = 8 * kCh + 4;          // 64 h + 20: likewise, dK
   static constexpr int kColOne = 8 * kCh + 8;         // 4 columns of 0x7F7F7F7F (written by h = 0)
-  static constexpr int kColDv = 256, kColDk = (D == 128) ? 384 : 256;
+  static constexpr int kColDv = 256, kColDk = (DV && DK) ? 384 : 256;
   static constexpr int kSmemK = 0;
   static constexpr int kSmemV = kTileBytes;                          // the DV role has no V tile
   static constexpr int kSmemQ = DK ? 2 * kTileBytes : kTileBytes;    // [kStages]
@@ -89,8 +89,12 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
   uint64_t* bar_s = bars + 1;        // [2] S^T landed (MMA commit); the second one: the second buffer of the DV role
   uint64_t* bar_dp = bars + 3;       // dP^T landed
   uint64_t* bar_p = bars + 4;        // P^T codes and words written (DK role: S^T in registers); one arrival per compute warp
+  uint64_t* bar_p1 = bars + 26;      // DV role: the same for odd tiles.  S^T of tile i + 1 is issued before the MMA warp has seen the
+                                     // codes of tile i, so the compute warps can be two hand-offs ahead of it: with one barrier its
+                                     // parity test could miss a phase and wait for good
   uint64_t* bar_k = bars + 5;        // dS^T codes and words written
   uint64_t* bar_done = bars + 6;     // the tile's chains done (MMA commit): columns and staging tile are free
+  uint64_t* bar_acc = bars + 7;      // every chain of the CTA done (MMA commit behind the last one)
   uint64_t* full_q = bars + 8;       // [kStages] Q and the vectors landed
   uint64_t* full_d = bars + 12;      // [kStages] dO landed
   uint64_t* vec_ok = bars + 16;      // [kStages] the vectors landed and -lse * log2e is written
@@ -116,8 +120,10 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
     mbar_init(bar_s + 1, 1);
     mbar_init(bar_dp, 1);
     mbar_init(bar_p, C::kComputeWarps);
+    mbar_init(bar_p1, C::kComputeWarps);
     mbar_init(bar_k, C::kComputeWarps);
     mbar_init(bar_done, 1);
+    mbar_init(bar_acc, 1);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(full_q + s, 1);
       mbar_init(full_d + s, 1);
@@ -153,7 +159,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       for (int i = 0; i < n_it; ++i) {
         const int st = i % C::kStages;
         if (i >= C::kStages && !wait_or_abort(empty + st, ((i / C::kStages) - 1) & 1, abort_flag)) {
-          raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+          raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDkDv);
           break;
         }
         uint8_t* v = smem + C::kSmemVec + st * C::kVecBytes;
@@ -191,7 +197,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       __syncwarp();
       if (lane == 0) mbar_arrive(vec_ok + st);
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDkDv);
   } else if (warp == C::kComputeWarps) {
     // ------------------------------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop (uniform values stay in uniform registers), one elected thread issues.
@@ -250,7 +256,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         if (i > 0 && !(ok = wait_warp(bar_done, ph ^ 1, abort_flag))) break;
         if (!(ok = issue_s(i + 1))) break;
       }
-      if (!(ok = wait_warp(bar_p, ph, abort_flag))) break;
+      if (!(ok = DK ? wait_warp(bar_p, ph, abort_flag) : wait_warp((i & 1) ? bar_p1 : bar_p, (i >> 1) & 1, abort_flag))) break;
       if (DV) {
         if (!DK && !(ok = landed(full_d, i))) break;
         tc_fence_after();
@@ -261,6 +267,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           if (!DK) {
             tc_commit(bar_done);
             tc_commit(empty + i % C::kStages);
+            if (i == n_it - 1) tc_commit(bar_acc);
           }
         }
       }
@@ -273,6 +280,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           chain_acc(tmem + C::kColDk, tmem + C::kColDp + C::kColCodes, tmem + C::kColDp + C::kColXk, tmem + C::kColDp + C::kColOne, b_lo, i == 0);
           tc_commit(bar_done);
           tc_commit(empty + i % C::kStages);
+          if (i == n_it - 1) tc_commit(bar_acc);
           if (p.ds_codes != nullptr) {                   // the dS^T codes of the tile, from its staging tile, to the workspace
             tma_store_2d(&tm_ds, smem + C::kSmemWs + (i & 1) * C::kCodeBytes, 0, ws_row);
             bulk_commit_group();
@@ -292,7 +300,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       }
     }
     if (DK && p.ds_codes != nullptr) bulk_wait_group<0>();
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDkDv);
   } else if (warp < C::kComputeWarps) {
     // ------------------------------------------------------------------------------------------ compute warps
     constexpr int CH = C::kCh;
@@ -371,7 +379,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if ((tid & 31) == 0) mbar_arrive(bar_p);
+          if ((tid & 31) == 0) mbar_arrive(ph ? bar_p1 : bar_p);
         }
       }
       float am[2] = {0.f, 0.f};
@@ -464,11 +472,11 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         ws_tile += qt0 * n_t;
       }
     }
-    // (the DV role's last codes may be written before the chains of the tile before are done: both phases by name)
-    if (!DK && ok && n_it > 1) ok = wait_warp(bar_done, n_it & 1, abort_flag);
-    if (ok) ok = wait_warp(bar_done, (n_it - 1) & 1, abort_flag);
+    // A barrier of its own: waiting for a phase of bar_done by its parity would, for a warp that comes late, mistake the end of
+    // the phase after it for one that is still to come.
+    if (ok) ok = wait_warp(bar_acc, 0, abort_flag);
     if (!ok) {
-      raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+      raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDkDv);
     } else {
       tc_fence_after();
       // two warps per lane quadrant: each writes 64 columns of every 128-column slice of the accumulators
@@ -499,48 +507,53 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
 constexpr int kKvGroups = 2;       // compute warpgroups (8 warps): with four, each warp's fixed work per tile is done sixteen times
                                    // (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256 the two are equal
 
-template <int D, bool DS32>
+template <int D, bool Roles>
 struct KvLaunch {
-  using Dk = KvCfg<D, D == 128, true, kKvGroups>;
-  using Dv = KvCfg<D, true, D == 128, kKvGroups>;
+  using Dk = KvCfg<D, !Roles, true, kKvGroups>;
+  using Dv = KvCfg<D, true, !Roles, kKvGroups>;
   static constexpr int kThreads = Dk::kThreads;
   static constexpr int kSmemBytes = Dk::kSmemBytes > Dv::kSmemBytes ? Dk::kSmemBytes : Dv::kSmemBytes;
 };
 
-// Head_dim 256: both roles in one grid, the longer one (dK) first: a short call's dV CTAs run beside its dK CTAs.
-template <int D, bool DS32>
-__global__ void __launch_bounds__(KvLaunch<D, DS32>::kThreads, 1)
+// Roles: dK and dV of a key tile by two CTAs, both kinds in one grid, the longer one (dK) first.
+template <int D, bool Roles, bool DS32>
+__global__ void __launch_bounds__(KvLaunch<D, Roles>::kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
-  if constexpr (D == 128) dkdv_tile<128, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
-  else if (blockIdx.z == 0) dkdv_tile<256, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
-  else dkdv_tile<256, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+  if constexpr (!Roles) dkdv_tile<D, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+  else dkdv_tile<D, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
 }
 
-template <int D, bool DS32>
+template <int D, bool Roles, bool DS32>
 static cudaError_t launch_kv_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                                const CUtensorMap& tds, const BwdParams& p, cudaStream_t stream) {
-  using L = KvLaunch<D, DS32>;
+  using L = KvLaunch<D, Roles>;
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, Roles, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) return e;
     done[dev] = true;
   }
-  const dim3 grid(p.B * p.Hk, p.N / 128, D == 128 ? 1 : 2);
+  const dim3 grid(p.B * p.Hk, p.N / 128, Roles ? 2 : 1);
   count_launch();
-  return launch_chained(bwd_dkdv_kernel<D, DS32>, grid, L::kThreads, L::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
+  return launch_chained(bwd_dkdv_kernel<D, Roles, DS32>, grid, L::kThreads, L::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
 }
 
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const CUtensorMap& tdo, const CUtensorMap* tds_or_null, const BwdParams& p,
                             cudaStream_t stream) {
   const CUtensorMap& tds = (tds_or_null != nullptr) ? *tds_or_null : tq;     // unused by the kernel without a workspace
-  if (D == 128) return (p.ds32 ? launch_kv_t<128, true> : launch_kv_t<128, false>)(tq, tk, tv, tdo, tds, p, stream);
-  return (p.ds32 ? launch_kv_t<256, true> : launch_kv_t<256, false>)(tq, tk, tv, tdo, tds, p, stream);
+  // Head_dim 256 has no choice.  At head_dim 128 the roles cost a second S^T and a second exponential per element, so they
+  // are for grids that leave half of the SMs without a CTA: each role's chain per tile is the shorter one then (the same
+  // bits: the accumulators do not depend on each other).
+  if (D != 128) return (p.ds32 ? launch_kv_t<256, true, true> : launch_kv_t<256, true, false>)(tq, tk, tv, tdo, tds, p, stream);
+  if (2ll * p.B * p.Hk * (p.N / 128) <= sm_count())
+    return (p.ds32 ? launch_kv_t<128, true, true> : launch_kv_t<128, true, false>)(tq, tk, tv, tdo, tds, p, stream);
+  return (p.ds32 ? launch_kv_t<128, false, true> : launch_kv_t<128, false, false>)(tq, tk, tv, tdo, tds, p, stream);
 }
 
 }  // namespace dm

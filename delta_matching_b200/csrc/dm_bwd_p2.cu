@@ -112,7 +112,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
             tma_load_2d(sK + st * C::kKBytes + sub * 16384, &tm_k, full + st, sub * 128, bhk * p.N + it * 128);
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDqPass2);
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------------------------------ MMA issuer
@@ -145,7 +145,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
           if (it == n_it - 1) tc_commit(dq_full + acc);
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDqPass2);
     }
   } else if (warp < 4) {
     // ------------------------------------------------------------------------------------------ scale words
@@ -219,7 +219,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         if ((tid & 31) == 0) mbar_arrive(full + st);
       }
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDqPass2);
   } else {
     // ------------------------------------------------------------------------------------------ dQ read-out
     const int quad = warp & 3;
@@ -255,7 +255,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
       __syncwarp();
       if ((tid & 31) == 0) mbar_arrive(dq_free + acc);
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDqPass2);
   }
   tc_fence_before();
   __syncthreads();
@@ -266,17 +266,14 @@ template <int D>
 static cudaError_t launch_p2_t(const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream) {
   using C = DqP2Cfg<D>;
   static bool attr_set[64] = {};
-  static int sm_count[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(bwd_dq_p2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
+  const int sms = sm_count();
   const int items = (p.N / 128) * p.B * p.H;
   count_launch();
   return launch_chained(bwd_dq_p2_kernel<D>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, p);

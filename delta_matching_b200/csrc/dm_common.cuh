@@ -13,6 +13,12 @@ enum : int {
   kStatusTimeoutMma = 2,        // MMA issuer gave up waiting for operands or for the compute warps
   kStatusTimeoutCompute = 3,    // compute warps gave up waiting for an accumulator
   kStatusTimeoutProbe = 4,
+  // which kernel it was, added to the code
+  kInForward = 1 << 4,
+  kInDelta = 2 << 4,
+  kInDkDv = 3 << 4,
+  kInDq = 4 << 4,
+  kInDqPass2 = 5 << 4,
 };
 
 constexpr float kLog2e = 1.4426950408889634f;

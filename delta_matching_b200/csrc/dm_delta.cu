@@ -136,7 +136,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
           }
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDelta);
     }
   } else if (warp == 17) {
     // ------------------------------------------------------------------------------------------ MMA issuer
@@ -174,7 +174,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         }
         tc_commit(bar_qfree);
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDelta);
     }
   } else {
     // ------------------------------------------------------------------------------------------ compute groups
@@ -288,7 +288,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         if (ok) p.delta[static_cast<size_t>(bh) * p.N + row] = static_cast<float>(p.norm ? n / dd : n);
       }
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDelta);
   }
   tc_fence_before();
   __syncthreads();
@@ -307,13 +307,8 @@ static cudaError_t launch_delta_t(const CUtensorMap& tq, const CUtensorMap& tk, 
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  static int sm_count[64] = {};
-  if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
-    cudaError_t e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-  }
   const int n_items = (p.N / 128) * p.B * p.H;
-  const int ctas = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
+  const int ctas = sm_count();
   count_launch();
   return launch_chained(delta_kernel<D>, n_items < ctas ? n_items : ctas, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, p);
 }

@@ -152,7 +152,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             tma_load_2d(sV + st * C::kTileBytes + s * 16384, &tm_v, full_v + st, s * 128, row);
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInForward);
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------------------------------ MMA issuer
@@ -218,7 +218,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           tc_commit(o_bar(gt));
         }
       }
-      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInForward);
     }
   } else {
     // ------------------------------------------------------------------------------------------ softmax / epilogue
@@ -388,7 +388,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       p.lse[static_cast<size_t>(bh) * p.N + row] = (m + log2f(l)) * kLn2;
     }
-    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute);
+    if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInForward);
   }
   tc_fence_before();
   __syncthreads();
@@ -407,12 +407,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  static int sm_count[64] = {};
-  if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
-    cudaError_t e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-  }
-  const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
+  const int sms = sm_count();
   const int items = (p.N / 128) * p.B * p.H;
   const int ctas = sms * ((D == 128) ? 2 : 1);              // co-resident CTAs: 256 of the 512 TMEM columns each at D = 128
   count_launch();

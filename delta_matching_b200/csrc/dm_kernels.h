@@ -98,6 +98,9 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, int sme
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// SMs of the current device (looked up once per device).
+int sm_count();
+
 // Kernel launches made by the library in this process (every launcher counts its own).
 void count_launch(int n = 1);
 long long launch_count();

@@ -73,12 +73,14 @@ __global__ void kmean_fold_kernel(const KMeanParams p) {
     const float* src = p.partial + static_cast<size_t>(bh) * nchunk * p.D + c;
     float s = 0.f;
     int j = 0;
-    for (; j + 8 <= nchunk; j += 8) {               // eight loads in flight, added in chunk order
-      float v[8];
+    // Bound by the latency of its loads, 0.6 us a batch: 32 in flight, added in chunk order (with eight the fold of 512 chunks
+    // took longer than the chunk sums themselves: q, k, v producers at N=32768 H=64 Hk=8 206 -> 181 us).
+    for (; j + 32 <= nchunk; j += 32) {
+      float v[32];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = src[static_cast<size_t>(j + u) * p.D];
+      for (int u = 0; u < 32; ++u) v[u] = src[static_cast<size_t>(j + u) * p.D];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) s += v[u];
+      for (int u = 0; u < 32; ++u) s += v[u];
     }
     for (; j < nchunk; ++j) s += src[static_cast<size_t>(j) * p.D];
     p.mean[static_cast<size_t>(bh) * p.D + c] = s / static_cast<float>(p.N);
@@ -97,13 +99,13 @@ cudaError_t launch_kmean(const KMeanParams& p, cudaStream_t stream) {
 cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream);
 // kMean / kStale: the K tensor alone subtracts a mean and the dO tensor of the stale mode alone reads O; compiled out
 // elsewhere, the kernel needs fewer registers and more of its small CTAs fit an SM (more loads in flight).
+// Executed by 128 threads (tid 0-127), which meet at the named barrier `bar`.
 template <int D, bool kMean, bool kStale>
-__device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int bh, float* wmax) {
+__device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int bh, float* wmax, int tid = threadIdx.x, int bar = 1) {
   constexpr int kTpr = D / 16;           // threads per token row (16 elements each)
   constexpr int kRpp = 128 / kTpr;       // rows per pass
   constexpr int kPass = 32 / kRpp;
   const int b = bh / p.H, h = bh % p.H;
-  const int tid = threadIdx.x;
   const int c16 = tid % kTpr, r0 = tid / kTpr;
   const __nv_bfloat16* xb = p.x + b * p.sb + h * p.sh + static_cast<int64_t>(blk) * 32 * p.sn + c16 * 16;
 
@@ -150,7 +152,7 @@ __device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int b
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
   if ((tid & 31) == 0) wmax[tid >> 5] = amax;
-  __syncthreads();
+  bar_sync(bar, 128);
   amax = fmaxf(fmaxf(wmax[0], wmax[1]), fmaxf(wmax[2], wmax[3]));
   const uint32_t sb = pow2_sb(amax, 127u);
   const float inv = sb_to_inv(sb);
@@ -170,17 +172,17 @@ __device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int b
 }
 
 template <int D, bool kMean, bool kStale>
-__global__ void __launch_bounds__(128) quant_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(128, D == 128 ? 10 : 6) quant_kernel(const QuantParams p) {
   __shared__ float wmax[4];
   grid_dep_wait();
   quant_block<D, kMean, kStale>(p, blockIdx.x, blockIdx.y, wmax);
 }
 
-// Q, V and the chunk sums of the K mean in one launch: the three need nothing from each other, and as separate launches
+// Longer sequences.  Q, V and the chunk sums of the K mean in one launch: the three need nothing from each other, and as separate launches
 // of a few microseconds each they spend a good part of their time filling and draining the GPU.  The grid is the
 // concatenation [K-mean chunks | Q blocks | V blocks] (the chunk sums first: the fold and the K quantiser wait for them).
 template <int D>
-__global__ void __launch_bounds__(128) quant_qv_kmean_kernel(const QuantParams pq, const QuantParams pv, const KMeanParams pk) {
+__global__ void __launch_bounds__(128, D == 128 ? 10 : 6) quant_qv_kmean_kernel(const QuantParams pq, const QuantParams pv, const KMeanParams pk) {
   __shared__ float wmax[4];
   __shared__ float red[KMeanTile<D>::kRpp][D];
   grid_dep_wait();
@@ -197,8 +199,124 @@ __global__ void __launch_bounds__(128) quant_qv_kmean_kernel(const QuantParams p
   }
 }
 
+// Q, K and V of a short sequence in one launch.  A CTA has one group of 128 threads per 64 tokens; the K CTA of a (batch, kv
+// head) holds the whole head in registers between the chunk sums, their fold and the quantisation (K is read once), the other
+// CTAs take one 32-token block of Q or V per group.  For N / 64 groups of 32 x D / 128 bf16 values a thread: up to
+// kShortTokens tokens.  Three launches of one or two microseconds each before (N=256: 6.6 us and three times the host's launch time).
+template <int D>
+constexpr int kShortTokens = (D == 128) ? 512 : 256;
+
+// The packed values are what stays in registers between the passes over them, not their fp32 forms.
+template <int N>
+__device__ __forceinline__ void keep_packed(uint4 (&x)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(x[i].x), "+r"(x[i].y), "+r"(x[i].z), "+r"(x[i].w));
+}
+
+template <int D>
+__device__ __forceinline__ void quant_k_head(const QuantParams& p, float* mean_out, int bh, float* red, float* mean, float* wmax) {
+  constexpr int kTpr = D / 8, kRpp = 128 / kTpr, kPass = 64 / kRpp;      // thread layout of the chunk sums (kmean_block)
+  const int b = bh / p.H, h = bh % p.H;
+  const int group = threadIdx.x / 128, tid = threadIdx.x % 128, n_chunk = p.N / 64;
+  const int c8 = tid % kTpr, r0 = tid / kTpr;
+  const __nv_bfloat16* base = p.x + b * p.sb + h * p.sh + static_cast<int64_t>(group) * 64 * p.sn + c8 * 8;
+  uint4 x[kPass];
+#pragma unroll
+  for (int i = 0; i < kPass; ++i) x[i] = __ldg(reinterpret_cast<const uint4*>(base + (r0 + i * kRpp) * p.sn));
+  {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < kPass; ++i) {
+      float f[8];
+      bf16x8_to_float(x[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += f[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[(group * kRpp + r0) * D + c8 * 8 + j] = acc[j];
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < D; c += blockDim.x) {      // the sums of the chunks, then their fold, in the order of kmean_block
+    float s = 0.f;
+    for (int g = 0; g < n_chunk; ++g) {
+      float t = red[g * kRpp * D + c];
+#pragma unroll
+      for (int r = 1; r < kRpp; ++r) t += red[(g * kRpp + r) * D + c];
+      s += t;
+    }
+    s /= static_cast<float>(p.N);
+    mean[c] = s;
+    mean_out[static_cast<size_t>(bh) * D + c] = s;
+  }
+  __syncthreads();
+  keep_packed(x);
+  float m[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) m[j] = mean[c8 * 8 + j];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {                   // the two 32-token blocks of the group's chunk
+    float amax = 0.f;
+#pragma unroll
+    for (int i = half * kPass / 2; i < (half + 1) * kPass / 2; ++i) {
+      float f[8];
+      bf16x8_to_float(x[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf((f[j] - m[j]) * p.prescale));
+    }
+    amax = warp_max(amax);
+    if ((tid & 31) == 0) wmax[group * 8 + half * 4 + (tid >> 5)] = amax;
+  }
+  bar_sync(1 + group, 128);
+  keep_packed(x);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const float* w4 = wmax + group * 8 + half * 4;
+    const uint32_t sb = pow2_sb(fmaxf(fmaxf(w4[0], w4[1]), fmaxf(w4[2], w4[3])), 127u);
+    const float inv = sb_to_inv(sb);
+    if (tid == 0) p.scales[static_cast<size_t>(bh) * (p.N / 32) + group * 2 + half] = sb_to_scale(sb);
+#pragma unroll
+    for (int i = half * kPass / 2; i < (half + 1) * kPass / 2; ++i) {
+      float f[8];
+      bf16x8_to_float(x[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = ((f[j] - m[j]) * p.prescale) * inv;
+      uint2 w;
+      w.x = cvt_e4m3x4(f[0], f[1], f[2], f[3]);
+      w.y = cvt_e4m3x4(f[4], f[5], f[6], f[7]);
+      *reinterpret_cast<uint2*>(p.codes + (static_cast<size_t>(bh) * p.N + group * 64 + r0 + i * kRpp) * D + c8 * 8) = w;
+    }
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kShortTokens<D> * 2) quant_qkv_short_kernel(const QuantParams pq, const QuantParams pk, const QuantParams pv, float* mean_out) {
+  constexpr int kGroups = kShortTokens<D> / 64, kRpp = KMeanTile<D>::kRpp;
+  __shared__ float red[kGroups * kRpp * D];
+  __shared__ float mean[D];
+  __shared__ float wmax[kGroups * 8];
+  grid_dep_wait();
+  const int n_k = pk.B * pk.H, groups = blockDim.x / 128;
+  if (static_cast<int>(blockIdx.x) < n_k) {
+    quant_k_head<D>(pk, mean_out, blockIdx.x, red, mean, wmax);
+    return;
+  }
+  const int group = threadIdx.x / 128, blocks = pq.N / 32;
+  int i = (static_cast<int>(blockIdx.x) - n_k) * groups + group;
+  const int n_q = blocks * pq.B * pq.H, n_v = blocks * pv.B * pv.H;
+  if (i < n_q) quant_block<D, false, false>(pq, i % blocks, i / blocks, wmax + 4 * group, threadIdx.x % 128, 1 + group);
+  else if ((i -= n_q) < n_v) quant_block<D, false, false>(pv, i % blocks, i / blocks, wmax + 4 * group, threadIdx.x % 128, 1 + group);
+}
+
 cudaError_t launch_quant_qkv(const QuantParams& pq, const QuantParams& pk, const QuantParams& pv, const KMeanParams& pm,
                              cudaStream_t stream) {
+  const int short_tokens = pq.D == 128 ? kShortTokens<128> : kShortTokens<256>;
+  if (pm.N <= short_tokens) {
+    const int groups = pm.N / 64;                        // 2 .. 8 (N is a multiple of 128)
+    const long long qv = static_cast<long long>(pq.N / 32) * (pq.B * pq.H + pv.B * pv.H);
+    count_launch();
+    return launch_chained(pq.D == 128 ? quant_qkv_short_kernel<128> : quant_qkv_short_kernel<256>,
+                          static_cast<unsigned>(pk.B * pk.H + (qv + groups - 1) / groups), groups * 128, 0, stream, pq, pk, pv, pm.mean);
+  }
   const long long blocks = static_cast<long long>(pm.N / 64) * pm.B * pm.Hk + static_cast<long long>(pq.N / 32) * pq.B * pq.H +
                            static_cast<long long>(pv.N / 32) * pv.B * pv.H;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;

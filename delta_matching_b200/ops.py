@@ -33,6 +33,7 @@ _DEBUG = os.environ.get("DM_DEBUG", "0") not in ("", "0")
 
 STATUS_TEXT = {1: "TMA producer gave up waiting for a free stage", 2: "MMA issuer gave up waiting",
                3: "compute warps gave up waiting for an accumulator", 4: "probe kernel gave up waiting"}
+STATUS_KERNEL = {1: "forward", 2: "matched delta", 3: "dK/dV", 4: "dQ", 5: "dQ pass 2"}     # v >> 4
 
 
 def _ptr(t):
@@ -85,7 +86,7 @@ def _raise_if_set(idx: int) -> None:
     if v != 0:
         w[0] = 0
         raise RuntimeError(f"delta_matching: a kernel on cuda:{idx} reported status {v} "
-                           f"({STATUS_TEXT.get(v, 'unknown')}); its outputs are invalid")
+                           f"({STATUS_KERNEL.get(v >> 4, 'kernel')}: {STATUS_TEXT.get(v & 15, 'unknown')}); its outputs are invalid")
 
 
 def check_status(device=None) -> None:

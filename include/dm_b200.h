@@ -35,6 +35,7 @@ extern "C" {
 #define DM_STATUS_TIMEOUT_MMA 2
 #define DM_STATUS_TIMEOUT_COMPUTE 3
 #define DM_STATUS_TIMEOUT_PROBE 4
+/* the low four bits; the bits above name the kernel: 1 forward, 2 matched delta, 3 dK/dV, 4 dQ, 5 dQ pass 2 */
 
 /* Library identity.  Replaces the build-sanity ops build_gt() / build_hd128() / build_bf16dp() of
  * csrc/delta_matching_api.cpp:683-715: dm_version() is MAJOR * 10000 + MINOR * 100 + PATCH; dm_numerics() names the

@@ -1,0 +1,37 @@
+"""The variants that small problems take, against the forms that large ones take: the producers of a short sequence in one
+launch, dK and dV as two roles.  What a (batch, head) unit computes must not depend on
+how many units the call has, so the bits of a small call are those of the same units inside a large one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,N,H,Hk,D", [(1, 256, 2, 1, 128), (2, 512, 3, 3, 128), (1, 128, 2, 2, 256), (3, 256, 2, 1, 256)])
+def test_short_producers_equal_the_separate_ones(B, N, H, Hk, D, oracle):
+    from delta_matching_b200 import ops
+    q, k, v, _ = (t.transpose(1, 2) for t in oracle.make_inputs(B, N, H, Hk, D, seed=71, device="cuda"))
+    k = k + 0.5
+    q8, qs, k8, ks, v8, vs, km = ops.quant_qkv(q, k, v)
+    mean = ops.kmean(k)
+    assert torch.equal(km, mean)
+    for (codes, scales), (c, s) in (((q8, qs), ops.quant_rows(q, D ** -0.5)), ((k8, ks), ops.quant_rows(k, 1.0, mean)), ((v8, vs), ops.quant_rows(v))):
+        assert torch.equal(codes.view(torch.uint8), c.view(torch.uint8)) and torch.equal(scales, s)
+
+
+@pytest.mark.parametrize("N,rep,D,causal,mode,scale", [(256, 1, 128, True, "matched", 1.0), (1280, 3, 128, True, "matched", 4.0), (768, 2, 128, False, "stale", 12.0),
+                                                       (384, 1, 256, True, "matched", 1.0), (640, 2, 256, False, "stale", 6.0)])
+def test_a_unit_has_the_same_bits_in_a_small_and_a_large_call(N, rep, D, causal, mode, scale, oracle):
+    import delta_matching_b200 as dm
+    units = -(-160 // (N // 128))                        # more work items than SMs
+    q, k, v, do = oracle.make_inputs(units, N, rep, 1, D, seed=72, device="cuda", qk_scale=scale)
+
+    def step(b0, b1):
+        leaves = [t[b0:b1].detach().requires_grad_() for t in (q, k, v)]
+        o = dm.dm_attn_func(*leaves, causal=causal, mode=mode)
+        return (o.detach(),) + torch.autograd.grad(o, leaves, do[b0:b1])
+
+    whole = step(0, units)
+    for u in (0, units - 1):
+        for a, b in zip(step(u, u + 1), whole):
+            assert torch.equal(a, b[u:u + 1])
