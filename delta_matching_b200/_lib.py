@@ -46,6 +46,7 @@ SIGNATURES = {
                          _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "dm_attn_bwd": (_I, [_P, _L, _L, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                          _P, _P, _P, _P, _L, _I, _P, _P]),
+    "dm_attn_bwd_workspace_bytes": (_L, [_I, _I, _I, _I, _I, _I]),
     "dm_dbg_mma_tile": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P]),
     "dm_dbg_wait_expiry": (_I, [_P, _P, _P, ctypes.c_longlong, _P, _P]),
     "dm_launch_count": (ctypes.c_longlong, []),
@@ -128,7 +129,7 @@ def native_attn():
                     raise RuntimeError("delta_matching_b200: _dm_native.so is not built or does not load: run `python -m "
                                        f"delta_matching_b200.build` in the checkout ({e})") from e
                 addr = lambda name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value
-                _dm_native.bind(addr("dm_attn_fwd"), addr("dm_attn_bwd"), addr("dm_last_error"), addr("dm_bwd_workspace_bytes"),
+                _dm_native.bind(addr("dm_attn_fwd"), addr("dm_attn_bwd"), addr("dm_last_error"), addr("dm_attn_bwd_workspace_bytes"),
                                 addr("dm_quant_qkv_workspace_bytes"),
                                 lambda idx: ops.status_word(torch.device("cuda", idx)).data_ptr(), ops._raise_if_set,
                                 lambda *a: ops.bwd_fp8(*a[:11], ds32=a[11]), ops._SMALL_WS, ops._MAX_WS_TILES)

@@ -268,6 +268,24 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
   return e == cudaSuccess ? 0 : cuda_fail(e, "forward launch");
 }
 
+// Which backward dm_attn_bwd runs (same results).  The key-stationary kernel takes as long as its longest chain, (H / Hk)
+// (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.7 us a tile; the tile-parallel
+// pair takes its share of all tiles at about 3.7 us.  Forward + backward, chain / tiles per SM: 16 (N=1024 H=8 Hk=2) 92 -> 60 us;
+// 4.6 (N=8192 H=4 Hk=1) 594 -> 440; 2.3 (N=16384 H=2 Hk=1) 810 -> 758; 2.2 (N=2048 H=32 Hk=8) 222 -> 214; 2.05 (B=4 N=1024 H=16 Hk=4) 140 ->
+// 140; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  The line is drawn at 2.2, and at 2 GiB of workspace.
+static bool tile_parallel(int B, int N, int H, int Hk, int causal) {
+  const long long n_t = N / 128, tiles = static_cast<long long>(B) * H * (causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
+  const long long chain = H / Hk * n_t;
+  return 10 * chain * dm::sm_count() >= 22 * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
+}
+
+int64_t dm_attn_bwd_workspace_bytes(int B, int N, int H, int Hk, int D, int causal) {
+  const int64_t base = dm_bwd_workspace_bytes(B, N, H, D);
+  if (base == 0 || Hk <= 0 || H % Hk || !tile_parallel(B, N, H, Hk, causal)) return base;
+  const int64_t tiles = static_cast<int64_t>(B) * H * (N / 128) * (N / 128);
+  return tiles * (2 * 16384 + 16 + 512);
+}
+
 int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, const void* o,
                 const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
                 const float* lse, void* do8, float* dos, float* delta, int B, int N, int H, int Hk, int D, int causal,
@@ -276,7 +294,7 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   DM_TRY(check_sm100());
   DM_TRY(check_strides("d_o", do_sb, do_sh, do_sn));
   const bool kernels = (flags & DM_ATTN_DELTA_ONLY) == 0;
-  const int64_t need = dm_bwd_workspace_bytes(B, N, H, D);
+  const int64_t need = dm_attn_bwd_workspace_bytes(B, N, H, Hk, D, causal);
   const uint64_t tiles = static_cast<uint64_t>(B) * H * (N / 128) * (N / 128);
   if (kernels && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
     return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed (16-byte aligned)", (long long)workspace_bytes, (long long)need);
@@ -307,8 +325,19 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   p.B = B; p.H = H; p.Hk = Hk; p.N = N; p.causal = causal ? 1 : 0; p.status = status;
   p.ds32 = (flags & DM_DS_BLOCK32) ? 1 : 0;
   p.ds_codes = static_cast<uint8_t*>(workspace);
-  p.ds_words = p.ds_codes + tiles * 16384;
   DM_TRY(make_code_map(&tds, workspace, tiles * 128, 128));
+  if (tile_parallel(B, N, H, Hk, causal)) {
+    // workspace: dS^T tiles, P^T tiles, dS words, P words
+    CUtensorMap tp;
+    DM_TRY(make_code_map(&tp, p.ds_codes + tiles * 16384, tiles * 128, 128));
+    p.ds_words = p.ds_codes + tiles * 2 * 16384;
+    p.p_words = p.ds_words + tiles * 16;
+    e = dm::launch_bwd_tiles(D, tq, tk, tv, td, tds, tp, p, st);
+    if (e != cudaSuccess) return cuda_fail(e, "backward tile launch");
+    e = dm::launch_bwd_stream(D, tq, tk, td, tds, tp, p, st);
+    return e == cudaSuccess ? 0 : cuda_fail(e, "backward streaming launch");
+  }
+  p.ds_words = p.ds_codes + tiles * 16384;
   e = dm::launch_bwd_dkdv(D, tq, tk, tv, td, &tds, p, st);
   if (e != cudaSuccess) return cuda_fail(e, "backward dK/dV launch");
   e = dm::launch_bwd_dq_p2(D, tds, tk, p, st);

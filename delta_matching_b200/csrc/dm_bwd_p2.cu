@@ -11,6 +11,10 @@
 // dS blocks of 128 queries x 32 keys the four words of a tile are equal; with 32 x 32 blocks they differ.  The tile is the A operand of dQ in MN-major form
 // (M = queries contiguous); K is the B operand in MN-major form as in the other kernels.
 //
+// Behind the tile-parallel pass (dm_bwd_tiles.cu) the same kernel, with All, also makes dV = sum P^T dO and dK = sum dS^T Q of
+// every (key tile, kv head), over the group's heads and their query tiles in the order of the key-stationary kernel: there
+// the code tile is the A operand as it lies, K-major (M = keys), and dO / Q the MN-major B operand.
+//
 // One persistent CTA per SM, 320 threads: warps 0-3 write the per-tile scale words into TMEM (byte j = dS scale x K
 // scale of key block j; warp b writes the word of query block b into its 32 rows), warps 4-7 write dQ out (at head_dim 128 two accumulators alternate
 // between items; at head_dim 256 one accumulator fills the columns, and an item's first chain waits for the read-out
@@ -41,9 +45,77 @@ struct DqP2Cfg {
   static_assert(kSmemBytes <= 232448, "shared memory budget");
 };
 
-template <int D>
+// A work item: one accumulator.  kDq: (head, query tile), over key tiles.  kDk, kDv: (kv head, key tile), over (head of the
+// group, query tile).  With All, dK and dV of all key tiles come first, the most tiles first, then dQ likewise.
+enum : int { kDq = 0, kDk = 1, kDv = 2 };
+struct StreamItem {
+  int kind, head, tile;        // head: query head (kDq) or kv head; tile: query tile or key tile
+  int n_it, first, per_head;   // tiles; kDk, kDv: first query tile, query tiles per head
+};
+template <bool All>
+__device__ __forceinline__ int stream_item_count(const BwdParams& p, int n_t) {
+  return n_t * p.B * (p.H + (All ? 2 * p.Hk : 0));
+}
+template <bool All>
+__device__ __forceinline__ StreamItem stream_item(const BwdParams& p, int n_t, int item) {
+  StreamItem r;
+  const int BH = p.B * p.H, BHk = p.B * p.Hk, kv_items = All ? 2 * n_t * BHk : 0;
+  if (All && item < kv_items) {
+    r.kind = kDk + (item & 1);
+    item >>= 1;
+    r.tile = item / BHk;
+    r.head = item % BHk;
+    r.first = p.causal ? r.tile : 0;
+    r.per_head = n_t - r.first;
+    r.n_it = r.per_head * (p.H / p.Hk);
+  } else {
+    item -= kv_items;
+    r.kind = kDq;
+    r.tile = n_t - 1 - item / BH;
+    r.head = item % BH;
+    r.n_it = p.causal ? (r.tile + 1) : n_t;
+    r.first = 0;
+    r.per_head = r.n_it;
+  }
+  return r;
+}
+// Position inside an item: the tile's index in the workspace and its B operand's row (K, Q or dO codes).
+template <bool All>
+struct StreamWalk {
+  int ws, ws_step, row, left, per_head, ws_wrap, row_wrap;
+  __device__ __forceinline__ void set(const BwdParams& p, int n_t, const StreamItem& it) {
+    const int rep = p.H / p.Hk;
+    if (!All || it.kind == kDq) {
+      ws = (it.head * n_t + it.tile) * n_t;
+      ws_step = 1;
+      row = ((it.head / p.H) * p.Hk + (it.head % p.H) / rep) * p.N;
+      ws_wrap = row_wrap = 0;
+    } else {
+      const int bh = (it.head / p.Hk) * p.H + (it.head % p.Hk) * rep;
+      ws = (bh * n_t + it.first) * n_t + it.tile;
+      ws_step = n_t;
+      row = bh * p.N + it.first * 128;
+      ws_wrap = it.first * n_t;                // from the end of one head to the first live query tile of the next
+      row_wrap = it.first * 128;
+    }
+    left = per_head = it.per_head;
+  }
+  __device__ __forceinline__ void next() {
+    ws += ws_step;
+    row += 128;
+    if (All && --left == 0) {
+      left = per_head;
+      ws += ws_wrap;
+      row += row_wrap;
+    }
+  }
+};
+
+template <int D, bool All>
 __global__ void __launch_bounds__(DqP2Cfg<D>::kThreads, 1)
-bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k, const BwdParams p) {
+bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k,
+                  const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_q,
+                  const __grid_constant__ CUtensorMap tm_do, const BwdParams p) {
   using C = DqP2Cfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -63,10 +135,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int n_t = p.N / 128;
-  const int BH = p.B * p.H;
-  const int n_items = n_t * BH;
-  const int rep = p.H / p.Hk;
-  const int nblk = p.N / 32;
+  const int n_items = stream_item_count<All>(p, n_t);
   const int first_item = static_cast<int>(blockIdx.x), item_step = static_cast<int>(gridDim.x);
 
   if (tid == 0) {
@@ -99,17 +168,18 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
       bool ok = true;
       uint32_t g = 0;
       for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k) {
-        const int qt = n_t - 1 - item / BH, bh = item % BH;
-        const int bhk = (bh / p.H) * p.Hk + (bh % p.H) / rep;
-        const int n_it = p.causal ? (qt + 1) : n_t;
-        const int tile0 = (bh * n_t + qt) * n_t;
-        for (int it = 0; it < n_it; ++it, ++g) {
+        const StreamItem itm = stream_item<All>(p, n_t, item);
+        StreamWalk<All> wk;
+        wk.set(p, n_t, itm);
+        const CUtensorMap* ta = (All && itm.kind == kDv) ? &tm_p : &tm_ds;
+        const CUtensorMap* tb = !All || itm.kind == kDq ? &tm_k : itm.kind == kDk ? &tm_q : &tm_do;
+        for (int it = 0; it < itm.n_it; ++it, ++g, wk.next()) {
           const uint32_t st = g % C::kStages;
           if (g >= C::kStages && !(ok = wait_or_abort(empty + st, ((g / C::kStages) - 1) & 1, abort_flag))) break;
           mbar_expect_tx(full + st, C::kDsBytes + C::kKBytes);
-          tma_load_2d(sDs + st * C::kDsBytes, &tm_ds, full + st, 0, (tile0 + it) * 128);
+          tma_load_2d(sDs + st * C::kDsBytes, ta, full + st, 0, wk.ws * 128);
           for (int sub = 0; sub < C::kSub; ++sub)
-            tma_load_2d(sK + st * C::kKBytes + sub * 16384, &tm_k, full + st, sub * 128, bhk * p.N + it * 128);
+            tma_load_2d(sK + st * C::kKBytes + sub * 16384, tb, full + st, sub * 128, wk.row);
         }
       }
       if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDqPass2);
@@ -121,8 +191,10 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
       bool ok = true;
       uint32_t g = 0, n_done = 0;
       for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k, ++n_done) {
-        const int qt = n_t - 1 - item / BH;
-        const int n_it = p.causal ? (qt + 1) : n_t;
+        const StreamItem itm = stream_item<All>(p, n_t, item);
+        const int n_it = itm.n_it;
+        const bool kv_item = All && itm.kind != kDq;
+        const uint32_t a_step = kv_item ? 2 : 256, idesc = kv_item ? idesc_mxf8(128, 128, false, true, 0, 0) : idesc_mxf8(128, 128, true, true, 0, 0);
         const uint32_t acc = n_done % C::kAccs;
         // the accumulator was last used kAccs items ago: its read-out must be complete
         if (n_done >= C::kAccs && !(ok = wait_or_abort(dq_free + acc, ((n_done / C::kAccs) - 1) & 1, abort_flag))) break;
@@ -131,14 +203,15 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
           if (!(ok = wait_or_abort(full + st, (g / C::kStages) & 1, abort_flag))) break;
           tc_fence_after();
           // dQ += dS K over the tile's 128 keys: A = dS^T tile read MN-major, B = K tile read MN-major; both advance
-          // by 32 key rows (4096 bytes) per step; byte ks of the scale word belongs to key block ks
+          // by 32 key rows (4096 bytes) per step; byte ks of the scale word belongs to key block ks.  dK, dV: A K-major, 32
+          // bytes (queries) per step.
           const uint32_t ds_lo = ds_lo0 + st * (C::kDsBytes >> 4), k_lo = k_lo0 + st * (C::kKBytes >> 4);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
             for (int sub = 0; sub < C::kSub; ++sub)
-              mma_mxf8_ss(tmem + C::kColDq + D * acc + 128 * sub, ds_lo + ks * 256, k_lo + sub * 1024 + ks * 256,
-                          idesc_mxf8(128, 128, true, true, ks, 0), tmem + C::kColSf + 4 * st, tmem + C::kColOne,
+              mma_mxf8_ss(tmem + C::kColDq + D * acc + 128 * sub, ds_lo + ks * a_step, k_lo + sub * 1024 + ks * 256,
+                          idesc | (static_cast<uint32_t>(ks) << 29), tmem + C::kColSf + 4 * st, tmem + C::kColOne,
                           (it > 0) || (ks > 0));
           }
           tc_commit(empty + st);
@@ -150,50 +223,56 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
   } else if (warp < 4) {
     // ------------------------------------------------------------------------------------------ scale words
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    const uint32_t* words = reinterpret_cast<const uint32_t*>(p.ds_words);
     tmem_st4(tmem + lane_base + C::kColOne, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
     bool ok = true;
-    // The tile's dS scale word and its four K scales come from global memory: they are requested kAhead tiles before
-    // they are used, through a walk over the CTA's (item, key tile) sequence that runs ahead of the consuming one.
+    // The tile's scale word and the four scales it is multiplied with come from global memory: they are requested kAhead
+    // tiles before they are used, through a walk over the CTA's (item, tile) sequence that runs ahead of the consuming one.
+    //   dQ: the word of this warp's query block (byte = key block) and the tile's four K scales
+    //   dK: byte `warp` (this warp's key block) of the words of the four query blocks and their Q scales
+    //   dV: this row's own word, finished
     constexpr int kAhead = 4;
-    struct Walk {
-      int k, item, it, n_it;
-      const uint32_t* w_ptr;
-      const float4* ks_ptr;
+    int pre_k = 0, pre_item = first_item, pre_left = 0, pre_kind = kDq;
+    StreamWalk<All> pre;
+    auto pre_set = [&]() {
+      if (pre_item >= n_items) return;
+      const StreamItem itm = stream_item<All>(p, n_t, pre_item);
+      pre.set(p, n_t, itm);
+      pre_left = itm.n_it;
+      pre_kind = itm.kind;
     };
-    auto walk_set = [&](Walk& wk) {
-      if (wk.item >= n_items) return;
-      const int qt = n_t - 1 - wk.item / BH, bh = wk.item % BH;
-      const int bhk = (bh / p.H) * p.Hk + (bh % p.H) / rep;
-      wk.it = 0;
-      wk.n_it = p.causal ? (qt + 1) : n_t;
-      wk.w_ptr = words + static_cast<size_t>(bh * n_t + qt) * n_t * 4 + warp;   // this warp's query block of each tile
-      wk.ks_ptr = reinterpret_cast<const float4*>(p.ks + static_cast<size_t>(bhk) * nblk);
-    };
-    auto walk_next = [&](Walk& wk) {
-      if (++wk.it == wk.n_it) {
-        wk.item = sched_item(++wk.k, first_item, item_step);
-        walk_set(wk);
-      }
-    };
-    Walk pre{0, first_item, 0, 0, nullptr, nullptr};
-    walk_set(pre);
+    pre_set();
     uint32_t w_q[kAhead];
     float4 k_q[kAhead];
+    auto request = [&](uint32_t& w, float4& f) {
+      if (pre_item >= n_items) return;
+      if (!All || pre_kind == kDq) {
+        w = reinterpret_cast<const uint32_t*>(p.ds_words)[static_cast<size_t>(pre.ws) * 4 + warp];
+        f = *reinterpret_cast<const float4*>(p.ks + pre.row / 32);
+      } else if (pre_kind == kDk) {
+        const uint4 v = *reinterpret_cast<const uint4*>(p.ds_words + static_cast<size_t>(pre.ws) * 16);
+        const int sh = 8 * warp;
+        w = pack4((v.x >> sh) & 0xFF, (v.y >> sh) & 0xFF, (v.z >> sh) & 0xFF, (v.w >> sh) & 0xFF);
+        f = *reinterpret_cast<const float4*>(p.qs + pre.row / 32);
+      } else {
+        w = reinterpret_cast<const uint32_t*>(p.p_words)[static_cast<size_t>(pre.ws) * 128 + tid];
+        f = make_float4(1.f, 1.f, 1.f, 1.f);
+      }
+      if (--pre_left == 0) {
+        pre_item = sched_item(++pre_k, first_item, item_step);
+        pre_set();
+      } else {
+        pre.next();
+      }
+    };
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       w_q[i] = 0;
       k_q[i] = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (pre.item < n_items) {
-        w_q[i] = pre.w_ptr[4 * pre.it];
-        k_q[i] = pre.ks_ptr[pre.it];
-        walk_next(pre);
-      }
+      request(w_q[i], k_q[i]);
     }
     uint32_t g = 0;
     for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k) {
-      const int qt = n_t - 1 - item / BH;
-      const int n_it = p.causal ? (qt + 1) : n_t;
+      const int n_it = stream_item<All>(p, n_t, item).n_it;
       for (int it = 0; it < n_it; ++it, ++g) {
         const uint32_t w = w_q[0];
         const float4 k4 = k_q[0];
@@ -202,11 +281,7 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
           w_q[i] = w_q[i + 1];
           k_q[i] = k_q[i + 1];
         }
-        if (pre.item < n_items) {
-          w_q[kAhead - 1] = pre.w_ptr[4 * pre.it];
-          k_q[kAhead - 1] = pre.ks_ptr[pre.it];
-          walk_next(pre);
-        }
+        request(w_q[kAhead - 1], k_q[kAhead - 1]);
         const uint32_t word = pack4(sb_mul(w & 0xFF, scale_to_sb(k4.x)), sb_mul((w >> 8) & 0xFF, scale_to_sb(k4.y)),
                                     sb_mul((w >> 16) & 0xFF, scale_to_sb(k4.z)), sb_mul(w >> 24, scale_to_sb(k4.w)));
         const uint32_t st = g % C::kStages;
@@ -228,13 +303,17 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
     bool ok = true;
     uint32_t n_done = 0;
     for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k, ++n_done) {
-      const int qt = n_t - 1 - item / BH, bh = item % BH;
-      const int b = bh / p.H, h = bh % p.H;
+      const StreamItem itm = stream_item<All>(p, n_t, item);
+      const bool kv_item = All && itm.kind != kDq;
+      const int heads = kv_item ? p.Hk : p.H, b = itm.head / heads, h = itm.head % heads;
+      const float mul = kv_item ? 1.0f : p.sm_scale;
       const uint32_t acc = n_done % C::kAccs;
       if (!(ok = wait_warp(dq_full + acc, (n_done / C::kAccs) & 1, abort_flag))) break;
       tc_fence_after();
-      __nv_bfloat16* dst = p.dq + static_cast<int64_t>(b) * p.dq_sb + static_cast<int64_t>(qt * 128 + r) * p.dq_sn +
-                           static_cast<int64_t>(h) * p.dq_sh;
+      const int64_t token = itm.tile * 128 + r;
+      __nv_bfloat16* dst = p.dq + b * p.dq_sb + token * p.dq_sn + h * p.dq_sh;
+      if (All && itm.kind == kDk) dst = p.dk + b * p.dk_sb + token * p.dk_sn + h * p.dk_sh;
+      if (All && itm.kind == kDv) dst = p.dv + b * p.dv_sb + token * p.dv_sn + h * p.dv_sh;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t rr[32];
@@ -243,8 +322,8 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         uint32_t w[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(rr[2 * e]) * p.sm_scale,
-                                                   __uint_as_float(rr[2 * e + 1]) * p.sm_scale);
+          __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(rr[2 * e]) * mul,
+                                                   __uint_as_float(rr[2 * e + 1]) * mul);
           w[e] = *reinterpret_cast<uint32_t*>(&v);
         }
         uint4* d4 = reinterpret_cast<uint4*>(dst + 32 * c);
@@ -262,25 +341,31 @@ bwd_dq_p2_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
   if (warp == 9) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-template <int D>
-static cudaError_t launch_p2_t(const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream) {
+template <int D, bool All>
+static cudaError_t launch_stream_t(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMap& tp, const CUtensorMap& tq,
+                                   const CUtensorMap& tdo, const BwdParams& p, cudaStream_t stream) {
   using C = DqP2Cfg<D>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_dq_p2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_stream_kernel<D, All>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   const int sms = sm_count();
-  const int items = (p.N / 128) * p.B * p.H;
+  const int items = (p.N / 128) * p.B * (p.H + (All ? 2 * p.Hk : 0));
   count_launch();
-  return launch_chained(bwd_dq_p2_kernel<D>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, p);
+  return launch_chained(bwd_stream_kernel<D, All>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, tp, tq, tdo, p);
 }
 
 cudaError_t launch_bwd_dq_p2(int D, const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream) {
-  return D == 128 ? launch_p2_t<128>(tds, tk, p, stream) : launch_p2_t<256>(tds, tk, p, stream);
+  return (D == 128 ? launch_stream_t<128, false> : launch_stream_t<256, false>)(tds, tk, tds, tk, tk, p, stream);   // the last three unused
+}
+
+cudaError_t launch_bwd_stream(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds,
+                              const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream) {
+  return (D == 128 ? launch_stream_t<128, true> : launch_stream_t<256, true>)(tds, tk, tp, tq, tdo, p, stream);
 }
 
 }  // namespace dm

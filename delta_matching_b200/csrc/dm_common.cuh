@@ -19,6 +19,7 @@ enum : int {
   kInDkDv = 3 << 4,
   kInDq = 4 << 4,
   kInDqPass2 = 5 << 4,
+  kInTiles = 6 << 4,
 };
 
 constexpr float kLog2e = 1.4426950408889634f;

@@ -51,6 +51,7 @@ struct BwdParams {
   float* sum_abs_pdp;          // optional (B, H, N): sum_j |P_ij dP_ij|; may be null
   uint8_t* ds_codes;           // optional dS workspace: tile (bh, qt, kt) at ((bh n_t + qt) n_t + kt) x 16384
   uint8_t* ds_words;           // bytes, [key][query] e4m3 codes; then per tile 16 UE8M0 bytes [query block][key block]
+  uint8_t* p_words;            // tile-parallel backward: per tile 512 UE8M0 bytes [key][query block] of the P^T codes, times dO's
   float sm_scale;
   int B, H, Hk, N;
   int causal;
@@ -114,6 +115,11 @@ cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk,
                             cudaStream_t stream);
 cudaError_t launch_bwd_dq(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                           const CUtensorMap& tdo, const BwdParams& p, cudaStream_t stream);
+// Tile-parallel backward: the P^T and dS^T codes of every tile, then dV, dK and dQ streamed from them.
+cudaError_t launch_bwd_tiles(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                             const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream);
+cudaError_t launch_bwd_stream(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds,
+                              const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_dq_p2(int D, const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream);
 // Q, K, V in three launches: [K-mean chunk sums | Q | V], the fold of the chunk sums, K (pk.mean = pm.mean).

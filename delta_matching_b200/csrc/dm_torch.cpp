@@ -39,7 +39,7 @@ struct Lib {
   decltype(&dm_attn_fwd) fwd = nullptr;
   decltype(&dm_attn_bwd) bwd = nullptr;
   decltype(&dm_last_error) last_error = nullptr;
-  decltype(&dm_bwd_workspace_bytes) bwd_workspace_bytes = nullptr;
+  decltype(&dm_attn_bwd_workspace_bytes) bwd_workspace_bytes = nullptr;
   decltype(&dm_quant_qkv_workspace_bytes) quant_workspace_bytes = nullptr;
 } g_lib;
 
@@ -177,7 +177,7 @@ variable_list run_backward(const Tensor& d_o_in, const Tensor& saved, const Tens
   uint8_t* p = static_cast<uint8_t*>(saved.mutable_data_ptr());
   // The dS workspace of the whole call, as long as no bound is set and it is no larger than what ops takes without asking the
   // device how much memory is free; otherwise ops.bwd_fp8 plans the ranges.
-  const int64_t ws_bytes = g_lib.bwd_workspace_bytes(s.B, s.N, s.H, s.D);
+  const int64_t ws_bytes = g_lib.bwd_workspace_bytes(s.B, s.N, s.H, s.Hk, s.D, (flags & kCausal) ? 1 : 0);
   const int64_t n_t = s.N / 128;
   const bool whole = ws_bytes <= g_small_ws && n_t * n_t * s.H * s.B <= g_max_tiles && std::getenv("DM_BWD_WORKSPACE_MB") == nullptr &&
                      std::getenv("DM_BWD_WS_LIMIT_GB") == nullptr;
@@ -327,7 +327,7 @@ PyObject* bind(PyObject*, PyObject* args) {
   g_lib.fwd = reinterpret_cast<decltype(&dm_attn_fwd)>(a[0]);
   g_lib.bwd = reinterpret_cast<decltype(&dm_attn_bwd)>(a[1]);
   g_lib.last_error = reinterpret_cast<decltype(&dm_last_error)>(a[2]);
-  g_lib.bwd_workspace_bytes = reinterpret_cast<decltype(&dm_bwd_workspace_bytes)>(a[3]);
+  g_lib.bwd_workspace_bytes = reinterpret_cast<decltype(&dm_attn_bwd_workspace_bytes)>(a[3]);
   g_lib.quant_workspace_bytes = reinterpret_cast<decltype(&dm_quant_qkv_workspace_bytes)>(a[4]);
   Py_INCREF(sw);
   Py_INCREF(ris);

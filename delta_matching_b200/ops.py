@@ -33,7 +33,8 @@ _DEBUG = os.environ.get("DM_DEBUG", "0") not in ("", "0")
 
 STATUS_TEXT = {1: "TMA producer gave up waiting for a free stage", 2: "MMA issuer gave up waiting",
                3: "compute warps gave up waiting for an accumulator", 4: "probe kernel gave up waiting"}
-STATUS_KERNEL = {1: "forward", 2: "matched delta", 3: "dK/dV", 4: "dQ", 5: "dQ pass 2"}     # v >> 4
+STATUS_KERNEL = {1: "forward", 2: "matched delta", 3: "dK/dV", 4: "dQ", 5: "streaming pass",
+                 6: "tile pass"}     # v >> 4
 
 
 def _ptr(t):

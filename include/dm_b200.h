@@ -35,7 +35,7 @@ extern "C" {
 #define DM_STATUS_TIMEOUT_MMA 2
 #define DM_STATUS_TIMEOUT_COMPUTE 3
 #define DM_STATUS_TIMEOUT_PROBE 4
-/* the low four bits; the bits above name the kernel: 1 forward, 2 matched delta, 3 dK/dV, 4 dQ, 5 dQ pass 2 */
+/* the low four bits; the bits above name the kernel: 1 forward, 2 matched delta, 3 dK/dV, 4 dQ, 5 streaming pass, 6 tile pass */
 
 /* Library identity.  Replaces the build-sanity ops build_gt() / build_hd128() / build_bf16dp() of
  * csrc/delta_matching_api.cpp:683-715: dm_version() is MAJOR * 10000 + MINOR * 100 + PATCH; dm_numerics() names the
@@ -171,8 +171,9 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
 
 /* dm_attn_bwd = dm_quant_do, dm_delta, dm_bwd_ws with parts = 3.  o == NULL: the matched delta (dm_delta, or dm_delta_sum with
  * DM_ATTN_DELTA_SUM); o = the forward's contiguous (B, N, H, D) output: the stale delta.  do8, dos, delta are filled here;
- * dq, dk, dv are contiguous token-major.  flags: DM_DS_BLOCK32, DM_ATTN_DELTA_SUM, DM_ATTN_DELTA_ONLY (stop behind
+ * dq, dk, dv are contiguous token-major.  workspace: dm_attn_bwd_workspace_bytes, 16-byte aligned.  flags: DM_DS_BLOCK32, DM_ATTN_DELTA_SUM, DM_ATTN_DELTA_ONLY (stop behind
  * do8, dos and delta: for callers that split the rest over several dm_bwd_ws calls; dq, dk, dv and workspace are unused). */
+int64_t dm_attn_bwd_workspace_bytes(int B, int N, int H, int Hk, int D, int causal);     /* 0 for a shape the kernels do not take */
 #define DM_ATTN_DELTA_SUM 8
 #define DM_ATTN_DELTA_ONLY 16
 int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, const void* o,

@@ -1,5 +1,5 @@
 """The variants that small problems take, against the forms that large ones take: the producers of a short sequence in one
-launch, dK and dV as two roles.  What a (batch, head) unit computes must not depend on
+launch, dK and dV as two roles, the tile-parallel backward.  What a (batch, head) unit computes must not depend on
 how many units the call has, so the bits of a small call are those of the same units inside a large one."""
 import pytest
 import torch
@@ -17,6 +17,27 @@ def test_short_producers_equal_the_separate_ones(B, N, H, Hk, D, oracle):
     assert torch.equal(km, mean)
     for (codes, scales), (c, s) in (((q8, qs), ops.quant_rows(q, D ** -0.5)), ((k8, ks), ops.quant_rows(k, 1.0, mean)), ((v8, vs), ops.quant_rows(v))):
         assert torch.equal(codes.view(torch.uint8), c.view(torch.uint8)) and torch.equal(scales, s)
+
+
+@pytest.mark.parametrize("B,N,H,Hk,D,causal,mode,numerics", [
+    (1, 256, 2, 2, 128, True, "matched", "sm100-mx"),              # fewer tiles than SMs
+    (1, 1024, 8, 1, 128, True, "matched", "sm100-mx"),             # two or three tiles per CTA, key tiles change inside one
+    (2, 1536, 6, 2, 128, False, "stale", "sm100-mx-ds32"),
+    (1, 4096, 4, 1, 128, True, "stale", "sm100-mx"),               # many tiles per CTA: every ring wraps
+    (1, 128, 3, 1, 256, True, "matched", "sm100-mx"),
+    (1, 1920, 6, 2, 256, False, "stale", "sm100-mx"),
+    (1, 1664, 4, 1, 256, True, "matched", "sm100-mx-d256-ds32"),
+])
+def test_tile_parallel_backward_equals_the_key_stationary_one(B, N, H, Hk, D, causal, mode, numerics, oracle):
+    """dm_attn_func takes the tile-parallel backward for these shapes, the op layer always the key-stationary one."""
+    from delta_matching_b200 import _lib, ops
+    from .helpers import run_api, run_ops
+    assert _lib.lib().dm_attn_bwd_workspace_bytes(B, N, H, Hk, D, int(causal)) > ops.bwd_workspace_bytes(B, N, H, D)
+    q, k, v, do = oracle.make_inputs(B, N, H, Hk, D, seed=73, device="cuda")
+    got = run_api(q, k, v, do, causal, mode, numerics)
+    want = run_ops(q, k, v, do, causal, mode, numerics=numerics)
+    for nm in ("dQ", "dK", "dV"):
+        assert torch.equal(got[nm], want[nm]), nm
 
 
 @pytest.mark.parametrize("N,rep,D,causal,mode,scale", [(256, 1, 128, True, "matched", 1.0), (1280, 3, 128, True, "matched", 4.0), (768, 2, 128, False, "stale", 12.0),
