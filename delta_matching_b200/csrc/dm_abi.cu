@@ -2,6 +2,7 @@
 // no synchronisation.  Validation mirrors the op-level checks of csrc/delta_matching_api.cpp:73-98, 126-148 (device
 // memory, alignment, shape constraints, causal => equal sequence lengths by construction) and reports through
 // dm_last_error instead of TORCH_CHECK.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -279,11 +280,37 @@ static bool tile_parallel(int B, int N, int H, int Hk, int causal) {
   return 10 * chain * dm::sm_count() >= 22 * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
 }
 
+// Workspace of `units` query heads with both tile sets: dS^T tiles, P^T tiles, dS words, P words.
+static int64_t both_tiles_bytes(int64_t heads, int N) {
+  const int64_t n_t = N / 128;
+  return heads * n_t * n_t * (2 * 16384 + 16 + 512);
+}
+
+// Head_dim 256 otherwise: ranges of whole batches, or of kv groups of one batch, whose two tile sets stay within 4 GiB.  Returns
+// the batches and groups of a range (the last ones may be smaller), or false where not even one group fits.
+static bool p_ranges(int B, int N, int H, int Hk, int& batches, int& groups) {
+  const int64_t cap = 4ll << 30, per_group = both_tiles_bytes(H / Hk, N);
+  batches = static_cast<int>(std::min<int64_t>(B, cap / (per_group * Hk)));
+  groups = Hk;
+  if (batches == 0) {
+    batches = 1;
+    groups = static_cast<int>(std::min<int64_t>(Hk, cap / per_group));
+  }
+  if (groups == 0) return false;
+  // ranges as equal as possible
+  const int nb = (B + batches - 1) / batches, ng = (Hk + groups - 1) / groups;
+  batches = (B + nb - 1) / nb;
+  groups = (Hk + ng - 1) / ng;
+  return true;
+}
+
 int64_t dm_attn_bwd_workspace_bytes(int B, int N, int H, int Hk, int D, int causal) {
   const int64_t base = dm_bwd_workspace_bytes(B, N, H, D);
-  if (base == 0 || Hk <= 0 || H % Hk || !tile_parallel(B, N, H, Hk, causal)) return base;
-  const int64_t tiles = static_cast<int64_t>(B) * H * (N / 128) * (N / 128);
-  return tiles * (2 * 16384 + 16 + 512);
+  if (base == 0 || Hk <= 0 || H % Hk) return base;
+  if (tile_parallel(B, N, H, Hk, causal)) return both_tiles_bytes(static_cast<int64_t>(B) * H, N);
+  int batches, groups;
+  if (D == 256 && p_ranges(B, N, H, Hk, batches, groups)) return both_tiles_bytes(static_cast<int64_t>(batches) * groups * (H / Hk), N);
+  return base;
 }
 
 int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, const void* o,
@@ -298,7 +325,9 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   const uint64_t tiles = static_cast<uint64_t>(B) * H * (N / 128) * (N / 128);
   if (kernels && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
     return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed (16-byte aligned)", (long long)workspace_bytes, (long long)need);
-  if (kernels && tiles * 128 >= (1ull << 31))
+  int batches = B, groups = Hk;
+  const bool tile_form = tile_parallel(B, N, H, Hk, causal), p_form = !tile_form && D == 256 && p_ranges(B, N, H, Hk, batches, groups);
+  if (kernels && !p_form && tiles * 128 >= (1ull << 31))
     return fail(DM_ERR_ARG, "delta_matching: B * H * (N / 128)^2 = %llu tiles exceed one workspace (split the heads)", (unsigned long long)tiles);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t hd = static_cast<int64_t>(H) * D, kd = static_cast<int64_t>(Hk) * D;
@@ -325,9 +354,41 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   p.B = B; p.H = H; p.Hk = Hk; p.N = N; p.causal = causal ? 1 : 0; p.status = status;
   p.ds32 = (flags & DM_DS_BLOCK32) ? 1 : 0;
   p.ds_codes = static_cast<uint8_t*>(workspace);
+  if (p_form) {
+    const int rep = H / Hk;
+    for (int b0 = 0; b0 < B; b0 += batches) {
+      for (int g0 = 0; g0 < Hk; g0 += groups) {
+        dm::BwdParams c = p;
+        c.B = std::min(batches, B - b0);
+        c.Hk = std::min(groups, Hk - g0);
+        c.H = c.Hk * rep;
+        const int64_t hq = static_cast<int64_t>(b0) * H + g0 * rep, hkv = static_cast<int64_t>(b0) * Hk + g0;     // heads before the range
+        const int64_t rq = static_cast<int64_t>(c.B) * c.H * N, rk = static_cast<int64_t>(c.B) * c.Hk * N;
+        c.qs += hq * (N / 32); c.dos += hq * (N / 32); c.lse += hq * N; c.delta += hq * N;
+        c.ks += hkv * (N / 32); c.vs += hkv * (N / 32);
+        c.dq += b0 * c.dq_sb + g0 * rep * c.dq_sh;
+        c.dk += b0 * c.dk_sb + g0 * c.dk_sh;
+        c.dv += b0 * c.dv_sb + g0 * c.dv_sh;
+        const int64_t t = static_cast<int64_t>(c.B) * c.H * (N / 128) * (N / 128);
+        c.ds_words = c.ds_codes + t * 2 * 16384;
+        c.p_words = c.ds_words + t * 16;
+        CUtensorMap tp;
+        DM_TRY(make_code_map(&tq, static_cast<const uint8_t*>(q8) + hq * N * D, rq, D));
+        DM_TRY(make_code_map(&tk, static_cast<const uint8_t*>(k8) + hkv * N * D, rk, D));
+        DM_TRY(make_code_map(&tv, static_cast<const uint8_t*>(v8) + hkv * N * D, rk, D));
+        DM_TRY(make_code_map(&td, static_cast<const uint8_t*>(do8) + hq * N * D, rq, D));
+        DM_TRY(make_code_map(&tds, c.ds_codes, t * 128, 128));
+        DM_TRY(make_code_map(&tp, c.ds_codes + t * 16384, t * 128, 128));
+        e = dm::launch_bwd_dk_and_p(tq, tk, tv, td, tds, tp, c, st);
+        if (e != cudaSuccess) return cuda_fail(e, "backward dK launch");
+        e = dm::launch_bwd_stream_dq_dv(tk, td, tds, tp, c, st);
+        if (e != cudaSuccess) return cuda_fail(e, "backward streaming launch");
+      }
+    }
+    return 0;
+  }
   DM_TRY(make_code_map(&tds, workspace, tiles * 128, 128));
-  if (tile_parallel(B, N, H, Hk, causal)) {
-    // workspace: dS^T tiles, P^T tiles, dS words, P words
+  if (tile_form) {
     CUtensorMap tp;
     DM_TRY(make_code_map(&tp, p.ds_codes + tiles * 16384, tiles * 128, 128));
     p.ds_words = p.ds_codes + tiles * 2 * 16384;

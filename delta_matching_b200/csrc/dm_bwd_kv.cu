@@ -29,11 +29,14 @@ namespace dm {
 // With sixteen warps on 32 queries each and one 128-column region that S^T and dP^T shared (what this kernel did before), every
 // link of the chain was exposed and the fixed work of a warp per tile was done sixteen times.
 //
-// Head_dim 256: one accumulator fills 256 columns, so a key tile is two CTAs (and so it is in small grids at head_dim 128): a DV role (S^T, P^T codes, dV; the columns of dP^T
-// are a second S^T buffer, and the words lie beside the codes) and a DK role (S^T, dP^T, dS codes, dK and the dS tiles for
-// the workspace), each with the other half of the work compiled out.
-template <int D, bool DV, bool DK, int G>
+// Head_dim 256: one accumulator fills 256 columns.  Either a key tile is two CTAs (and so it is in small grids at head_dim 128): a
+// DV role (S^T, P^T codes, dV; the columns of dP^T are a second S^T buffer, and the words lie beside the codes) and a DK role
+// (S^T, dP^T, dS codes, dK and the dS tiles for the workspace), each with the other half of the work compiled out.  Or, PO, the DK
+// role also leaves the P^T tiles in the workspace, and dV is streamed from them beside dQ (dm_bwd_p2.cu), which saves the
+// DV role's S^T and exponentials.
+template <int D, bool DV, bool DK, int G, bool PO = false>
 struct KvCfg {
+  static_assert(!PO || (DK && !DV && G == 2), "P^T tiles go out of the DK role");
   static_assert((D == 128 || D == 256) && (DV || DK) && !(D == 256 && DV && DK), "two accumulators of 256 columns fill the TMEM");
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
@@ -53,7 +56,7 @@ struct KvCfg {
   static constexpr int kSmemV = kTileBytes;                          // the DV role has no V tile
   static constexpr int kSmemQ = DK ? 2 * kTileBytes : kTileBytes;    // [kStages]
   static constexpr int kSmemDo = kSmemQ + kStages * kTileBytes;      // [kStages]
-  static constexpr int kSmemWs = kSmemDo + kStages * kTileBytes;     // two staging tiles of dS^T codes
+  static constexpr int kSmemWs = kSmemDo + kStages * kTileBytes;     // two staging tiles of dS^T codes (PO: one, and one of P^T codes)
   static constexpr int kSmemVec = kSmemWs + (DK ? 2 * kCodeBytes : 0);   // [kStages] vectors of the query tile (bytes):
   static constexpr int kVecLse = 0, kVecDelta = 512, kVecQs = 1024, kVecDos = 1040, kVecBytes = 1056;
   static constexpr int kSmemXch = kSmemVec + kStages * kVecBytes;    // [2 parities][8 warps] floats
@@ -79,10 +82,10 @@ __device__ __forceinline__ void store_bf16_row32(const uint32_t (&r)[32], __nv_b
 
 // DS32: the dS scale is taken per (32 queries x 32 keys), which is one 32-column block of one warp, instead of the contract's
 // (128 queries x 32 keys), for which the two warps of a key quadrant exchange their maxima.
-template <int D, bool DV, bool DK, bool DS32, int G>
+template <int D, bool DV, bool DK, bool DS32, int G, bool PO = false>
 __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
-                                          const CUtensorMap& tm_do, const CUtensorMap& tm_ds, const BwdParams& p) {
-  using C = KvCfg<D, DV, DK, G>;
+                                          const CUtensorMap& tm_do, const CUtensorMap& tm_ds, const CUtensorMap& tm_p, const BwdParams& p) {
+  using C = KvCfg<D, DV, DK, G, PO>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemBar);
   uint64_t* bar_kv = bars + 0;       // K and V landed
@@ -99,6 +102,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
   uint64_t* full_d = bars + 12;      // [kStages] dO landed
   uint64_t* vec_ok = bars + 16;      // [kStages] the vectors landed and -lse * log2e is written
   uint64_t* empty = bars + 20;       // [kStages] the chains of the stage's tile are done (MMA commit)
+  uint64_t* bar_po = bars + 27;      // PO: P^T codes of the tile in their staging tile (one arrival per compute warp)
+  uint64_t* po_free = bars + 28;     // PO: they have been read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 25);
 
@@ -124,6 +129,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
     mbar_init(bar_k, C::kComputeWarps);
     mbar_init(bar_done, 1);
     mbar_init(bar_acc, 1);
+    mbar_init(bar_po, C::kComputeWarps);
+    mbar_init(po_free, 1);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(full_q + s, 1);
       mbar_init(full_d + s, 1);
@@ -198,6 +205,26 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       if (lane == 0) mbar_arrive(vec_ok + st);
     }
     if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDkDv);
+  } else if (PO && warp == C::kComputeWarps + 3) {
+    // ------------------------------------------------------------------------------------------ P^T store warp
+    if (elect_one()) {
+      bool ok = true;
+      int row = (((b * p.H + hk * rep) * n_t + qt0) * n_t + kt) * 128, left = n_qi;
+      for (int i = 0; i < n_it; ++i) {
+        if (!(ok = wait_or_abort(bar_po, i & 1, abort_flag))) break;
+        tma_store_2d(&tm_p, smem + C::kSmemWs + C::kCodeBytes, 0, row);
+        bulk_commit_group();
+        bulk_wait_group_read<0>();
+        mbar_arrive(po_free);
+        row += 128 * n_t;
+        if (--left == 0) {
+          left = n_qi;
+          row += 128 * n_t * qt0;
+        }
+      }
+      bulk_wait_group<0>();
+      if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutProducer + kInDkDv);
+    }
   } else if (warp == C::kComputeWarps) {
     // ------------------------------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop (uniform values stay in uniform registers), one elected thread issues.
@@ -282,7 +309,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           tc_commit(empty + i % C::kStages);
           if (i == n_it - 1) tc_commit(bar_acc);
           if (p.ds_codes != nullptr) {                   // the dS^T codes of the tile, from its staging tile, to the workspace
-            tma_store_2d(&tm_ds, smem + C::kSmemWs + (i & 1) * C::kCodeBytes, 0, ws_row);
+            tma_store_2d(&tm_ds, smem + C::kSmemWs + (PO ? 0 : (i & 1) * C::kCodeBytes), 0, ws_row);
             bulk_commit_group();
           }
         }
@@ -294,7 +321,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         if (i + 1 < n_it) {
           // the scale words of these chains lie where dP^T of the next tile lands
           if (!(ok = wait_warp(bar_done, ph, abort_flag))) break;
-          bulk_wait_group_read<1>();                     // tile i + 1 writes its codes where those of tile i - 1 were
+          bulk_wait_group_read<PO ? 0 : 1>();            // tile i + 1 writes its codes where those of tile i - 1 (PO: i) were
           if (!(ok = issue_dp(i + 1))) break;
         }
       }
@@ -354,22 +381,28 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         for (int c = 0; c < CH; ++c) {
           const float2 cc = splat2((ks_row * (c ? qs2.y : qs2.x)) * kLog2e);
           float pm0 = 0.f, pm1 = 0.f;
+          if (PO && c == 0 && i > 0) ok = wait_warp(po_free, ph ^ 1, abort_flag);
 #pragma unroll
           for (int e = 0; e < 16; e += 2) {
             const float4 l4 = lds_f4(va + C::kVecLse + 128 * c + 8 * e);     // -lse * log2e
             pr[c][e] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e]), __uint_as_float(rs[c][2 * e + 1])), cc, make_float2(l4.x, l4.y)));
             pr[c][e + 1] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e + 2]), __uint_as_float(rs[c][2 * e + 3])), cc, make_float2(l4.z, l4.w)));
-            if (DV) {
+            if (DV || PO) {
               pm0 = max3(pm0, pr[c][e].x, pr[c][e].y);
               pm1 = max3(pm1, pr[c][e + 1].x, pr[c][e + 1].y);
             }
           }
-          if (DV) {
+          if (DV || PO) {
             // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread and block
             const uint32_t psb = pow2_sb(fmaxf(pm0, pm1), 0u);
             uint32_t w[8];
             codes32(pr[c], sb_to_inv(psb), w);
-            tmem_st8(t_s + C::kColCodes + 8 * c, w);
+            if (DV) tmem_st8(t_s + C::kColCodes + 8 * c, w);
+            if (PO) {                                      // as a [key][query] tile, like the dS^T codes below
+              const int j = 2 * CH * half + 2 * c;
+              sts_u4(ws_a + C::kCodeBytes + ((j ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+              sts_u4(ws_a + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
+            }
             xv |= sb_mul(psb, scale_to_sb(c ? dos2.y : dos2.x)) << (8 * c);
           }
         }
@@ -381,6 +414,11 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           __syncwarp();
           if ((tid & 31) == 0) mbar_arrive(ph ? bar_p1 : bar_p);
         }
+      }
+      if (PO && ok) {
+        fence_async_smem();
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(bar_po);
       }
       float am[2] = {0.f, 0.f};
       if (DK && ok) ok = wait_warp(bar_dp, ph, abort_flag);
@@ -436,7 +474,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
             for (int g = 1; g < G; ++g) mx = fmaxf(mx, lds_f(xch_a + 4 * (ph * 16 + 4 * g + quad)));
             dsb[0] = dsb[1] = pow2_sb(mx, 127u);
           }
-          const uint32_t ws_row = ws_a + ph * C::kCodeBytes;
+          const uint32_t ws_row = ws_a + (PO ? 0 : ph * C::kCodeBytes);
 #pragma unroll
           for (int c = 0; c < CH; ++c) {
             uint32_t w[8];
@@ -464,6 +502,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           tc_fence_before();
           __syncwarp();
           if ((tid & 31) == 0) mbar_arrive(bar_k);
+          if (PO)                                          // dV scale bytes of the tile, [key][query block]
+            *reinterpret_cast<uint16_t*>(p.p_words + static_cast<size_t>(ws_tile) * 512 + r * 4 + 2 * half) = static_cast<uint16_t>(xv);
         }
       }
       ws_tile += n_t;
@@ -507,53 +547,62 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
 constexpr int kKvGroups = 2;       // compute warpgroups (8 warps): with four, each warp's fixed work per tile is done sixteen times
                                    // (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256 the two are equal
 
-template <int D, bool Roles>
+// How dK and dV of a key tile are made: by one CTA; by two, both kinds in one grid, the longer one (dK) first; or dK here and dV
+// from the P^T tiles that the launch leaves in the workspace.
+enum KvForm { kKvOne, kKvRoles, kKvDkAndP };
+
+template <int D, int Form>
 struct KvLaunch {
-  using Dk = KvCfg<D, !Roles, true, kKvGroups>;
-  using Dv = KvCfg<D, true, !Roles, kKvGroups>;
+  using Dk = KvCfg<D, Form == kKvOne, true, kKvGroups, Form == kKvDkAndP>;
+  using Dv = KvCfg<D, true, Form == kKvOne, kKvGroups>;
   static constexpr int kThreads = Dk::kThreads;
   static constexpr int kSmemBytes = Dk::kSmemBytes > Dv::kSmemBytes ? Dk::kSmemBytes : Dv::kSmemBytes;
 };
 
-// Roles: dK and dV of a key tile by two CTAs, both kinds in one grid, the longer one (dK) first.
-template <int D, bool Roles, bool DS32>
-__global__ void __launch_bounds__(KvLaunch<D, Roles>::kThreads, 1)
+template <int D, int Form, bool DS32>
+__global__ void __launch_bounds__(KvLaunch<D, Form>::kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
-  if constexpr (!Roles) dkdv_tile<D, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
-  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
-  else dkdv_tile<D, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, p);
+                const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_p, const BwdParams p) {
+  if constexpr (Form == kKvOne) dkdv_tile<D, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else if constexpr (Form == kKvDkAndP) dkdv_tile<D, false, true, DS32, kKvGroups, true>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else dkdv_tile<D, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
 }
 
-template <int D, bool Roles, bool DS32>
+template <int D, int Form, bool DS32>
 static cudaError_t launch_kv_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                               const CUtensorMap& tds, const BwdParams& p, cudaStream_t stream) {
-  using L = KvLaunch<D, Roles>;
+                               const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream) {
+  using L = KvLaunch<D, Form>;
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, Roles, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, Form, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) return e;
     done[dev] = true;
   }
-  const dim3 grid(p.B * p.Hk, p.N / 128, Roles ? 2 : 1);
+  const dim3 grid(p.B * p.Hk, p.N / 128, Form == kKvRoles ? 2 : 1);
   count_launch();
-  return launch_chained(bwd_dkdv_kernel<D, Roles, DS32>, grid, L::kThreads, L::kSmemBytes, stream, tq, tk, tv, tdo, tds, p);
+  return launch_chained(bwd_dkdv_kernel<D, Form, DS32>, grid, L::kThreads, L::kSmemBytes, stream, tq, tk, tv, tdo, tds, tp, p);
 }
 
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const CUtensorMap& tdo, const CUtensorMap* tds_or_null, const BwdParams& p,
                             cudaStream_t stream) {
   const CUtensorMap& tds = (tds_or_null != nullptr) ? *tds_or_null : tq;     // unused by the kernel without a workspace
-  // Head_dim 256 has no choice.  At head_dim 128 the roles cost a second S^T and a second exponential per element, so they
-  // are for grids that leave half of the SMs without a CTA: each role's chain per tile is the shorter one then (the same
-  // bits: the accumulators do not depend on each other).
-  if (D != 128) return (p.ds32 ? launch_kv_t<256, true, true> : launch_kv_t<256, true, false>)(tq, tk, tv, tdo, tds, p, stream);
+  // At head_dim 128 the roles cost a second S^T and a second exponential per element, so they are for grids that leave half of
+  // the SMs without a CTA: each role's chain per tile is the shorter one then (the same bits: the accumulators do not
+  // depend on each other).
+  if (D != 128) return (p.ds32 ? launch_kv_t<256, kKvRoles, true> : launch_kv_t<256, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
   if (2ll * p.B * p.Hk * (p.N / 128) <= sm_count())
-    return (p.ds32 ? launch_kv_t<128, true, true> : launch_kv_t<128, true, false>)(tq, tk, tv, tdo, tds, p, stream);
-  return (p.ds32 ? launch_kv_t<128, false, true> : launch_kv_t<128, false, false>)(tq, tk, tv, tdo, tds, p, stream);
+    return (p.ds32 ? launch_kv_t<128, kKvRoles, true> : launch_kv_t<128, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
+  return (p.ds32 ? launch_kv_t<128, kKvOne, true> : launch_kv_t<128, kKvOne, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
+}
+
+cudaError_t launch_bwd_dk_and_p(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream) {
+  return (p.ds32 ? launch_kv_t<256, kKvDkAndP, true> : launch_kv_t<256, kKvDkAndP, false>)(tq, tk, tv, tdo, tds, tp, p, stream);
 }
 
 }  // namespace dm

@@ -11,7 +11,7 @@
 // dS blocks of 128 queries x 32 keys the four words of a tile are equal; with 32 x 32 blocks they differ.  The tile is the A operand of dQ in MN-major form
 // (M = queries contiguous); K is the B operand in MN-major form as in the other kernels.
 //
-// Behind the tile-parallel pass (dm_bwd_tiles.cu) the same kernel, with All, also makes dV = sum P^T dO and dK = sum dS^T Q of
+// Behind the tile-parallel pass (dm_bwd_tiles.cu) the same kernel also makes dV = sum P^T dO and dK = sum dS^T Q of
 // every (key tile, kv head), over the group's heads and their query tiles in the order of the key-stationary kernel: there
 // the code tile is the A operand as it lies, K-major (M = keys), and dO / Q the MN-major B operand.
 //
@@ -46,23 +46,27 @@ struct DqP2Cfg {
 };
 
 // A work item: one accumulator.  kDq: (head, query tile), over key tiles.  kDk, kDv: (kv head, key tile), over (head of the
-// group, query tile).  With All, dK and dV of all key tiles come first, the most tiles first, then dQ likewise.
+// group, query tile).  dK and dV of all key tiles come first, the most tiles first, then dQ likewise.
 enum : int { kDq = 0, kDk = 1, kDv = 2 };
+enum : int { kOnlyDq = 0, kDqDkDv = 1, kDqDv = 2 };      // Kinds of items in a launch
 struct StreamItem {
   int kind, head, tile;        // head: query head (kDq) or kv head; tile: query tile or key tile
   int n_it, first, per_head;   // tiles; kDk, kDv: first query tile, query tiles per head
 };
-template <bool All>
+template <int Kinds>
 __device__ __forceinline__ int stream_item_count(const BwdParams& p, int n_t) {
-  return n_t * p.B * (p.H + (All ? 2 * p.Hk : 0));
+  return n_t * p.B * (p.H + (Kinds == kDqDkDv ? 2 * p.Hk : Kinds == kDqDv ? p.Hk : 0));
 }
-template <bool All>
+template <int Kinds>
 __device__ __forceinline__ StreamItem stream_item(const BwdParams& p, int n_t, int item) {
   StreamItem r;
-  const int BH = p.B * p.H, BHk = p.B * p.Hk, kv_items = All ? 2 * n_t * BHk : 0;
-  if (All && item < kv_items) {
-    r.kind = kDk + (item & 1);
-    item >>= 1;
+  const int BH = p.B * p.H, BHk = p.B * p.Hk, kv_items = Kinds == kDqDkDv ? 2 * n_t * BHk : Kinds == kDqDv ? n_t * BHk : 0;
+  if (item < kv_items) {
+    r.kind = kDv;
+    if (Kinds == kDqDkDv) {
+      r.kind = kDk + (item & 1);
+      item >>= 1;
+    }
     r.tile = item / BHk;
     r.head = item % BHk;
     r.first = p.causal ? r.tile : 0;
@@ -80,12 +84,12 @@ __device__ __forceinline__ StreamItem stream_item(const BwdParams& p, int n_t, i
   return r;
 }
 // Position inside an item: the tile's index in the workspace and its B operand's row (K, Q or dO codes).
-template <bool All>
+template <int Kinds>
 struct StreamWalk {
   int ws, ws_step, row, left, per_head, ws_wrap, row_wrap;
   __device__ __forceinline__ void set(const BwdParams& p, int n_t, const StreamItem& it) {
     const int rep = p.H / p.Hk;
-    if (!All || it.kind == kDq) {
+    if (Kinds == kOnlyDq || it.kind == kDq) {
       ws = (it.head * n_t + it.tile) * n_t;
       ws_step = 1;
       row = ((it.head / p.H) * p.Hk + (it.head % p.H) / rep) * p.N;
@@ -103,7 +107,7 @@ struct StreamWalk {
   __device__ __forceinline__ void next() {
     ws += ws_step;
     row += 128;
-    if (All && --left == 0) {
+    if (Kinds != kOnlyDq && --left == 0) {
       left = per_head;
       ws += ws_wrap;
       row += row_wrap;
@@ -111,7 +115,7 @@ struct StreamWalk {
   }
 };
 
-template <int D, bool All>
+template <int D, int Kinds>
 __global__ void __launch_bounds__(DqP2Cfg<D>::kThreads, 1)
 bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_q,
@@ -135,7 +139,7 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int n_t = p.N / 128;
-  const int n_items = stream_item_count<All>(p, n_t);
+  const int n_items = stream_item_count<Kinds>(p, n_t);
   const int first_item = static_cast<int>(blockIdx.x), item_step = static_cast<int>(gridDim.x);
 
   if (tid == 0) {
@@ -168,11 +172,11 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
       bool ok = true;
       uint32_t g = 0;
       for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k) {
-        const StreamItem itm = stream_item<All>(p, n_t, item);
-        StreamWalk<All> wk;
+        const StreamItem itm = stream_item<Kinds>(p, n_t, item);
+        StreamWalk<Kinds> wk;
         wk.set(p, n_t, itm);
-        const CUtensorMap* ta = (All && itm.kind == kDv) ? &tm_p : &tm_ds;
-        const CUtensorMap* tb = !All || itm.kind == kDq ? &tm_k : itm.kind == kDk ? &tm_q : &tm_do;
+        const CUtensorMap* ta = (Kinds != kOnlyDq && itm.kind == kDv) ? &tm_p : &tm_ds;
+        const CUtensorMap* tb = Kinds == kOnlyDq || itm.kind == kDq ? &tm_k : itm.kind == kDk ? &tm_q : &tm_do;
         for (int it = 0; it < itm.n_it; ++it, ++g, wk.next()) {
           const uint32_t st = g % C::kStages;
           if (g >= C::kStages && !(ok = wait_or_abort(empty + st, ((g / C::kStages) - 1) & 1, abort_flag))) break;
@@ -191,9 +195,9 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
       bool ok = true;
       uint32_t g = 0, n_done = 0;
       for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k, ++n_done) {
-        const StreamItem itm = stream_item<All>(p, n_t, item);
+        const StreamItem itm = stream_item<Kinds>(p, n_t, item);
         const int n_it = itm.n_it;
-        const bool kv_item = All && itm.kind != kDq;
+        const bool kv_item = Kinds != kOnlyDq && itm.kind != kDq;
         const uint32_t a_step = kv_item ? 2 : 256, idesc = kv_item ? idesc_mxf8(128, 128, false, true, 0, 0) : idesc_mxf8(128, 128, true, true, 0, 0);
         const uint32_t acc = n_done % C::kAccs;
         // the accumulator was last used kAccs items ago: its read-out must be complete
@@ -232,10 +236,10 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
     //   dV: this row's own word, finished
     constexpr int kAhead = 4;
     int pre_k = 0, pre_item = first_item, pre_left = 0, pre_kind = kDq;
-    StreamWalk<All> pre;
+    StreamWalk<Kinds> pre;
     auto pre_set = [&]() {
       if (pre_item >= n_items) return;
-      const StreamItem itm = stream_item<All>(p, n_t, pre_item);
+      const StreamItem itm = stream_item<Kinds>(p, n_t, pre_item);
       pre.set(p, n_t, itm);
       pre_left = itm.n_it;
       pre_kind = itm.kind;
@@ -245,7 +249,7 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
     float4 k_q[kAhead];
     auto request = [&](uint32_t& w, float4& f) {
       if (pre_item >= n_items) return;
-      if (!All || pre_kind == kDq) {
+      if (Kinds == kOnlyDq || pre_kind == kDq) {
         w = reinterpret_cast<const uint32_t*>(p.ds_words)[static_cast<size_t>(pre.ws) * 4 + warp];
         f = *reinterpret_cast<const float4*>(p.ks + pre.row / 32);
       } else if (pre_kind == kDk) {
@@ -272,7 +276,7 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
     }
     uint32_t g = 0;
     for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k) {
-      const int n_it = stream_item<All>(p, n_t, item).n_it;
+      const int n_it = stream_item<Kinds>(p, n_t, item).n_it;
       for (int it = 0; it < n_it; ++it, ++g) {
         const uint32_t w = w_q[0];
         const float4 k4 = k_q[0];
@@ -303,8 +307,8 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
     bool ok = true;
     uint32_t n_done = 0;
     for (int k = 0, item; ok && (item = sched_item(k, first_item, item_step)) < n_items; ++k, ++n_done) {
-      const StreamItem itm = stream_item<All>(p, n_t, item);
-      const bool kv_item = All && itm.kind != kDq;
+      const StreamItem itm = stream_item<Kinds>(p, n_t, item);
+      const bool kv_item = Kinds != kOnlyDq && itm.kind != kDq;
       const int heads = kv_item ? p.Hk : p.H, b = itm.head / heads, h = itm.head % heads;
       const float mul = kv_item ? 1.0f : p.sm_scale;
       const uint32_t acc = n_done % C::kAccs;
@@ -312,8 +316,8 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
       tc_fence_after();
       const int64_t token = itm.tile * 128 + r;
       __nv_bfloat16* dst = p.dq + b * p.dq_sb + token * p.dq_sn + h * p.dq_sh;
-      if (All && itm.kind == kDk) dst = p.dk + b * p.dk_sb + token * p.dk_sn + h * p.dk_sh;
-      if (All && itm.kind == kDv) dst = p.dv + b * p.dv_sb + token * p.dv_sn + h * p.dv_sh;
+      if (Kinds != kOnlyDq && itm.kind == kDk) dst = p.dk + b * p.dk_sb + token * p.dk_sn + h * p.dk_sh;
+      if (Kinds != kOnlyDq && itm.kind == kDv) dst = p.dv + b * p.dv_sb + token * p.dv_sn + h * p.dv_sh;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t rr[32];
@@ -341,7 +345,7 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
   if (warp == 9) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-template <int D, bool All>
+template <int D, int Kinds>
 static cudaError_t launch_stream_t(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMap& tp, const CUtensorMap& tq,
                                    const CUtensorMap& tdo, const BwdParams& p, cudaStream_t stream) {
   using C = DqP2Cfg<D>;
@@ -349,23 +353,28 @@ static cudaError_t launch_stream_t(const CUtensorMap& tds, const CUtensorMap& tk
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_stream_kernel<D, All>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_stream_kernel<D, Kinds>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   const int sms = sm_count();
-  const int items = (p.N / 128) * p.B * (p.H + (All ? 2 * p.Hk : 0));
+  const int items = (p.N / 128) * p.B * (p.H + (Kinds == kDqDkDv ? 2 * p.Hk : Kinds == kDqDv ? p.Hk : 0));
   count_launch();
-  return launch_chained(bwd_stream_kernel<D, All>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, tp, tq, tdo, p);
+  return launch_chained(bwd_stream_kernel<D, Kinds>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tds, tk, tp, tq, tdo, p);
 }
 
 cudaError_t launch_bwd_dq_p2(int D, const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream) {
-  return (D == 128 ? launch_stream_t<128, false> : launch_stream_t<256, false>)(tds, tk, tds, tk, tk, p, stream);   // the last three unused
+  return (D == 128 ? launch_stream_t<128, kOnlyDq> : launch_stream_t<256, kOnlyDq>)(tds, tk, tds, tk, tk, p, stream);   // the last three unused
 }
 
 cudaError_t launch_bwd_stream(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds,
                               const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream) {
-  return (D == 128 ? launch_stream_t<128, true> : launch_stream_t<256, true>)(tds, tk, tp, tq, tdo, p, stream);
+  return (D == 128 ? launch_stream_t<128, kDqDkDv> : launch_stream_t<256, kDqDkDv>)(tds, tk, tp, tq, tdo, p, stream);
+}
+
+cudaError_t launch_bwd_stream_dq_dv(const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds, const CUtensorMap& tp,
+                                    const BwdParams& p, cudaStream_t stream) {
+  return launch_stream_t<256, kDqDv>(tds, tk, tp, tk, tdo, p, stream);
 }
 
 }  // namespace dm

@@ -120,6 +120,11 @@ cudaError_t launch_bwd_tiles(int D, const CUtensorMap& tq, const CUtensorMap& tk
                              const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_stream(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds,
                               const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream);
+// Head_dim 256: dK, the dS^T and the P^T tiles; then dV and dQ streamed from them.
+cudaError_t launch_bwd_dk_and_p(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream);
+cudaError_t launch_bwd_stream_dq_dv(const CUtensorMap& tk, const CUtensorMap& tdo, const CUtensorMap& tds, const CUtensorMap& tp,
+                                    const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_dq_p2(int D, const CUtensorMap& tds, const CUtensorMap& tk, const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream);
 // Q, K, V in three launches: [K-mean chunk sums | Q | V], the fold of the chunk sums, K (pk.mean = pm.mean).
