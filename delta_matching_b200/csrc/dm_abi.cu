@@ -273,11 +273,12 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
 // (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.7 us a tile; the tile-parallel
 // pair takes its share of all tiles at about 3.7 us.  Forward + backward, chain / tiles per SM: 16 (N=1024 H=8 Hk=2) 92 -> 60 us;
 // 4.6 (N=8192 H=4 Hk=1) 594 -> 440; 2.3 (N=16384 H=2 Hk=1) 810 -> 758; 2.2 (N=2048 H=32 Hk=8) 222 -> 214; 2.05 (B=4 N=1024 H=16 Hk=4) 140 ->
-// 140; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  The line is drawn at 2.2, and at 2 GiB of workspace.
-static bool tile_parallel(int B, int N, int H, int Hk, int causal) {
+// 140; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  Head_dim 256: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152 -> 143; 1.45
+// (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 -> 495.  The lines are drawn at 2.2 and 1.6, and at 2 GiB of workspace.
+static bool tile_parallel(int B, int N, int H, int Hk, int D, int causal) {
   const long long n_t = N / 128, tiles = static_cast<long long>(B) * H * (causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
   const long long chain = H / Hk * n_t;
-  return 10 * chain * dm::sm_count() >= 22 * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
+  return 10 * chain * dm::sm_count() >= (D == 128 ? 22 : 16) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
 }
 
 // Workspace of `units` query heads with both tile sets: dS^T tiles, P^T tiles, dS words, P words.
@@ -307,7 +308,7 @@ static bool p_ranges(int B, int N, int H, int Hk, int& batches, int& groups) {
 int64_t dm_attn_bwd_workspace_bytes(int B, int N, int H, int Hk, int D, int causal) {
   const int64_t base = dm_bwd_workspace_bytes(B, N, H, D);
   if (base == 0 || Hk <= 0 || H % Hk) return base;
-  if (tile_parallel(B, N, H, Hk, causal)) return both_tiles_bytes(static_cast<int64_t>(B) * H, N);
+  if (tile_parallel(B, N, H, Hk, D, causal)) return both_tiles_bytes(static_cast<int64_t>(B) * H, N);
   int batches, groups;
   if (D == 256 && p_ranges(B, N, H, Hk, batches, groups)) return both_tiles_bytes(static_cast<int64_t>(batches) * groups * (H / Hk), N);
   return base;
@@ -326,7 +327,7 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   if (kernels && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
     return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed (16-byte aligned)", (long long)workspace_bytes, (long long)need);
   int batches = B, groups = Hk;
-  const bool tile_form = tile_parallel(B, N, H, Hk, causal), p_form = !tile_form && D == 256 && p_ranges(B, N, H, Hk, batches, groups);
+  const bool tile_form = tile_parallel(B, N, H, Hk, D, causal), p_form = !tile_form && D == 256 && p_ranges(B, N, H, Hk, batches, groups);
   if (kernels && !p_form && tiles * 128 >= (1ull << 31))
     return fail(DM_ERR_ARG, "delta_matching: B * H * (N / 128)^2 = %llu tiles exceed one workspace (split the heads)", (unsigned long long)tiles);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
