@@ -11,8 +11,9 @@
 // ctypes handle, so that DM_SO decides for both which library runs.  attn() returns None whenever a call is not one it
 // serves as it stands (a violated constraint, a tensor subclass, a functorch or dispatch-mode wrapper); the caller then
 // takes the Python route, which raises the contract's exceptions or serves the call.
-#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
@@ -32,7 +33,7 @@
 namespace {
 
 using at::Tensor;
-using torch::autograd::AutogradContext;
+using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
 struct Lib {
@@ -101,10 +102,11 @@ Tensor bf16_on(at::IntArrayRef size, const at::Device& dev) {
   return Tensor(at::detail::empty_cuda(size, at::kBFloat16, dev, std::nullopt));
 }
 
-// What the backward reads: codes and scales of q, k, v and the LSE.
+// What the backward reads: codes and scales of q, k, v and the LSE; and the scratch of the K mean, which is small (a sixteenth
+// of K's codes) and not worth an allocation of its own.
 struct Saved {
   Carve c;
-  int64_t q8, k8, v8, qs, ks, vs, lse;
+  int64_t q8, k8, v8, qs, ks, vs, lse, mean, part;
   explicit Saved(const Shape& s) {
     q8 = c.take(s.rows_q() * s.D);
     k8 = c.take(s.rows_k() * s.D);
@@ -113,6 +115,8 @@ struct Saved {
     ks = c.take(s.rows_k() / 8);
     vs = c.take(s.rows_k() / 8);
     lse = c.take(s.rows_q() * 4);
+    mean = c.take(static_cast<int64_t>(s.B) * s.Hk * s.D * 4);
+    part = c.take(static_cast<int64_t>(g_lib.quant_workspace_bytes(s.B, s.N, s.Hk, s.D)));
   }
 };
 
@@ -147,20 +151,14 @@ Tensor run_forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, c
   const Tensor q = rows(q_in), k = rows(k_in), v = rows(v_in);
   const bool hm = (flags & kHeadMajor) != 0;
   const Strides sq(q, hm), sk(k, hm), sv(v, hm);
-  Saved L(s);
-  const int64_t kept = L.c.size();
-  const int64_t mean = L.c.take(static_cast<int64_t>(s.B) * s.Hk * s.D * 4);
-  const int64_t part = L.c.take(static_cast<int64_t>(g_lib.quant_workspace_bytes(s.B, s.N, s.Hk, s.D)));
-  // a forward whose codes are kept leaves the scratch of the K mean out of the kept buffer
-  Tensor saved = bytes_on(saved_out ? kept : L.c.size(), dev);
-  Tensor scratch = saved_out ? bytes_on(L.c.size() - kept, dev) : saved;
+  const Saved L(s);
+  Tensor saved = bytes_on(L.c.size(), dev);
   uint8_t* p = static_cast<uint8_t*>(saved.mutable_data_ptr());
-  uint8_t* t = static_cast<uint8_t*>(scratch.mutable_data_ptr()) - (saved_out ? kept : 0);
   Tensor o = bf16_on({s.B, s.N, s.H, s.D}, dev);
   check(g_lib.fwd(q.const_data_ptr(), sq.b, sq.h, sq.n, k.const_data_ptr(), sk.b, sk.h, sk.n, v.const_data_ptr(), sv.b, sv.h, sv.n,
                   s.B, s.N, s.H, s.Hk, s.D, (flags & kCausal) ? 1 : 0, p + L.q8, p + L.k8, p + L.v8,
                   reinterpret_cast<float*>(p + L.qs), reinterpret_cast<float*>(p + L.ks), reinterpret_cast<float*>(p + L.vs),
-                  reinterpret_cast<float*>(t + mean), t + part, o.mutable_data_ptr(), reinterpret_cast<float*>(p + L.lse), status,
+                  reinterpret_cast<float*>(p + L.mean), p + L.part, o.mutable_data_ptr(), reinterpret_cast<float*>(p + L.lse), status,
                   c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
   if (saved_out) *saved_out = std::move(saved);
   return o;
@@ -220,28 +218,28 @@ variable_list run_backward(const Tensor& d_o_in, const Tensor& saved, const Tens
   return {dq, dk, dv};
 }
 
-struct Attn : public torch::autograd::Function<Attn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, int64_t flags) {
-    const bool hm = (flags & kHeadMajor) != 0;
-    const Shape s{static_cast<int>(q.size(0)), static_cast<int>(q.size(hm ? 2 : 1)), static_cast<int>(q.size(hm ? 1 : 2)),
-                  static_cast<int>(k.size(hm ? 1 : 2)), static_cast<int>(q.size(3))};
-    Tensor saved;
-    Tensor o = run_forward(q, k, v, s, flags, &saved);
-    ctx->save_for_backward((flags & kMatched) ? variable_list{saved} : variable_list{saved, o});   // the matched delta never reads O
-    ctx->saved_data["shape"] = (static_cast<int64_t>(s.B) << 32) | (static_cast<int64_t>(s.H) << 16) | s.Hk;     // each below 2^16
-    ctx->saved_data["size"] = (static_cast<int64_t>(s.N) << 16) | (static_cast<int64_t>(s.D) << 5) | flags;
-    return o;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const int64_t a = ctx->saved_data["shape"].toInt(), b = ctx->saved_data["size"].toInt(), flags = b & 31;
-    const Shape s{static_cast<int>(a >> 32), static_cast<int>(b >> 16), static_cast<int>((a >> 16) & 0xFFFF), static_cast<int>(a & 0xFFFF),
-                  static_cast<int>((b >> 5) & 0x7FF)};
-    const bool twice = at::GradMode::is_enabled() && grads[0].requires_grad();
+Shape shape_of(const Tensor& q, const Tensor& k, int64_t flags) {
+  const bool hm = (flags & kHeadMajor) != 0;
+  return {static_cast<int>(q.size(0)), static_cast<int>(q.size(hm ? 2 : 1)), static_cast<int>(q.size(hm ? 1 : 2)),
+          static_cast<int>(k.size(hm ? 1 : 2)), static_cast<int>(q.size(3))};
+}
+
+// The autograd node.  (torch::autograd::Function would do, at some 4 us more per forward + backward for its context, the map of
+// saved values and the generic wrapping of inputs and outputs.)
+struct AttnBackward : public torch::autograd::Node {
+  SavedVariable saved, o;       // o: stale delta only, the matched delta never reads O
+  Shape s;
+  int64_t flags = 0;
+
+  variable_list apply(variable_list&& grads) override {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor d_o = grads[0].defined() ? grads[0] : input_metadata(0).zeros_like();
+    const bool twice = at::GradMode::is_enabled() && d_o.requires_grad();
     variable_list g;
     {
       const at::AutoGradMode no_grad(false);
-      g = run_backward(grads[0], saved[0], saved.size() > 1 ? saved[1] : Tensor(), s, flags);
+      const Tensor buffer = saved.unpack();
+      g = run_backward(d_o, buffer, (flags & kMatched) ? Tensor() : o.unpack(shared_from_this()), s, flags);
       if (flags & kHeadMajor)
         for (Tensor& t : g) t = t.permute({0, 2, 1, 3});
     }
@@ -250,10 +248,32 @@ struct Attn : public torch::autograd::Function<Attn> {
       g = torch::autograd::DelayedError("trying to differentiate twice a function that was marked with @once_differentiable", 3)
               .apply(std::move(g));
     }
-    g.emplace_back();
     return g;
   }
+  void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    saved.reset_data();
+    o.reset_data();
+  }
+  std::string name() const override { return "DeltaMatchingAttnBackward"; }
 };
+
+Tensor with_graph(const Tensor& q, const Tensor& k, const Tensor& v, int64_t flags) {
+  const Shape s = shape_of(q, k, flags);
+  Tensor buffer, o;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    o = run_forward(q, k, v, s, flags, &buffer);
+  }
+  std::shared_ptr<AttnBackward> node(new AttnBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+  node->s = s;
+  node->flags = flags;
+  torch::autograd::set_history(o, node);
+  node->saved = SavedVariable(buffer, false);
+  if (!(flags & kMatched)) node->o = SavedVariable(o, true);
+  return o;
+}
 
 // (ds32, norm) of a numerics arm, or -1 for a name that is none at this head_dim (ops.NUMERICS, attn._numerics).
 int64_t numerics_flags(PyObject* name, int64_t D) {
@@ -307,11 +327,10 @@ PyObject* attn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     pybind11::gil_scoped_release no_gil;
     if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
-      o = Attn::apply(q, k, v, flags);
+      o = with_graph(q, k, v, flags);
     } else {
-      const Shape s{static_cast<int>(B), static_cast<int>(N), static_cast<int>(H), static_cast<int>(Hk), static_cast<int>(D)};
       const at::AutoDispatchBelowADInplaceOrView below;
-      o = run_forward(q, k, v, s, flags, nullptr);
+      o = run_forward(q, k, v, shape_of(q, k, flags), flags, nullptr);
     }
   }
   return THPVariable_Wrap(std::move(o));
