@@ -64,27 +64,37 @@ __global__ void __launch_bounds__(128) kmean_partial_kernel(const KMeanParams p)
   kmean_block<D>(p, blockIdx.x, blockIdx.y, red);
 }
 
-// Stage 2: one CTA per (batch, kv head): serial fold of the chunk sums in chunk order, divided by N.
+// Mean of one column: serial fold of the chunk sums in chunk order, divided by N.  Bound by the latency of its loads, 0.6 us a
+// batch: 32 in flight, added in chunk order (with eight the fold of 512 chunks took longer than the chunk sums themselves: q, k, v
+// producers at N=32768 H=64 Hk=8 206 -> 181 us).
+__device__ __forceinline__ float kmean_column(const KMeanParams& p, int bh, int c) {
+  const int nchunk = p.N / 64;
+  const float* src = p.partial + static_cast<size_t>(bh) * nchunk * p.D + c;
+  float s = 0.f;
+  int j = 0;
+  for (; j + 32 <= nchunk; j += 32) {
+    float v[32];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) v[u] = src[static_cast<size_t>(j + u) * p.D];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) s += v[u];
+  }
+  if (j < nchunk) {
+    float v[32];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) v[u] = (j + u < nchunk) ? src[static_cast<size_t>(j + u) * p.D] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 32; ++u)
+      if (j + u < nchunk) s += v[u];
+  }
+  return s / static_cast<float>(p.N);
+}
+
+// Stage 2: one CTA per (batch, kv head).
 __global__ void kmean_fold_kernel(const KMeanParams p) {
   grid_dep_wait();
   const int bh = blockIdx.x;
-  const int nchunk = p.N / 64;
-  for (int c = threadIdx.x; c < p.D; c += blockDim.x) {
-    const float* src = p.partial + static_cast<size_t>(bh) * nchunk * p.D + c;
-    float s = 0.f;
-    int j = 0;
-    // Bound by the latency of its loads, 0.6 us a batch: 32 in flight, added in chunk order (with eight the fold of 512 chunks
-    // took longer than the chunk sums themselves: q, k, v producers at N=32768 H=64 Hk=8 206 -> 181 us).
-    for (; j + 32 <= nchunk; j += 32) {
-      float v[32];
-#pragma unroll
-      for (int u = 0; u < 32; ++u) v[u] = src[static_cast<size_t>(j + u) * p.D];
-#pragma unroll
-      for (int u = 0; u < 32; ++u) s += v[u];
-    }
-    for (; j < nchunk; ++j) s += src[static_cast<size_t>(j) * p.D];
-    p.mean[static_cast<size_t>(bh) * p.D + c] = s / static_cast<float>(p.N);
-  }
+  for (int c = threadIdx.x; c < p.D; c += blockDim.x) p.mean[static_cast<size_t>(bh) * p.D + c] = kmean_column(p, bh, c);
 }
 
 cudaError_t launch_kmean(const KMeanParams& p, cudaStream_t stream) {
@@ -101,7 +111,8 @@ cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream);
 // elsewhere, the kernel needs fewer registers and more of its small CTAs fit an SM (more loads in flight).
 // Executed by 128 threads (tid 0-127), which meet at the named barrier `bar`.
 template <int D, bool kMean, bool kStale>
-__device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int bh, float* wmax, int tid = threadIdx.x, int bar = 1) {
+__device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int bh, float* wmax, int tid = threadIdx.x, int bar = 1,
+                                            const float* mean_row = nullptr) {
   constexpr int kTpr = D / 16;           // threads per token row (16 elements each)
   constexpr int kRpp = 128 / kTpr;       // rows per pass
   constexpr int kPass = 32 / kRpp;
@@ -111,10 +122,10 @@ __device__ __forceinline__ void quant_block(const QuantParams& p, int blk, int b
 
   float mean[kMean ? 16 : 1];
   if (kMean) {
-    const float4* mp = reinterpret_cast<const float4*>(p.mean + static_cast<size_t>(bh) * D + c16 * 16);
+    const float4* mp = reinterpret_cast<const float4*>((mean_row != nullptr ? mean_row : p.mean + static_cast<size_t>(bh) * D) + c16 * 16);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float4 v = __ldg(mp + i);
+      const float4 v = mp[i];
       mean[4 * i] = v.x; mean[4 * i + 1] = v.y; mean[4 * i + 2] = v.z; mean[4 * i + 3] = v.w;
     }
   }
@@ -197,6 +208,22 @@ __global__ void __launch_bounds__(128, D == 128 ? 10 : 6) quant_qv_kmean_kernel(
     i -= n_q;
     quant_block<D, false, false>(pv, i % (pv.N / 32), i / (pv.N / 32), wmax);
   }
+}
+
+// K with the fold of its chunk sums: a CTA of four groups of 128 threads folds all columns of its head into shared memory, then
+// each group quantises 32 tokens.
+template <int D>
+__global__ void __launch_bounds__(512, D == 128 ? 2 : 1) quant_k_fold_kernel(const QuantParams p, const KMeanParams pm) {
+  __shared__ float mean[D];
+  __shared__ float wmax[16];
+  grid_dep_wait();
+  const int bh = blockIdx.y, group = threadIdx.x / 128;
+  if (threadIdx.x < D) {
+    mean[threadIdx.x] = kmean_column(pm, bh, threadIdx.x);
+    if (blockIdx.x == 0) pm.mean[static_cast<size_t>(bh) * D + threadIdx.x] = mean[threadIdx.x];
+  }
+  __syncthreads();
+  quant_block<D, true, false>(p, 4 * blockIdx.x + group, bh, wmax + 4 * group, threadIdx.x % 128, 1 + group, mean);
 }
 
 // Q, K and V of a short sequence in one launch.  A CTA has one group of 128 threads per 64 tokens; the K CTA of a (batch, kv
@@ -322,10 +349,19 @@ cudaError_t launch_quant_qkv(const QuantParams& pq, const QuantParams& pk, const
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
   cudaError_t e = launch_chained(pq.D == 128 ? quant_qv_kmean_kernel<128> : quant_qv_kmean_kernel<256>, static_cast<unsigned>(blocks), 128,
                                  0, stream, pq, pv, pm);
-  if (e == cudaSuccess) e = launch_chained(kmean_fold_kernel, pm.B * pm.Hk, 128, 0, stream, pm);
-  count_launch(2);
+  count_launch();
   if (e != cudaSuccess) return e;
-  return launch_quant(pk, stream);                      // K, centred by the mean that the fold has just written
+  // Then K, centred.  Every CTA of K folds the chunk sums for itself, which saves the fold's launch, as long as what they read
+  // for it together is small (a head's sums, N / 64 rows, once per 128 tokens).  Forward + backward: N=1024 H=8 Hk=2 80.0 -> 77.1 us,
+  // N=1920 H=6 Hk=2 D=256 (0.9 MiB) 94.2 -> 91.3; B=3 N=1792 H=15 Hk=5 (2.9 MiB) 203.1 -> 204.2, N=4096 H=32 Hk=8 (8 MiB) 470 -> 473.
+  if (static_cast<long long>(pm.B) * pm.Hk * (pm.N / 128) * (pm.N / 64) * pm.D * 4 <= (1ll << 20)) {
+    count_launch();
+    return launch_chained(pq.D == 128 ? quant_k_fold_kernel<128> : quant_k_fold_kernel<256>, dim3(pm.N / 128, pm.B * pm.Hk), 512, 0, stream, pk, pm);
+  }
+  e = launch_chained(kmean_fold_kernel, pm.B * pm.Hk, 128, 0, stream, pm);
+  count_launch();
+  if (e != cudaSuccess) return e;
+  return launch_quant(pk, stream);
 }
 
 cudaError_t launch_quant(const QuantParams& p, cudaStream_t stream) {

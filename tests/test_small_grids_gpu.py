@@ -7,8 +7,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,N,H,Hk,D", [(1, 256, 2, 1, 128), (2, 512, 3, 3, 128), (1, 128, 2, 2, 256), (3, 256, 2, 1, 256)])
-def test_short_producers_equal_the_separate_ones(B, N, H, Hk, D, oracle):
+@pytest.mark.parametrize("B,N,H,Hk,D", [(1, 256, 2, 1, 128), (2, 512, 3, 3, 128), (1, 128, 2, 2, 256), (3, 256, 2, 1, 256),
+                                         (2, 768, 4, 2, 128), (1, 2304, 2, 1, 128), (1, 384, 2, 2, 256), (1, 4096, 1, 1, 256)])
+def test_joined_producers_equal_the_separate_ones(B, N, H, Hk, D, oracle):
     from delta_matching_b200 import ops
     q, k, v, _ = (t.transpose(1, 2) for t in oracle.make_inputs(B, N, H, Hk, D, seed=71, device="cuda"))
     k = k + 0.5
