@@ -1,14 +1,8 @@
-// Backward of delta-matching fp8 attention on sm_100a: all matmuls on tcgen05 with TMEM accumulators, bit-deterministic
-// (one writer per output element, fixed loop orders, no atomics, no O(N^2) workspace).
+// dQ of the backward without a workspace, on sm_100a: all matmuls on tcgen05 with TMEM accumulators, bit-deterministic (one
+// writer per output element, fixed loop orders, no atomics).  dK and dV: dm_bwd_kv.cu; dQ from stored dS tiles: dm_bwd_p2.cu.
 //
-//   kernel 1 (dK/dV, key-stationary): CTA = (128-key tile, kv head, batch); loops over the query heads of the GQA group
-//     and their 128-query tiles: S^T = K8 Q8^T, dP^T = V8 dO8^T (kind::f8f6f4), P^T codes and dS^T codes written to TMEM,
-//     dV += P^T dO and dK += dS^T Q as block-scaled chains (kind::mxf8f6f4).  The group is reduced in TMEM, dK / dV are
-//     rounded to bf16 once per KV head.  With a workspace it also leaves the dS^T code tiles there for the streaming dQ
-//     kernel (dm_bwd_p2.cu).  Head_dim 256 runs it as two launches, one per accumulator.
-//   kernel 2 (dQ, query-stationary, the form without a workspace): CTA = (128-query tile, query head, batch); loops over
-//     key tiles: S, dP recomputed, dS codes staged in shared memory, dQ += dS K block-scaled; dQ * softmax_scale rounded
-//     to bf16 once.
+//   Query-stationary: CTA = (128-query tile, query head, batch); loops over key tiles: S, dP recomputed, dS codes staged in
+//   shared memory, dQ += dS K block-scaled; dQ * softmax_scale rounded to bf16 once.  Also the form of the identity probe.
 //
 // Numerics (delta_matching/reference.py:476-518 with preset "sm100-mx", :612-613; kernel-side rules
 // delta_matching/sm100/dm_bwd_sm100.py:5413-5433, 6175-6224 and attention_math_sm100.py:26-45):
@@ -16,8 +10,8 @@
 //   P^T codes: power-of-two scale per (key, 32 queries), amax 0 -> byte 0;   SFA_dV = p_sb (+) dos_sb
 //   dS codes:  power-of-two scale per (128 queries x 32 keys), amax 0 -> scale 1;  SFA_dK = ds_sb (+) qs_sb,
 //              dQ's scale along keys = ds_sb (+) ks_sb;  dQ = (dS K) * D^-0.5.
-// Both kernels evaluate P and dS with the same operations on the same accumulators, so the dS codes of kernel 2 are the
-// codes of kernel 1 whenever the two MMA orientations return the same fp32 sums.
+// P and dS are evaluated with the operations of the dK / dV kernel on the same accumulators, so the dS codes are that kernel's
+// whenever the two MMA orientations return the same fp32 sums.
 #include <cuda_bf16.h>
 #include "dm_common.cuh"
 #include "dm_kernels.h"
