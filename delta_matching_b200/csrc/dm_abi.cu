@@ -272,13 +272,13 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
 // Which backward dm_attn_bwd runs (same results).  The key-stationary kernel takes as long as its longest chain, (H / Hk)
 // (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.7 us a tile; the tile-parallel
 // pair takes its share of all tiles at about 3.7 us.  Forward + backward, chain / tiles per SM: 16 (N=1024 H=8 Hk=2) 92 -> 60 us;
-// 4.6 (N=8192 H=4 Hk=1) 594 -> 440; 2.3 (N=16384 H=2 Hk=1) 810 -> 758; 2.2 (N=2048 H=32 Hk=8) 222 -> 214; 2.05 (B=4 N=1024 H=16 Hk=4) 140 ->
-// 140; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  Head_dim 256: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152 -> 143; 1.45
-// (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 -> 495.  The lines are drawn at 2.2 and 1.6, and at 2 GiB of workspace.
+// 4.6 (N=8192 H=4 Hk=1) 594 -> 440; 2.3 (N=16384 H=2 Hk=1) 810 -> 758; 2.2 (N=2048 H=32 Hk=8) 222 -> 214; 2.06 (B=4 N=1024 H=16 Hk=4) 139 ->
+// 134.5; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  Head_dim 256: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152 -> 143; 1.45
+// (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 -> 495.  The lines are drawn at 2.0 and 1.6, and at 2 GiB of workspace.
 static bool tile_parallel(int B, int N, int H, int Hk, int D, int causal) {
   const long long n_t = N / 128, tiles = static_cast<long long>(B) * H * (causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
   const long long chain = H / Hk * n_t;
-  return 10 * chain * dm::sm_count() >= (D == 128 ? 22 : 16) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
+  return 10 * chain * dm::sm_count() >= (D == 128 ? 20 : 16) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
 }
 
 // Workspace of `units` query heads with both tile sets: dS^T tiles, P^T tiles, dS words, P words.
