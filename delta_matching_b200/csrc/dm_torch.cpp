@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/core/PythonFallbackKernel.h>
@@ -224,6 +225,16 @@ Shape shape_of(const Tensor& q, const Tensor& k, int64_t flags) {
           static_cast<int>(k.size(hm ? 1 : 2)), static_cast<int>(q.size(3))};
 }
 
+// dQ, dK, dV in the layout of the inputs; an undefined dO is a zero one.
+variable_list gradients(const Tensor& grad, const Tensor& saved, const Tensor& o, const Shape& s, int64_t flags) {
+  const at::AutoGradMode no_grad(false);
+  const Tensor d_o = grad.defined() ? grad : at::zeros({s.B, s.N, s.H, s.D}, saved.options().dtype(at::kBFloat16));
+  variable_list g = run_backward(d_o, saved, o, s, flags);
+  if (flags & kHeadMajor)
+    for (Tensor& t : g) t = t.permute({0, 2, 1, 3});
+  return g;
+}
+
 // The autograd node.  (torch::autograd::Function would do, at some 4 us more per forward + backward for its context, the map of
 // saved values and the generic wrapping of inputs and outputs.)
 struct AttnBackward : public torch::autograd::Node {
@@ -233,15 +244,11 @@ struct AttnBackward : public torch::autograd::Node {
 
   variable_list apply(variable_list&& grads) override {
     const std::lock_guard<std::mutex> lock(mutex_);
-    const Tensor d_o = grads[0].defined() ? grads[0] : input_metadata(0).zeros_like();
-    const bool twice = at::GradMode::is_enabled() && d_o.requires_grad();
+    const bool twice = at::GradMode::is_enabled() && grads[0].defined() && grads[0].requires_grad();
     variable_list g;
     {
-      const at::AutoGradMode no_grad(false);
-      const Tensor buffer = saved.unpack();
-      g = run_backward(d_o, buffer, (flags & kMatched) ? Tensor() : o.unpack(shared_from_this()), s, flags);
-      if (flags & kHeadMajor)
-        for (Tensor& t : g) t = t.permute({0, 2, 1, 3});
+      const at::AutoGradMode no_grad(false);      // for the unpack hooks
+      g = gradients(grads[0], saved.unpack(), (flags & kMatched) ? Tensor() : o.unpack(shared_from_this()), s, flags);
     }
     if (twice) {      // what torch.autograd.function.once_differentiable does: a second derivative raises when it is taken
       for (Tensor& t : g) t = t.detach().requires_grad_();
@@ -249,6 +256,45 @@ struct AttnBackward : public torch::autograd::Node {
               .apply(std::move(g));
     }
     return g;
+  }
+  // Compiled autograd: what the pass depends on, and the pass as a function of it that the recorded graph calls (opaque: the
+  // kernels take addresses, there is nothing to trace through).
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    args.collect(saved, false);
+    args.collect(o, true);
+    for (const int64_t x : {int64_t(s.B), int64_t(s.N), int64_t(s.H), int64_t(s.Hk), int64_t(s.D), flags}) args.collect(x);
+  }
+  variable_list apply_with_saved(const variable_list& grads, torch::dynamo::autograd::SwapSavedVariables& swap) override {
+    using torch::dynamo::autograd::IValuePacker;
+    swap.before(saved);
+    swap.before(o);
+    torch::dynamo::autograd::PackedArgs packed;
+    std::vector<at::TypePtr> schema;
+    auto pack = [&](const auto& x) {
+      packed.pack(x);
+      schema.push_back(IValuePacker<std::decay_t<decltype(x)>>::packed_type());
+    };
+    for (const int64_t x : {flags, int64_t(s.B), int64_t(s.N), int64_t(s.H), int64_t(s.Hk), int64_t(s.D)}) pack(x);
+    pack(saved.unpack());
+    if (!(flags & kMatched)) pack(o.unpack(shared_from_this()));
+    const auto& compiler = torch::dynamo::autograd::getPyCompilerInterface();
+    const std::string fn = compiler->bind_function(swap.get_py_compiler(), name(), &AttnBackward::apply_recorded, std::move(schema),
+                                                   /*is_custom_function=*/true, /*is_traceable=*/false);
+    variable_list g = compiler->call_function(
+        swap.get_py_compiler(), "apply_functional", fn, grads, packed.vec(),
+        IValuePacker<std::vector<std::optional<torch::autograd::InputMetadata>>>::pack(torch::dynamo::autograd::get_input_metadata(next_edges())));
+    swap.after(saved);
+    swap.after(o);
+    return g;
+  }
+  static variable_list apply_recorded(const variable_list& grads, const std::vector<c10::IValue>& args) {
+    torch::dynamo::autograd::PackedArgs packed(args);
+    auto i = [&] { return static_cast<int>(packed.unpack<int64_t>()); };
+    const int64_t flags = packed.unpack<int64_t>();
+    Shape s;
+    s.B = i(); s.N = i(); s.H = i(); s.Hk = i(); s.D = i();
+    const Tensor buffer = packed.unpack<Tensor>();
+    return gradients(grads[0], buffer, (flags & kMatched) ? Tensor() : packed.unpack<Tensor>(), s, flags);
   }
   void release_variables() override {
     const std::lock_guard<std::mutex> lock(mutex_);
