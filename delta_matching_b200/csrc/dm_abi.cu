@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 
 #include "../../include/dm_b200.h"
 #include "dm_kernels.h"
@@ -76,8 +77,24 @@ int make_code_map(CUtensorMap* m, const void* base, uint64_t rows, int D) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-int check_device_ptr(const void* p, const char* name) {
+int check_address(const void* p, const char* name) {
   if (p == nullptr) return fail(DM_ERR_ARG, "delta_matching: %s is NULL (every tensor must be a CUDA buffer)", name);
+  if (!aligned16(p)) return fail(DM_ERR_ARG, "delta_matching: %s must be 16-byte aligned", name);
+  return 0;
+}
+
+struct NamedPtr {
+  const void* p;
+  const char* name;
+};
+int check_addresses(std::initializer_list<NamedPtr> ptrs) {
+  for (const NamedPtr& x : ptrs)
+    if (int r = check_address(x.p, x.name)) return r;
+  return 0;
+}
+
+int check_device_ptr(const void* p, const char* name) {
+  if (p == nullptr) return check_address(p, name);
   cudaPointerAttributes a;
   cudaError_t e = cudaPointerGetAttributes(&a, p);
   if (e != cudaSuccess) {
@@ -91,8 +108,7 @@ int check_device_ptr(const void* p, const char* name) {
   if (a.type == cudaMemoryTypeDevice && a.device != dev)
     return fail(DM_ERR_ARG, "delta_matching: %s is on device %d but the current device is %d (every tensor must be on the "
                             "same device)", name, a.device, dev);
-  if (!aligned16(p)) return fail(DM_ERR_ARG, "delta_matching: %s must be 16-byte aligned", name);
-  return 0;
+  return check_address(p, name);
 }
 
 int check_shape(int B, int N, int H, int Hk, int D) {
@@ -238,8 +254,8 @@ int dm_quant_do(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn,
 // ------------------------------------------------------------------------------------------------ whole passes
 // dm_attn_fwd / dm_attn_bwd launch what a forward or a backward of the attention layer needs in one call.  The separate
 // entry points above and below look every pointer up in the driver (cudaPointerGetAttributes, some 0.3 us each, about
-// forty of them in a training step) and encode the tensor maps once per kernel; here the caller vouches for its buffers and
-// every map is encoded once per pass.
+// forty of them in a training step) and encode the tensor maps once per kernel; here the caller vouches that its buffers are
+// memory of the current device, what a pointer itself shows (NULL, alignment) is checked, and every map is encoded once per pass.
 int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
                 const void* k, int64_t k_sb, int64_t k_sh, int64_t k_sn,
                 const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
@@ -247,10 +263,12 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
                 void* q8, void* k8, void* v8, float* qs, float* ks, float* vs, float* kmean, void* workspace,
                 void* o, float* lse, int* status, void* stream) {
   DM_TRY(check_shape(B, N, H, Hk, D));
-  DM_TRY(check_sm100());
+  DM_TRY(check_addresses({{q, "q"}, {k, "k"}, {v, "v"}, {q8, "q8"}, {k8, "k8"}, {v8, "v8"}, {qs, "q scales"}, {ks, "k scales"},
+                          {vs, "v scales"}, {kmean, "kmean"}, {workspace, "workspace"}, {o, "o"}, {lse, "lse"}}));
   DM_TRY(check_strides("q", q_sb, q_sh, q_sn));
   DM_TRY(check_strides("k", k_sb, k_sh, k_sn));
   DM_TRY(check_strides("v", v_sb, v_sh, v_sn));
+  DM_TRY(check_sm100());
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const float sm = static_cast<float>(1.0 / sqrt(static_cast<double>(D)));
   const dm::QuantParams pq = make_quant(q, q_sb, q_sh, q_sn, nullptr, sm, nullptr, 0, 0, 0, B, N, H, D, q8, qs, nullptr);
@@ -319,13 +337,17 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
                 const float* lse, void* do8, float* dos, float* delta, int B, int N, int H, int Hk, int D, int causal,
                 void* dq, void* dk, void* dv, void* workspace, int64_t workspace_bytes, int flags, int* status, void* stream) {
   DM_TRY(check_shape(B, N, H, Hk, D));
-  DM_TRY(check_sm100());
+  DM_TRY(check_addresses({{d_o, "d_o"}, {q8, "q8"}, {k8, "k8"}, {v8, "v8"}, {qs, "q scales"}, {ks, "k scales"}, {vs, "v scales"},
+                          {lse, "lse"}, {do8, "do8"}, {dos, "dO scales"}, {delta, "delta"}}));
+  if (o != nullptr) DM_TRY(check_address(o, "o"));
   DM_TRY(check_strides("d_o", do_sb, do_sh, do_sn));
   const bool kernels = (flags & DM_ATTN_DELTA_ONLY) == 0;
+  if (kernels) DM_TRY(check_addresses({{dq, "dq"}, {dk, "dk"}, {dv, "dv"}, {workspace, "workspace"}}));
+  DM_TRY(check_sm100());
   const int64_t need = dm_attn_bwd_workspace_bytes(B, N, H, Hk, D, causal);
   const uint64_t tiles = static_cast<uint64_t>(B) * H * (N / 128) * (N / 128);
-  if (kernels && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
-    return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed (16-byte aligned)", (long long)workspace_bytes, (long long)need);
+  if (kernels && workspace_bytes < need)
+    return fail(DM_ERR_ARG, "delta_matching: dS workspace of %lld bytes given, %lld needed", (long long)workspace_bytes, (long long)need);
   int batches = B, groups = Hk;
   const bool tile_form = tile_parallel(B, N, H, Hk, D, causal), p_form = !tile_form && D == 256 && p_ranges(B, N, H, Hk, batches, groups);
   if (kernels && !p_form && tiles * 128 >= (1ull << 31))

@@ -157,8 +157,9 @@ int dm_bwd_ws(const void* q8, const void* k8, const void* v8, const void* do8,
               void* workspace, int64_t workspace_bytes, int parts, int* status, void* stream);
 
 /* Whole passes: everything a forward, or a backward, of the attention layer launches, in one call (what the native PyTorch
- * path uses).  The kernels and their results are those of the separate entry points.  The caller vouches for the
- * pointers (device memory of the current device, 16-byte aligned): only shapes and strides are checked here.
+ * path uses).  The kernels and their results are those of the separate entry points.  The caller vouches that
+ * the pointers are memory of the current device, which is not looked up here; NULL and misaligned pointers (16 bytes), shapes
+ * and strides are refused as everywhere.
  *
  * dm_attn_fwd = dm_quant_qkv, dm_fwd.  q, k, v by element strides for (batch, head, token); o is contiguous (B, N, H, D).
  * kmean (B, Hk, D) fp32 and workspace (dm_quant_qkv_workspace_bytes) are scratch. */

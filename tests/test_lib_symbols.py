@@ -3,6 +3,8 @@ launched), and the ctypes prototypes cover exactly the declared functions."""
 import os
 import re
 
+import pytest
+
 from .conftest import ROOT
 
 
@@ -41,9 +43,31 @@ def test_argument_checks_without_gpu():
     assert rc == -1 and "65535" in _lib.last_error()
 
 
+@pytest.mark.parametrize("bad", [None, 0x1008], ids=["null", "misaligned"])
+def test_whole_pass_entry_points_refuse_bad_pointers(bad):
+    """Every buffer of dm_attn_fwd / dm_attn_bwd in turn NULL or 8 bytes off, before any CUDA call; the fine ones are made-up
+    addresses that a machine without a GPU never gets to use."""
+    from delta_matching_b200 import _lib
+    L = _lib.lib()
+    fine = 0x10000
+    st, shape = (256 * 256, 128, 256), (1, 256, 2, 2, 128, 1)
+    names = ("q", "k", "v", "q8", "k8", "v8", "q scales", "k scales", "v scales", "kmean", "workspace", "o", "lse")
+    for i, name in enumerate(names):
+        p = [bad if j == i else fine for j in range(13)]
+        assert L.dm_attn_fwd(p[0], *st, p[1], *st, p[2], *st, *shape, *p[3:], None, None) == -1
+        assert f" {name} " in _lib.last_error()
+    names = ("d_o", "q8", "k8", "v8", "q scales", "k scales", "v scales", "lse", "do8", "dO scales", "delta", "dq", "dk", "dv", "workspace", "o")
+    ws = L.dm_attn_bwd_workspace_bytes(*shape)
+    for i, name in enumerate(names):
+        if name == "o" and bad is None:                 # no O: the matched delta
+            continue
+        p = [bad if j == i else fine for j in range(16)]
+        assert L.dm_attn_bwd(p[0], *st, p[15], *p[1:11], *shape, *p[11:15], ws, 0, None, None) == -1
+        assert f" {name} " in _lib.last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from delta_matching_b200 import _lib
-    import pytest
     monkeypatch.setenv("DM_SO", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="does not exist"):
         _lib.library_path()
