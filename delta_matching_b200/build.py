@@ -52,7 +52,10 @@ def code_sha() -> str:
 
 def _build_native(verbose: bool) -> None:
     """g++ against the installed torch's headers; the module finds torch's libraries already loaded (it is imported behind
-    torch) and takes the kernel library's entry points as addresses, so it links neither by path."""
+    torch) and takes the kernel library's entry points as addresses, so it links neither by path.
+
+    The C++ runtime is named as the shared library that torch uses: a compiler without a libstdc++.so of its own links the
+    static one, and an exception that leaves the module's copy for torch's autograd engine ends the process."""
     import sysconfig
     import torch
     from torch.utils import cpp_extension
@@ -60,7 +63,8 @@ def _build_native(verbose: bool) -> None:
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, os.path.join(CSRC, NATIVE_SOURCE), "-o", NATIVE,
-           f"-L{lib_dir}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+           f"-L{lib_dir}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+           "-nostdlib++", "-l:libstdc++.so.6", "-lm"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {NATIVE_SOURCE}:\n{r.stdout}\n{r.stderr[-6000:]}")
@@ -69,12 +73,12 @@ def _build_native(verbose: bool) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile and link (skipped when the library is newer than a stamp of the sources' hash)."""
+    """Compile and link (skipped when a stamp says that the libraries come from these sources and this recipe)."""
     obj_dir = OBJ
     lib = LIB
     os.makedirs(obj_dir, exist_ok=True)
     stamp = os.path.join(obj_dir, "stamp.txt")
-    sha = code_sha()
+    sha = code_sha() + " " + hashlib.sha256(open(__file__, "rb").read()).hexdigest()[:12]
     if not force and os.path.isfile(lib) and os.path.isfile(NATIVE) and os.path.isfile(stamp) and open(stamp).read().strip() == sha:
         return lib
     srcs = list(SOURCES)
