@@ -82,6 +82,15 @@ Tensor rows(const Tensor& t) {
   return t;
 }
 
+// A saved tensor as the kernels read it, in order and aligned.  Unpack hooks may hand over anything (torch checks what hooks make
+// of a gradient, but not this): another layout is copied, another type, shape or device is refused.
+Tensor unpacked(const Tensor& t, const char* name, at::ScalarType type, at::IntArrayRef sizes, const at::Device& dev) {
+  TORCH_CHECK(t.defined() && t.layout() == at::kStrided && t.scalar_type() == type && t.sizes() == sizes && t.device() == dev,
+              "delta_matching: ", name, " must come back from saved-tensor hooks as a ", type, " tensor of shape ", sizes, " on ", dev);
+  const bool in_place = t.is_contiguous() && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
+  return in_place ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+
 // Sub-buffers of one allocation, each 256-byte aligned.
 class Carve {
  public:
@@ -166,14 +175,14 @@ Tensor run_forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, c
 }
 
 // dQ, dK, dV token-major.  `o`: the forward's output (stale delta), undefined for the matched delta.
-variable_list run_backward(const Tensor& d_o_in, const Tensor& saved, const Tensor& o, const Shape& s, int64_t flags) {
-  const at::Device dev = saved.device();
+variable_list run_backward(const Tensor& d_o_in, const Tensor& saved_in, const Tensor& o_in, const Shape& s, int64_t flags, const at::Device& dev) {
   const c10::cuda::CUDAGuard guard(dev);
   int* status = status_of(dev.index());
-  const Tensor d_o = rows(d_o_in);
-  const Strides sd(d_o, false);
   const Saved L(s);
-  uint8_t* p = static_cast<uint8_t*>(saved.mutable_data_ptr());
+  const Tensor d_o = rows(d_o_in), saved = unpacked(saved_in, "the saved codes", at::kByte, {L.c.size()}, dev);
+  const Tensor o = o_in.defined() ? unpacked(o_in, "the saved O", at::kBFloat16, {s.B, s.N, s.H, s.D}, dev) : o_in;
+  const Strides sd(d_o, false);
+  uint8_t* p = static_cast<uint8_t*>(saved.mutable_data_ptr());      // only read
   // The dS workspace of the whole call, as long as no bound is set and it is no larger than what ops takes without asking the
   // device how much memory is free; otherwise ops.bwd_fp8 plans the ranges.
   const int64_t ws_bytes = g_lib.bwd_workspace_bytes(s.B, s.N, s.H, s.Hk, s.D, (flags & kCausal) ? 1 : 0);
@@ -226,10 +235,10 @@ Shape shape_of(const Tensor& q, const Tensor& k, int64_t flags) {
 }
 
 // dQ, dK, dV in the layout of the inputs; an undefined dO is a zero one.
-variable_list gradients(const Tensor& grad, const Tensor& saved, const Tensor& o, const Shape& s, int64_t flags) {
+variable_list gradients(const Tensor& grad, const Tensor& saved, const Tensor& o, const Shape& s, int64_t flags, const at::Device& dev) {
   const at::AutoGradMode no_grad(false);
-  const Tensor d_o = grad.defined() ? grad : at::zeros({s.B, s.N, s.H, s.D}, saved.options().dtype(at::kBFloat16));
-  variable_list g = run_backward(d_o, saved, o, s, flags);
+  const Tensor d_o = grad.defined() ? grad : at::zeros({s.B, s.N, s.H, s.D}, at::TensorOptions(dev).dtype(at::kBFloat16));
+  variable_list g = run_backward(d_o, saved, o, s, flags, dev);
   if (flags & kHeadMajor)
     for (Tensor& t : g) t = t.permute({0, 2, 1, 3});
   return g;
@@ -248,7 +257,7 @@ struct AttnBackward : public torch::autograd::Node {
     variable_list g;
     {
       const at::AutoGradMode no_grad(false);      // for the unpack hooks
-      g = gradients(grads[0], saved.unpack(), (flags & kMatched) ? Tensor() : o.unpack(shared_from_this()), s, flags);
+      g = gradients(grads[0], saved.unpack(), (flags & kMatched) ? Tensor() : o.unpack(shared_from_this()), s, flags, input_metadata(0).device());
     }
     if (twice) {      // what torch.autograd.function.once_differentiable does: a second derivative raises when it is taken
       for (Tensor& t : g) t = t.detach().requires_grad_();
@@ -294,7 +303,7 @@ struct AttnBackward : public torch::autograd::Node {
     Shape s;
     s.B = i(); s.N = i(); s.H = i(); s.Hk = i(); s.D = i();
     const Tensor buffer = packed.unpack<Tensor>();
-    return gradients(grads[0], buffer, (flags & kMatched) ? Tensor() : packed.unpack<Tensor>(), s, flags);
+    return gradients(grads[0], buffer, (flags & kMatched) ? Tensor() : packed.unpack<Tensor>(), s, flags, buffer.device());
   }
   void release_variables() override {
     const std::lock_guard<std::mutex> lock(mutex_);
