@@ -25,6 +25,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -46,7 +47,7 @@ struct Lib {
 } g_lib;
 
 constexpr int kMaxDevices = 64;
-int* g_status[kMaxDevices] = {};          // pinned status words (ops.status_word), one per device that has been used
+std::atomic<int*> g_status[kMaxDevices] = {};  // pinned status words (ops.status_word), one per device that has been used
 PyObject* g_status_word = nullptr;        // ops: device index -> address of its status word
 PyObject* g_raise_if_set = nullptr;       // ops._raise_if_set
 PyObject* g_split_bwd = nullptr;          // ops.bwd_fp8: the backward under a workspace bound
@@ -132,11 +133,12 @@ struct Saved {
 
 // The word is read without a synchronisation, as every op does (ops._enter); a kernel that gave up makes this call raise.
 int* status_of(int dev) {
-  int* w = g_status[dev];
+  int* w = g_status[dev].load(std::memory_order_acquire);
   if (w == nullptr) {
     pybind11::gil_scoped_acquire gil;
     pybind11::object addr = pybind11::reinterpret_borrow<pybind11::object>(g_status_word)(dev);
-    w = g_status[dev] = reinterpret_cast<int*>(addr.cast<uintptr_t>());
+    w = reinterpret_cast<int*>(addr.cast<uintptr_t>());
+    g_status[dev].store(w, std::memory_order_release);
   }
   if (*static_cast<volatile int*>(w) != 0) {
     std::string msg;

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 
 import torch
 
@@ -28,6 +29,7 @@ NUMERICS = {
     "sm100-mx-d256-ds32": (True, True),
     "sm100-mx-nonorm": (False, False),
 }
+_STATUS_LOCK = threading.Lock()
 _STATUS = {}                              # device index -> int32 status word (pinned host memory the kernels write)
 _DEBUG = os.environ.get("DM_DEBUG", "0") not in ("", "0")
 
@@ -70,12 +72,16 @@ def _dev_index(device) -> int:
 def status_word(device) -> torch.Tensor:
     """The per-device int32 word the kernels set when a bounded wait runs out (0 = no problem).  It lives in pinned host
     memory, which the GPU writes directly (pinned allocations are mapped into the device's address space under unified
-    addressing), so the host reads it without a copy and without a synchronisation."""
+    addressing), so the host reads it without a copy and without a synchronisation.  There is one word per device for as long
+    as the process lives, whichever threads ask for it first: kernels in flight and the native route hold its address."""
     idx = _dev_index(device)
     w = _STATUS.get(idx)
     if w is None:
-        with torch.cuda.device(idx):
-            w = _STATUS[idx] = torch.zeros(1, dtype=torch.int32).pin_memory()
+        with _STATUS_LOCK:
+            w = _STATUS.get(idx)
+            if w is None:
+                with torch.cuda.device(idx):
+                    w = _STATUS[idx] = torch.zeros(1, dtype=torch.int32).pin_memory()
     return w
 
 

@@ -56,3 +56,41 @@ def test_non_current_device(oracle):
     for nm in NAMES:
         assert got[nm].device == q.device
         assert torch.equal(got[nm], ref[nm]), nm
+
+
+def test_host_threads_give_the_plain_call_s_bits(oracle):
+    """Host threads with a stream each run forward and backward passes of different shapes at the same time."""
+    import threading
+    from delta_matching_b200 import dm_attn_func
+    shapes = [(1, 512, 4, 2, 128, "matched"), (2, 256, 3, 1, 128, "stale"), (1, 384, 2, 2, 256, "matched"), (1, 1024, 8, 2, 128, "stale")]
+    inputs = [oracle.make_inputs(B, N, H, Hk, D, seed=51 + i, device="cuda") for i, (B, N, H, Hk, D, _) in enumerate(shapes)]
+
+    def step(i):
+        q, k, v, do = inputs[i]
+        leaves = [t.detach().requires_grad_() for t in (q, k, v)]
+        o = dm_attn_func(*leaves, causal=True, mode=shapes[i][5])
+        return (o.detach(),) + torch.autograd.grad(o, leaves, do)
+
+    want = [step(i) for i in range(len(shapes))]
+    torch.cuda.synchronize()
+    start, got, errors = threading.Barrier(len(shapes)), [None] * len(shapes), []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                got[i] = [step(i) for _ in range(8)]
+        except Exception as e:                            # carried to the test's thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for i, runs in enumerate(got):
+        for run in runs:
+            for a, b in zip(run, want[i]):
+                assert torch.equal(a, b)
