@@ -57,3 +57,24 @@ def test_a_unit_has_the_same_bits_in_a_small_and_a_large_call(N, rep, D, causal,
     for u in (0, units - 1):
         for a, b in zip(step(u, u + 1), whole):
             assert torch.equal(a, b[u:u + 1])
+
+
+@pytest.mark.parametrize("B,N,H,Hk,causal,mode,numerics", [
+    (5, 8192, 8, 8, True, "matched", "sm100-mx"),            # ranges of three and two batches
+    (1, 16384, 8, 4, True, "stale", "sm100-mx-d256-ds32"),   # two ranges of two kv groups
+    (3, 16384, 3, 3, False, "stale", "sm100-mx"),            # two batches, then one
+    (1, 16384, 9, 9, True, "matched", "sm100-mx"),           # kv groups in ranges of five and four
+])
+def test_ranges_of_the_wide_backward_equal_the_op_layer(B, N, H, Hk, causal, mode, numerics, oracle):
+    """Head_dim 256 calls whose two tile sets exceed one range: dm_attn_func goes range by range through the P^T form, the op layer
+    through the key-stationary kernel."""
+    from delta_matching_b200 import _lib, ops
+    from .helpers import run_api, run_ops
+    per_head = (N // 128) ** 2 * (2 * 16384 + 528)
+    ws = _lib.lib().dm_attn_bwd_workspace_bytes(B, N, H, Hk, 256, int(causal))
+    assert ops.bwd_workspace_bytes(1, N, 1, 256) < ws < B * H * per_head and ws % per_head == 0
+    q, k, v, do = oracle.make_inputs(B, N, H, Hk, 256, seed=74, device="cuda")
+    got = run_api(q, k, v, do, causal, mode, numerics)
+    want = run_ops(q, k, v, do, causal, mode, numerics=numerics)
+    for nm in ("dQ", "dK", "dV"):
+        assert torch.equal(got[nm], want[nm]), nm
