@@ -34,23 +34,25 @@ namespace dm {
 // (S^T, dP^T, dS codes, dK and the dS tiles for the workspace), each with the other half of the work compiled out.  Or, PO, the DK
 // role also leaves the P^T tiles in the workspace, and dV is streamed from them beside dQ (dm_bwd_p2.cu), which saves the
 // DV role's S^T and exponentials.
-template <int D, bool DV, bool DK, int G, bool PO = false>
+template <int D, bool DV, bool DK, bool PO = false>
 struct KvCfg {
-  static_assert(!PO || (DK && !DV && G == 2), "P^T tiles go out of the DK role");
+  static_assert(!PO || (DK && !DV), "P^T tiles go out of the DK role");
   static_assert((D == 128 || D == 256) && (DV || DK) && !(D == 256 && DV && DK), "two accumulators of 256 columns fill the TMEM");
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
   static constexpr int kCodeBytes = 128 * 128;         // dS^T code tile (does not depend on head_dim)
   static constexpr int kStages = (D == 128) ? 4 : 2;
-  static constexpr int kComputeWarps = 4 * G, kCh = 4 / G, kCols = 128 / G;
+  static constexpr int kComputeWarps = 8;              // with sixteen on one block of 32 queries each, a warp's fixed work per tile is
+                                                       // done sixteen times (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256
+                                                       // the two are equal
   static constexpr int kThreads = (kComputeWarps + 4) * 32;
   static constexpr int kTmemCols = 512;
   static constexpr int kColS = 0, kColDp = 128;        // fp32 accumulators, 128 columns each
   // What a warp writes over the 64 columns [64 h, 64 h + 64) that it has read, relative to the region:
   static constexpr int kColCodes = 0;        // 64 h + 8 c: codes of query block 2 h + c (P^T over S^T, dS^T over dP^T)
-  static constexpr int kColXv = 8 * kCh;          // 64 h + 16: 4 columns of the dV scale word of half h (byte c = block 2 h + c)
-  static constexpr int kColXk = 8 * kCh + 4;          // 64 h + 20: likewise, dK
-  static constexpr int kColOne = 8 * kCh + 8;         // 4 columns of 0x7F7F7F7F (written by h = 0)
+  static constexpr int kColXv = 16;          // 64 h + 16: 4 columns of the dV scale word of half h (byte c = block 2 h + c)
+  static constexpr int kColXk = 20;          // 64 h + 20: likewise, dK
+  static constexpr int kColOne = 24;         // 4 columns of 0x7F7F7F7F (written by h = 0)
   static constexpr int kColDv = 256, kColDk = (DV && DK) ? 384 : 256;
   static constexpr int kSmemK = 0;
   static constexpr int kSmemV = kTileBytes;                          // the DV role has no V tile
@@ -60,7 +62,7 @@ struct KvCfg {
   static constexpr int kSmemVec = kSmemWs + (DK ? 2 * kCodeBytes : 0);   // [kStages] vectors of the query tile (bytes):
   static constexpr int kVecLse = 0, kVecDelta = 512, kVecQs = 1024, kVecDos = 1040, kVecBytes = 1056;
   static constexpr int kSmemXch = kSmemVec + kStages * kVecBytes;    // [2 parities][8 warps] floats
-  static constexpr int kSmemBar = kSmemXch + 2 * 16 * 4;
+  static constexpr int kSmemBar = kSmemXch + 2 * 8 * 4;
   static constexpr int kSmemBytes = kSmemBar + 256;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
 };
@@ -82,10 +84,10 @@ __device__ __forceinline__ void store_bf16_row32(const uint32_t (&r)[32], __nv_b
 
 // DS32: the dS scale is taken per (32 queries x 32 keys), which is one 32-column block of one warp, instead of the contract's
 // (128 queries x 32 keys), for which the two warps of a key quadrant exchange their maxima.
-template <int D, bool DV, bool DK, bool DS32, int G, bool PO = false>
+template <int D, bool DV, bool DK, bool DS32, bool PO = false>
 __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                                           const CUtensorMap& tm_do, const CUtensorMap& tm_ds, const CUtensorMap& tm_p, const BwdParams& p) {
-  using C = KvCfg<D, DV, DK, G, PO>;
+  using C = KvCfg<D, DV, DK, PO>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemBar);
   uint64_t* bar_kv = bars + 0;       // K and V landed
@@ -246,10 +248,10 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
     auto chain_acc = [&](uint32_t d_tmem, uint32_t codes, uint32_t words, uint32_t ones, uint32_t b_lo, bool first) {
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
-        const uint32_t h = C::kCols * (ks / C::kCh);
+        const uint32_t h = 64 * (ks / 2);
 #pragma unroll
         for (int s = 0; s < C::kSub; ++s)
-          mma_mxf8_ts(d_tmem + s * 128, codes + h + 8 * (ks % C::kCh), b_lo + s * 1024 + ks * 256, idesc_mxf8(128, 128, false, true, ks % C::kCh, 0),
+          mma_mxf8_ts(d_tmem + s * 128, codes + h + 8 * (ks % 2), b_lo + s * 1024 + ks * 256, idesc_mxf8(128, 128, false, true, ks % 2, 0),
                       words + h, ones, !first || (ks > 0));
       }
     };
@@ -330,17 +332,16 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
     if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInDkDv);
   } else if (warp < C::kComputeWarps) {
     // ------------------------------------------------------------------------------------------ compute warps
-    constexpr int CH = C::kCh;
     const int half = warp >> 2;                        // query columns [64 half, 64 half + 64) of every tile
     const int quad = warp & 3;                         // lane quadrant = 32-key block of the dS scale
     const int r = tid & 127;                           // key row inside the tile = TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t t_s0 = tmem + lane_base + C::kCols * half, t_dp = t_s0 + C::kColDp;
+    const uint32_t t_s0 = tmem + lane_base + 64 * half, t_dp = t_s0 + C::kColDp;
     const int key = kt * 128 + r;
     const int nblk = p.N / 32;
     const float ks_row = p.ks[static_cast<size_t>(bhk) * nblk + key / 32];
     const float vs_row = DK ? p.vs[static_cast<size_t>(bhk) * nblk + key / 32] : 0.f;
-    const uint32_t vec_a = smem_u32(smem + C::kSmemVec) + 4 * C::kCols * half;       // this half's entries of the 128-query vectors
+    const uint32_t vec_a = smem_u32(smem + C::kSmemVec) + 256 * half;       // this half's entries of the 128-query vectors
     const uint32_t xch_a = smem_u32(smem + C::kSmemXch);
     const uint32_t ws_a = smem_u32(smem + C::kSmemWs) + r * 128;
     bool ok = true;
@@ -350,20 +351,20 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       const uint32_t ph = i & 1;
       const int st = i % C::kStages;
       const bool diag = p.causal && (left == n_qi);      // the first query tile of a causal sweep is the diagonal one
-      const uint32_t va = vec_a + st * C::kVecBytes, sc = va - (4 * C::kCols - 4 * C::kCh) * half;  // sc: the scales of this half's two blocks
+      const uint32_t va = vec_a + st * C::kVecBytes, sc = va - 248 * half;  // sc: the scales of this half's two blocks
       const uint32_t t_s = t_s0 + (DK ? 0 : 128 * ph);
-      float2 pr[CH][16];                                  // P, then (DK) -dS
+      float2 pr[2][16];                                   // P, then (DK) -dS
       float2 qs2, dos2;
       uint32_t xv = 0;
       if (ok) ok = wait_warp(vec_ok + st, (i / C::kStages) & 1, abort_flag);
       if (ok) ok = wait_warp(bar_s + (DK ? 0 : ph), DK ? ph : ((i >> 1) & 1), abort_flag);
       if (ok) {
         tc_fence_after();
-        qs2 = CH == 2 ? lds_f2(sc + C::kVecQs) : make_float2(lds_f(sc + C::kVecQs), 1.f);
-        dos2 = CH == 2 ? lds_f2(sc + C::kVecDos) : make_float2(lds_f(sc + C::kVecDos), 1.f);
-        uint32_t rs[CH][32];
+        qs2 = lds_f2(sc + C::kVecQs);
+        dos2 = lds_f2(sc + C::kVecDos);
+        uint32_t rs[2][32];
         tmem_ld32(t_s, rs[0]);
-        if constexpr (CH == 2) tmem_ld32(t_s + 32, rs[CH - 1]);
+        tmem_ld32(t_s + 32, rs[1]);
         tmem_wait_ld();
         if (!DV) {                                       // S^T of the next tile may land
           tc_fence_before();
@@ -372,13 +373,13 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         }
         if (diag) {
 #pragma unroll
-          for (int c = 0; c < CH; ++c)
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (r > C::kCols * half + 32 * c + e) rs[c][e] = 0xff800000u;   // -inf: key index above the query index
+              if (r > 64 * half + 32 * c + e) rs[c][e] = 0xff800000u;   // -inf: key index above the query index
         }
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
+        for (int c = 0; c < 2; ++c) {
           const float2 cc = splat2((ks_row * (c ? qs2.y : qs2.x)) * kLog2e);
           float pm0 = 0.f, pm1 = 0.f;
           if (PO && c == 0 && i > 0) ok = wait_warp(po_free, ph ^ 1, abort_flag);
@@ -399,7 +400,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
             codes32(pr[c], sb_to_inv(psb), w);
             if (DV) tmem_st8(t_s + C::kColCodes + 8 * c, w);
             if (PO) {                                      // as a [key][query] tile, like the dS^T codes below
-              const int j = 2 * CH * half + 2 * c;
+              const int j = 4 * half + 2 * c;
               sts_u4(ws_a + C::kCodeBytes + ((j ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
               sts_u4(ws_a + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
             }
@@ -424,9 +425,9 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       if (DK && ok) ok = wait_warp(bar_dp, ph, abort_flag);
       if (DK && ok) {
         tc_fence_after();
-        uint32_t rd[CH][32];
+        uint32_t rd[2][32];
         tmem_ld32(t_dp, rd[0]);
-        if constexpr (CH == 2) tmem_ld32(t_dp + 32, rd[CH - 1]);
+        tmem_ld32(t_dp + 32, rd[1]);
         tmem_wait_ld();
         if (half == 0) tmem_st4(t_dp + C::kColOne, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
         if (DV) {                                        // P^T codes and words are complete
@@ -437,7 +438,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           if ((tid & 31) == 0) mbar_arrive(bar_p);
         }
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
+        for (int c = 0; c < 2; ++c) {
           // -dS = P (delta - dP_acc a): a is a power of two, so the product is exact; the sign is undone by the codes' scale
           const float2 na = splat2(-(vs_row * (c ? dos2.y : dos2.x)));
           float am0 = 0.f, am1 = 0.f;
@@ -455,47 +456,44 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         }
         if (!DS32) {
           am[0] = warp_max(fmaxf(am[0], am[1]));
-          if ((tid & 31) == 0) sts_f(xch_a + 4 * (ph * 16 + warp), am[0]);
+          if ((tid & 31) == 0) sts_f(xch_a + 4 * (ph * 8 + warp), am[0]);
         }
       }
       if (DK) {
         // one dS scale per (128 queries x this quadrant's 32 keys): the two warps of the quadrant meet here (reached for every
         // tile, also after a failed wait).  With 32 x 32 blocks the warp's own maxima are the blocks'.
-        if (!DS32) bar_sync(1 + quad, 32 * G);
+        if (!DS32) bar_sync(1 + quad, 64);
         if (ok) {
           uint32_t dsb[2];
           if (DS32) {
-            dsb[1] = 0;
 #pragma unroll
-            for (int c = 0; c < CH; ++c) dsb[c] = pow2_sb(warp_max(am[c]), 127u);
+            for (int c = 0; c < 2; ++c) dsb[c] = pow2_sb(warp_max(am[c]), 127u);
           } else {
-            float mx = lds_f(xch_a + 4 * (ph * 16 + quad));
-#pragma unroll
-            for (int g = 1; g < G; ++g) mx = fmaxf(mx, lds_f(xch_a + 4 * (ph * 16 + 4 * g + quad)));
+            const float mx = fmaxf(lds_f(xch_a + 4 * (ph * 8 + quad)), lds_f(xch_a + 4 * (ph * 8 + 4 + quad)));
             dsb[0] = dsb[1] = pow2_sb(mx, 127u);
           }
           const uint32_t ws_row = ws_a + (PO ? 0 : ph * C::kCodeBytes);
 #pragma unroll
-          for (int c = 0; c < CH; ++c) {
+          for (int c = 0; c < 2; ++c) {
             uint32_t w[8];
             codes32(pr[c], -sb_to_inv(dsb[c]), w);
             tmem_st8(t_dp + C::kColCodes + 8 * c, w);
             if (p.ds_codes != nullptr) {
               // the same codes as a [key][query] tile in 128-byte-swizzled shared memory (16-byte chunk j of row r at
               // chunk j ^ (r % 8)), which the MMA warp stores to the workspace for pass 2
-              const int j = 2 * CH * half + 2 * c;
+              const int j = 4 * half + 2 * c;
               sts_u4(ws_row + ((j ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
               sts_u4(ws_row + (((j + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
             }
           }
-          const uint32_t xk = sb_mul(dsb[0], scale_to_sb(qs2.x)) | (CH == 2 ? (sb_mul(dsb[1], scale_to_sb(qs2.y)) << 8) : 0u);
+          const uint32_t xk = sb_mul(dsb[0], scale_to_sb(qs2.x)) | (sb_mul(dsb[1], scale_to_sb(qs2.y)) << 8);
           tmem_st4(t_dp + C::kColXk, xk, xk, xk, xk);
           if (p.ds_codes != nullptr) {
             fence_async_smem();
             // scale bytes of the tile for pass 2, [query block][key block]
             if ((tid & 31) == 0) {
 #pragma unroll
-              for (int c = 0; c < CH; ++c) p.ds_words[static_cast<size_t>(ws_tile) * 16 + (CH * half + c) * 4 + quad] = static_cast<uint8_t>(dsb[c]);
+              for (int c = 0; c < 2; ++c) p.ds_words[static_cast<size_t>(ws_tile) * 16 + (2 * half + c) * 4 + quad] = static_cast<uint8_t>(dsb[c]);
             }
           }
           tmem_wait_st();
@@ -521,8 +519,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       tc_fence_after();
       // two warps per lane quadrant: each writes 64 columns of every 128-column slice of the accumulators
 #pragma unroll 1
-      for (int s = 0; s < CH * C::kSub; ++s) {
-        const int col = 128 * (s / CH) + C::kCols * half + 32 * (s % CH);
+      for (int s = 0; s < 2 * C::kSub; ++s) {
+        const int col = 128 * (s / 2) + 64 * half + 32 * (s % 2);
         uint32_t rr[32];
         if (DV) {
           tmem_ld32(tmem + lane_base + C::kColDv + col, rr);
@@ -544,17 +542,14 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
   if (warp == C::kComputeWarps) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-constexpr int kKvGroups = 2;       // compute warpgroups (8 warps): with four, each warp's fixed work per tile is done sixteen times
-                                   // (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256 the two are equal
-
 // How dK and dV of a key tile are made: by one CTA; by two, both kinds in one grid, the longer one (dK) first; or dK here and dV
 // from the P^T tiles that the launch leaves in the workspace.
 enum KvForm { kKvOne, kKvRoles, kKvDkAndP };
 
 template <int D, int Form>
 struct KvLaunch {
-  using Dk = KvCfg<D, Form == kKvOne, true, kKvGroups, Form == kKvDkAndP>;
-  using Dv = KvCfg<D, true, Form == kKvOne, kKvGroups>;
+  using Dk = KvCfg<D, Form == kKvOne, true, Form == kKvDkAndP>;
+  using Dv = KvCfg<D, true, Form == kKvOne>;
   static constexpr int kThreads = Dk::kThreads;
   static constexpr int kSmemBytes = Dk::kSmemBytes > Dv::kSmemBytes ? Dk::kSmemBytes : Dv::kSmemBytes;
 };
@@ -564,10 +559,10 @@ __global__ void __launch_bounds__(KvLaunch<D, Form>::kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_p, const BwdParams p) {
-  if constexpr (Form == kKvOne) dkdv_tile<D, true, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else if constexpr (Form == kKvDkAndP) dkdv_tile<D, false, true, DS32, kKvGroups, true>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else dkdv_tile<D, true, false, DS32, kKvGroups>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  if constexpr (Form == kKvOne) dkdv_tile<D, true, true, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else if constexpr (Form == kKvDkAndP) dkdv_tile<D, false, true, DS32, true>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else dkdv_tile<D, true, false, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
 }
 
 template <int D, int Form, bool DS32>

@@ -11,10 +11,10 @@
 
 namespace dm {
 
-// kGroups compute warpgroups share a tile (128 / kGroups query columns per thread; thread = key row = TMEM lane), then the
-// MMA, TMA, vector and store warps.  S^T and dP^T are double-buffered in TMEM (2 x (128 + 128) columns) and nothing else is
+// Four compute warpgroups share a tile (thread = key row = TMEM lane, and one block of 32 queries; eight warps with two blocks
+// each take as long), then the MMA, TMA, vector and store warps.  S^T and dP^T are double-buffered in TMEM (2 x (128 + 128) columns) and nothing else is
 // there, so the MMAs of the next tile run under the arithmetic of this one and a Q / dO stage is free as soon as they are done.
-template <int D, int G>
+template <int D>
 struct TilesCfg {
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
@@ -22,7 +22,7 @@ struct TilesCfg {
   static constexpr int kKvBufs = (D == 128) ? 2 : 1;
   static constexpr int kStages = (D == 128) ? 2 : 1;
   static constexpr int kVecs = 4;
-  static constexpr int kComputeWarps = 4 * G, kCh = 4 / G, kCols = 128 / G;
+  static constexpr int kComputeWarps = 16;
   static constexpr int kThreads = (kComputeWarps + 4) * 32;
   static constexpr int kSmemK = 0;                                        // [kKvBufs] K, V
   static constexpr int kSmemQ = kKvBufs * 2 * kTileBytes;                 // [kStages]
@@ -75,12 +75,12 @@ struct TileWalk {
   }
 };
 
-template <int D, int G, bool DS32>
-__global__ void __launch_bounds__(TilesCfg<D, G>::kThreads, 1)
+template <int D, bool DS32>
+__global__ void __launch_bounds__(TilesCfg<D>::kThreads, 1)
 bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_p, const BwdParams p) {
-  using C = TilesCfg<D, G>;
+  using C = TilesCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemBar);
   uint64_t* kv_full = bars + 0;      // [2] K and V landed
@@ -263,11 +263,10 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else {
     // ------------------------------------------------------------------------------------------ compute warps
     // Operation for operation the arithmetic of dkdv_tile (dm_bwd_kv.cu); the codes go to shared memory instead of TMEM.
-    constexpr int CH = C::kCh;
-    const int part = warp >> 2;                        // query columns [kCols part, kCols part + kCols) of every tile
+    const int part = warp >> 2;                        // query block of every tile: columns [32 part, 32 part + 32)
     const int quad = warp & 3;                         // lane quadrant = 32-key block of the dS scale
     const int r = tid & 127;                           // key row inside the tile = TMEM lane
-    const uint32_t t_lane = tmem + (static_cast<uint32_t>(quad * 32) << 16) + C::kCols * part;
+    const uint32_t t_lane = tmem + (static_cast<uint32_t>(quad * 32) << 16) + 32 * part;
     const int nblk = p.N / 32;
     const uint32_t vec_a = smem_u32(smem + C::kSmemVec), xch_a = smem_u32(smem + C::kSmemXch);
     const uint32_t out_a = smem_u32(smem + C::kSmemOut) + r * 128;
@@ -287,23 +286,19 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const size_t tile = w.tile;
       w.next(p, n_t, rep);
       if (i + 1 < n_it) fetch();
-      const uint32_t va = vec_a + vs * C::kVecBytes + 4 * C::kCols * part, sc = vec_a + vs * C::kVecBytes + 4 * CH * part;
+      const uint32_t va = vec_a + vs * C::kVecBytes + 128 * part, sc = vec_a + vs * C::kVecBytes + 4 * part;
       const uint32_t t_s = t_lane + 256 * buf, o_row = out_a + buf * 2 * C::kCodeBytes;
-      float2 pr[CH][16];                               // P, then -dS
-      float qs_c[CH], dos_c[CH], am[CH];
-      uint32_t xv = 0, dsb[CH];
+      float2 pr[16];                                   // P, then -dS
+      float dos_c, am;
+      uint32_t xv = 0;
       if (ok) ok = wait_warp(vec_ok + vs, (i / C::kVecs) & 1, abort_flag);
       if (ok) ok = wait_warp(bar_s + buf, ph, abort_flag);
       if (ok) {
         tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          qs_c[c] = lds_f(sc + C::kVecQs + 4 * c);
-          dos_c[c] = lds_f(sc + C::kVecDos + 4 * c);
-        }
-        uint32_t rs[CH][32];
-#pragma unroll
-        for (int c = 0; c < CH; ++c) tmem_ld32(t_s + 32 * c, rs[c]);
+        const float qs_c = lds_f(sc + C::kVecQs);
+        dos_c = lds_f(sc + C::kVecDos);
+        uint32_t rs[32];
+        tmem_ld32(t_s, rs);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
@@ -311,100 +306,77 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (i >= 2) ok = wait_warp(stage_free + buf, ph ^ 1, abort_flag);     // the tile's staging is free
         if (diag) {
 #pragma unroll
-          for (int c = 0; c < CH; ++c)
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (r > C::kCols * part + 32 * c + e) rs[c][e] = 0xff800000u;   // -inf: key index above the query index
+          for (int e = 0; e < 32; ++e)
+            if (r > 32 * part + e) rs[e] = 0xff800000u;                        // -inf: key index above the query index
         }
+        const float2 cc = splat2((ks_row * qs_c) * kLog2e);
+        float pm0 = 0.f, pm1 = 0.f;
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          const float2 cc = splat2((ks_row * qs_c[c]) * kLog2e);
-          float pm0 = 0.f, pm1 = 0.f;
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float4 l4 = lds_f4(va + C::kVecLse + 128 * c + 8 * e);     // -lse * log2e
-            pr[c][e] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e]), __uint_as_float(rs[c][2 * e + 1])), cc, make_float2(l4.x, l4.y)));
-            pr[c][e + 1] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e + 2]), __uint_as_float(rs[c][2 * e + 3])), cc, make_float2(l4.z, l4.w)));
-            pm0 = max3(pm0, pr[c][e].x, pr[c][e].y);
-            pm1 = max3(pm1, pr[c][e + 1].x, pr[c][e + 1].y);
-          }
-          // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread and block; 16-byte chunk j of row r of the
-          // staging tile at chunk j ^ (r % 8) (128-byte swizzle)
-          const uint32_t psb = pow2_sb(fmaxf(pm0, pm1), 0u);
-          uint32_t wd[8];
-          codes32(pr[c], sb_to_inv(psb), wd);
-          const int j = 2 * CH * part + 2 * c;
-          sts_u4(o_row + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
-          sts_u4(o_row + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
-          xv |= sb_mul(psb, scale_to_sb(dos_c[c])) << (8 * c);
+        for (int e = 0; e < 16; e += 2) {
+          const float4 l4 = lds_f4(va + C::kVecLse + 8 * e);     // -lse * log2e
+          pr[e] = ex2_2(fma2(make_float2(__uint_as_float(rs[2 * e]), __uint_as_float(rs[2 * e + 1])), cc, make_float2(l4.x, l4.y)));
+          pr[e + 1] = ex2_2(fma2(make_float2(__uint_as_float(rs[2 * e + 2]), __uint_as_float(rs[2 * e + 3])), cc, make_float2(l4.z, l4.w)));
+          pm0 = max3(pm0, pr[e].x, pr[e].y);
+          pm1 = max3(pm1, pr[e + 1].x, pr[e + 1].y);
         }
+        // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread; 16-byte chunk j of row r of the staging tile
+        // at chunk j ^ (r % 8) (128-byte swizzle)
+        const uint32_t psb = pow2_sb(fmaxf(pm0, pm1), 0u);
+        uint32_t wd[8];
+        codes32(pr, sb_to_inv(psb), wd);
+        const int j = 2 * part;
+        sts_u4(o_row + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
+        sts_u4(o_row + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
+        xv = sb_mul(psb, scale_to_sb(dos_c));
         if (ok) ok = wait_warp(bar_dp + buf, ph, abort_flag);
       }
       if (ok) {
         tc_fence_after();
-        uint32_t rd[CH][32];
-#pragma unroll
-        for (int c = 0; c < CH; ++c) tmem_ld32(t_s + 128 + 32 * c, rd[c]);
+        uint32_t rd[32];
+        tmem_ld32(t_s + 128, rd);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(dp_free + buf);
+        // -dS = P (delta - dP_acc a): a is a power of two, so the product is exact; the sign is undone by the codes' scale
+        const float2 na = splat2(-(vs_row * dos_c));
+        float am0 = 0.f, am1 = 0.f;
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          // -dS = P (delta - dP_acc a): a is a power of two, so the product is exact; the sign is undone by the codes' scale
-          const float2 na = splat2(-(vs_row * dos_c[c]));
-          float am0 = 0.f, am1 = 0.f;
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float4 d4 = lds_f4(va + C::kVecDelta + 128 * c + 8 * e);
-            const float2 t0 = fma2(make_float2(__uint_as_float(rd[c][2 * e]), __uint_as_float(rd[c][2 * e + 1])), na, make_float2(d4.x, d4.y));
-            const float2 t1 = fma2(make_float2(__uint_as_float(rd[c][2 * e + 2]), __uint_as_float(rd[c][2 * e + 3])), na, make_float2(d4.z, d4.w));
-            pr[c][e] = mul2(pr[c][e], t0);
-            pr[c][e + 1] = mul2(pr[c][e + 1], t1);
-            am0 = max3(am0, fabsf(pr[c][e].x), fabsf(pr[c][e].y));
-            am1 = max3(am1, fabsf(pr[c][e + 1].x), fabsf(pr[c][e + 1].y));
-          }
-          am[c] = fmaxf(am0, am1);
+        for (int e = 0; e < 16; e += 2) {
+          const float4 d4 = lds_f4(va + C::kVecDelta + 8 * e);
+          const float2 t0 = fma2(make_float2(__uint_as_float(rd[2 * e]), __uint_as_float(rd[2 * e + 1])), na, make_float2(d4.x, d4.y));
+          const float2 t1 = fma2(make_float2(__uint_as_float(rd[2 * e + 2]), __uint_as_float(rd[2 * e + 3])), na, make_float2(d4.z, d4.w));
+          pr[e] = mul2(pr[e], t0);
+          pr[e + 1] = mul2(pr[e + 1], t1);
+          am0 = max3(am0, fabsf(pr[e].x), fabsf(pr[e].y));
+          am1 = max3(am1, fabsf(pr[e + 1].x), fabsf(pr[e + 1].y));
         }
-        if (!DS32) {
-          float m = am[0];
-#pragma unroll
-          for (int c = 1; c < CH; ++c) m = fmaxf(m, am[c]);
-          m = warp_max(m);
-          if ((tid & 31) == 0) sts_f(xch_a + 4 * (buf * 16 + warp), m);
-        }
+        am = warp_max(fmaxf(am0, am1));
+        if (!DS32 && (tid & 31) == 0) sts_f(xch_a + 4 * (buf * 16 + warp), am);
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(vec_empty + vs);
       }
       // one dS scale per (128 queries x this quadrant's 32 keys): the warps of the quadrant meet here (reached for every tile,
-      // also after a failed wait).  With 32 x 32 blocks the warp's own maxima are the blocks'.
-      if (!DS32 && G > 1) bar_sync(1 + quad, 32 * G);
+      // also after a failed wait).  With 32 x 32 blocks the warp's own maximum is the block's.
+      if (!DS32) bar_sync(1 + quad, 128);
       if (ok) {
-        float mx = 0.f;
         if (!DS32) {
-          mx = lds_f(xch_a + 4 * (buf * 16 + quad));
+          am = lds_f(xch_a + 4 * (buf * 16 + quad));
 #pragma unroll
-          for (int g = 1; g < G; ++g) mx = fmaxf(mx, lds_f(xch_a + 4 * (buf * 16 + 4 * g + quad)));
+          for (int g = 1; g < 4; ++g) am = fmaxf(am, lds_f(xch_a + 4 * (buf * 16 + 4 * g + quad)));
         }
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          dsb[c] = pow2_sb(DS32 ? warp_max(am[c]) : mx, 127u);
-          uint32_t wd[8];
-          codes32(pr[c], -sb_to_inv(dsb[c]), wd);
-          const int j = 2 * CH * part + 2 * c;
-          sts_u4(o_row + C::kCodeBytes + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
-          sts_u4(o_row + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
-        }
+        const uint32_t dsb = pow2_sb(am, 127u);
+        uint32_t wd[8];
+        codes32(pr, -sb_to_inv(dsb), wd);
+        const int j = 2 * part;
+        sts_u4(o_row + C::kCodeBytes + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
+        sts_u4(o_row + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
         fence_async_smem();
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(staged + buf);
         // the scale bytes last: global stores that are under way would hold up the proxy fence
-        if (CH == 2) *reinterpret_cast<uint16_t*>(p.p_words + tile * 512 + r * 4 + 2 * part) = static_cast<uint16_t>(xv);   // [key][query block]
-        else p.p_words[tile * 512 + r * 4 + part] = static_cast<uint8_t>(xv);
-        if ((tid & 31) == 0) {                         // [query block][key block]
-#pragma unroll
-          for (int c = 0; c < CH; ++c) p.ds_words[tile * 16 + (CH * part + c) * 4 + quad] = static_cast<uint8_t>(dsb[c]);
-        }
+        p.p_words[tile * 512 + r * 4 + part] = static_cast<uint8_t>(xv);                              // [key][query block]
+        if ((tid & 31) == 0) p.ds_words[tile * 16 + part * 4 + quad] = static_cast<uint8_t>(dsb);     // [query block][key block]
       }
     }
     if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInTiles);
@@ -414,17 +386,15 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp == C::kComputeWarps) tmem_dealloc(tmem, 512);
 }
 
-constexpr int kTilesGroups = 4;
-
 template <int D, bool DS32>
 static cudaError_t launch_tiles_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                                   const CUtensorMap& tds, const CUtensorMap& tp, const BwdParams& p, cudaStream_t stream) {
-  using C = TilesCfg<D, kTilesGroups>;
+  using C = TilesCfg<D>;
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_tiles_kernel<D, kTilesGroups, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(bwd_tiles_kernel<D, DS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     done[dev] = true;
   }
@@ -432,7 +402,7 @@ static cudaError_t launch_tiles_t(const CUtensorMap& tq, const CUtensorMap& tk, 
   const int total = p.B * p.H * (p.causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
   const int sms = sm_count();
   count_launch();
-  return launch_chained(bwd_tiles_kernel<D, kTilesGroups, DS32>, total < sms ? total : sms, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo,
+  return launch_chained(bwd_tiles_kernel<D, DS32>, total < sms ? total : sms, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo,
                         tds, tp, p);
 }
 
