@@ -12,6 +12,7 @@
 //   P^T codes: power-of-two scale per (key, 32 queries), amax 0 -> byte 0;   SFA_dV = p_sb (+) dos_sb
 //   dS codes:  power-of-two scale per (128 queries x 32 keys), amax 0 -> scale 1;  SFA_dK = ds_sb (+) qs_sb.
 #include <cuda_bf16.h>
+#include "dm_bwd_math.cuh"
 #include "dm_common.cuh"
 #include "dm_kernels.h"
 
@@ -381,29 +382,15 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const float2 cc = splat2((ks_row * (c ? qs2.y : qs2.x)) * kLog2e);
-          float pm0 = 0.f, pm1 = 0.f;
           if (PO && c == 0 && i > 0) ok = wait_warp(po_free, ph ^ 1, abort_flag);
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float4 l4 = lds_f4(va + C::kVecLse + 128 * c + 8 * e);     // -lse * log2e
-            pr[c][e] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e]), __uint_as_float(rs[c][2 * e + 1])), cc, make_float2(l4.x, l4.y)));
-            pr[c][e + 1] = ex2_2(fma2(make_float2(__uint_as_float(rs[c][2 * e + 2]), __uint_as_float(rs[c][2 * e + 3])), cc, make_float2(l4.z, l4.w)));
-            if (DV || PO) {
-              pm0 = max3(pm0, pr[c][e].x, pr[c][e].y);
-              pm1 = max3(pm1, pr[c][e + 1].x, pr[c][e + 1].y);
-            }
-          }
+          const float pm = p_block(rs[c], cc, va + C::kVecLse + 128 * c, pr[c]);
           if (DV || PO) {
             // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread and block
-            const uint32_t psb = pow2_sb(fmaxf(pm0, pm1), 0u);
+            const uint32_t psb = pow2_sb(pm, 0u);
             uint32_t w[8];
             codes32(pr[c], sb_to_inv(psb), w);
             if (DV) tmem_st8(t_s + C::kColCodes + 8 * c, w);
-            if (PO) {                                      // as a [key][query] tile, like the dS^T codes below
-              const int j = 4 * half + 2 * c;
-              sts_u4(ws_a + C::kCodeBytes + ((j ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
-              sts_u4(ws_a + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
-            }
+            if (PO) stage_codes(ws_a + C::kCodeBytes, r, 2 * half + c, w);     // like the dS^T codes below
             xv |= sb_mul(psb, scale_to_sb(c ? dos2.y : dos2.x)) << (8 * c);
           }
         }
@@ -439,20 +426,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          // -dS = P (delta - dP_acc a): a is a power of two, so the product is exact; the sign is undone by the codes' scale
           const float2 na = splat2(-(vs_row * (c ? dos2.y : dos2.x)));
-          float am0 = 0.f, am1 = 0.f;
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float4 d4 = lds_f4(va + C::kVecDelta + 128 * c + 8 * e);
-            const float2 t0 = fma2(make_float2(__uint_as_float(rd[c][2 * e]), __uint_as_float(rd[c][2 * e + 1])), na, make_float2(d4.x, d4.y));
-            const float2 t1 = fma2(make_float2(__uint_as_float(rd[c][2 * e + 2]), __uint_as_float(rd[c][2 * e + 3])), na, make_float2(d4.z, d4.w));
-            pr[c][e] = mul2(pr[c][e], t0);
-            pr[c][e + 1] = mul2(pr[c][e + 1], t1);
-            am0 = max3(am0, fabsf(pr[c][e].x), fabsf(pr[c][e].y));
-            am1 = max3(am1, fabsf(pr[c][e + 1].x), fabsf(pr[c][e + 1].y));
-          }
-          am[c] = fmaxf(am0, am1);
+          am[c] = neg_ds_block(rd[c], na, va + C::kVecDelta + 128 * c, pr[c]);
         }
         if (!DS32) {
           am[0] = warp_max(fmaxf(am[0], am[1]));
@@ -478,13 +453,8 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
             uint32_t w[8];
             codes32(pr[c], -sb_to_inv(dsb[c]), w);
             tmem_st8(t_dp + C::kColCodes + 8 * c, w);
-            if (p.ds_codes != nullptr) {
-              // the same codes as a [key][query] tile in 128-byte-swizzled shared memory (16-byte chunk j of row r at
-              // chunk j ^ (r % 8)), which the MMA warp stores to the workspace for pass 2
-              const int j = 4 * half + 2 * c;
-              sts_u4(ws_row + ((j ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
-              sts_u4(ws_row + (((j + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
-            }
+            // the same codes as a [key][query] tile, which the MMA warp stores to the workspace for pass 2
+            if (p.ds_codes != nullptr) stage_codes(ws_row, r, 2 * half + c, w);
           }
           const uint32_t xk = sb_mul(dsb[0], scale_to_sb(qs2.x)) | (sb_mul(dsb[1], scale_to_sb(qs2.y)) << 8);
           tmem_st4(t_dp + C::kColXk, xk, xk, xk, xk);

@@ -6,6 +6,7 @@
 // 32 tiles on 148 SMs.  Here the tiles are dealt out evenly, and what stays a chain is the accumulation alone, at about a
 // fifth of the time per tile.  The arithmetic, the order of every sum and so the bits are those of the key-stationary kernel.
 #include <cuda_bf16.h>
+#include "dm_bwd_math.cuh"
 #include "dm_common.cuh"
 #include "dm_kernels.h"
 
@@ -262,7 +263,7 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (!ok) raise_abort(abort_flag, p.status, kStatusTimeoutMma + kInTiles);
   } else {
     // ------------------------------------------------------------------------------------------ compute warps
-    // Operation for operation the arithmetic of dkdv_tile (dm_bwd_kv.cu); the codes go to shared memory instead of TMEM.
+    // As in dkdv_tile (dm_bwd_kv.cu), but the codes go to shared memory instead of TMEM.
     const int part = warp >> 2;                        // query block of every tile: columns [32 part, 32 part + 32)
     const int quad = warp & 3;                         // lane quadrant = 32-key block of the dS scale
     const int r = tid & 127;                           // key row inside the tile = TMEM lane
@@ -309,24 +310,12 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           for (int e = 0; e < 32; ++e)
             if (r > 32 * part + e) rs[e] = 0xff800000u;                        // -inf: key index above the query index
         }
-        const float2 cc = splat2((ks_row * qs_c) * kLog2e);
-        float pm0 = 0.f, pm1 = 0.f;
-#pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-          const float4 l4 = lds_f4(va + C::kVecLse + 8 * e);     // -lse * log2e
-          pr[e] = ex2_2(fma2(make_float2(__uint_as_float(rs[2 * e]), __uint_as_float(rs[2 * e + 1])), cc, make_float2(l4.x, l4.y)));
-          pr[e + 1] = ex2_2(fma2(make_float2(__uint_as_float(rs[2 * e + 2]), __uint_as_float(rs[2 * e + 3])), cc, make_float2(l4.z, l4.w)));
-          pm0 = max3(pm0, pr[e].x, pr[e].y);
-          pm1 = max3(pm1, pr[e + 1].x, pr[e + 1].y);
-        }
-        // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread; 16-byte chunk j of row r of the staging tile
-        // at chunk j ^ (r % 8) (128-byte swizzle)
-        const uint32_t psb = pow2_sb(fmaxf(pm0, pm1), 0u);
+        const float pm = p_block(rs, splat2((ks_row * qs_c) * kLog2e), va + C::kVecLse, pr);
+        // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread
+        const uint32_t psb = pow2_sb(pm, 0u);
         uint32_t wd[8];
         codes32(pr, sb_to_inv(psb), wd);
-        const int j = 2 * part;
-        sts_u4(o_row + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
-        sts_u4(o_row + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
+        stage_codes(o_row, r, part, wd);
         xv = sb_mul(psb, scale_to_sb(dos_c));
         if (ok) ok = wait_warp(bar_dp + buf, ph, abort_flag);
       }
@@ -338,20 +327,7 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(dp_free + buf);
-        // -dS = P (delta - dP_acc a): a is a power of two, so the product is exact; the sign is undone by the codes' scale
-        const float2 na = splat2(-(vs_row * dos_c));
-        float am0 = 0.f, am1 = 0.f;
-#pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-          const float4 d4 = lds_f4(va + C::kVecDelta + 8 * e);
-          const float2 t0 = fma2(make_float2(__uint_as_float(rd[2 * e]), __uint_as_float(rd[2 * e + 1])), na, make_float2(d4.x, d4.y));
-          const float2 t1 = fma2(make_float2(__uint_as_float(rd[2 * e + 2]), __uint_as_float(rd[2 * e + 3])), na, make_float2(d4.z, d4.w));
-          pr[e] = mul2(pr[e], t0);
-          pr[e + 1] = mul2(pr[e + 1], t1);
-          am0 = max3(am0, fabsf(pr[e].x), fabsf(pr[e].y));
-          am1 = max3(am1, fabsf(pr[e + 1].x), fabsf(pr[e + 1].y));
-        }
-        am = warp_max(fmaxf(am0, am1));
+        am = warp_max(neg_ds_block(rd, splat2(-(vs_row * dos_c)), va + C::kVecDelta, pr));
         if (!DS32 && (tid & 31) == 0) sts_f(xch_a + 4 * (buf * 16 + warp), am);
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(vec_empty + vs);
@@ -368,9 +344,7 @@ bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const uint32_t dsb = pow2_sb(am, 127u);
         uint32_t wd[8];
         codes32(pr, -sb_to_inv(dsb), wd);
-        const int j = 2 * part;
-        sts_u4(o_row + C::kCodeBytes + ((j ^ (r & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
-        sts_u4(o_row + C::kCodeBytes + (((j + 1) ^ (r & 7)) << 4), wd[4], wd[5], wd[6], wd[7]);
+        stage_codes(o_row + C::kCodeBytes, r, part, wd);
         fence_async_smem();
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(staged + buf);
