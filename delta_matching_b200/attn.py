@@ -1,8 +1,9 @@
 """The autograd route and the input contract.
 
-Eager calls on plain CUDA tensors run in C++ (csrc/dm_torch.cpp: the same checks, the same kernels, one call of the C ABI per
+Eager calls on plain CUDA tensors run in C++ (csrc/dm_torch.cpp: the same checks and results, one call of the C ABI per
 pass): at short sequences the host time of the Python route below is several times the kernels' own.  The Python route
-serves tracing compilers, tensor subclasses and function transforms, and raises the contract's exceptions.
+serves tracing compilers, tensor subclasses and function transforms, and raises the contract's exceptions.  Its backward is the
+op layer's, the key-stationary kernels for every shape; the C++ route's chooses between forms with the same bits.
 
 `dm_attn_func_bhnd(q, k, v, causal, softmax_scale, delta_mode)` on (B, H, N, D) inputs returns (B, N, H, D), as
 delta_matching/attn.py:121-127 does.  Forward: producers (codes, scales, K mean) then the forward kernel.  Backward: the

@@ -1,9 +1,10 @@
-// Backward pass 2: dQ = dS K from the quantised dS tiles that the dK / dV kernel left in a workspace.
+// Streaming pass of the backward: dQ = dS K from the quantised dS tiles that an earlier kernel left in a workspace, and, where it
+// left P^T tiles too, dV, or dV and dK.
 //
 // Reference structure: pass 1 writes dS codes, pass 2 multiplies them with K
 // (csrc/fq8_dq_pass2_hd128.h:407-442, launched from csrc/flash_bwd_fp8v10_launch.h:158-163).  The alternative without a
 // workspace (dm_bwd.cu: bwd_dq_kernel) recomputes S, dP and the exponentials per tile; this kernel only streams
-// 16 KiB dS^T tiles and K tiles through one block-scaled MMA chain per tile, so it is bound by the L2 / HBM stream.
+// 16 KiB code tiles and operand tiles through one block-scaled MMA chain per tile, so it is bound by the L2 / HBM stream.
 //
 // Workspace: tile (head bh, query tile qt, key tile kt) at index (bh * n_t + qt) * n_t + kt holds 128 x 128 e4m3 codes
 // as [key][query] (the layout the dK chain consumes), followed after all tiles by four 32-bit words per tile: word b
@@ -13,12 +14,14 @@
 //
 // Behind the tile-parallel pass (dm_bwd_tiles.cu) the same kernel also makes dV = sum P^T dO and dK = sum dS^T Q of
 // every (key tile, kv head), over the group's heads and their query tiles in the order of the key-stationary kernel: there
-// the code tile is the A operand as it lies, K-major (M = keys), and dO / Q the MN-major B operand.
+// the code tile is the A operand as it lies, K-major (M = keys), and dO / Q the MN-major B operand.  P^T tiles have a word per key row
+// (byte = query block), ready to use.  Behind the head_dim-256 DK role (dm_bwd_kv.cu) it makes dV and dQ.
 //
-// One persistent CTA per SM, 320 threads: warps 0-3 write the per-tile scale words into TMEM (byte j = dS scale x K
-// scale of key block j; warp b writes the word of query block b into its 32 rows), warps 4-7 write dQ out (at head_dim 128 two accumulators alternate
-// between items; at head_dim 256 one accumulator fills the columns, and an item's first chain waits for the read-out
-// of the previous item), warp 8 TMA, warp 9 MMA.  Items = (query tile, head), most key tiles first.
+// One persistent CTA per SM, 320 threads: warps 0-3 write the per-tile scale words into TMEM (code scale x operand scale of the four
+// blocks that a row is summed over; warp b writes rows [32 b, 32 b + 32), whose words are one and the same for dQ and dK), warps
+// 4-7 write the finished accumulator out (at head_dim 128 two accumulators alternate between items; at head_dim 256 one
+// accumulator fills the columns, and an item's first chain waits for the read-out of the previous item), warp 8 TMA, warp 9 MMA.
+// Items = (query tile, head) for dQ and (key tile, kv head) for dK and dV, in the order of stream_item.
 #include <cuda_bf16.h>
 #include "dm_common.cuh"
 #include "dm_kernels.h"

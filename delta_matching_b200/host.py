@@ -4,7 +4,8 @@
 the results are bit-identical to one un-chunked call) and runs three streams: host->device copies of chunk c + 1,
 kernels of chunk c and device->host copies of chunk c - 1 overlap, which hides the compute and one direction of the
 PCIe traffic behind the other.  The device work is the op sequence of `dm_attn_func` and its backward
-(delta_matching_b200/attn.py; reference surface: delta_matching/__init__.py:52-77), with the same input checks.
+(delta_matching_b200/attn.py; reference surface: delta_matching/__init__.py:52-77), with the same input checks and the same
+results.
 """
 from __future__ import annotations
 
@@ -47,8 +48,8 @@ def attn_step_host(q, k, v, do, *, causal=True, mode="matched", softmax_scale=No
     moved with strided copies; the default aims at eight.  Argument errors are those of `dm_attn_func`.
 
     Per chunk: q, k, v are copied in and the forward starts while dO is still on its way; O is copied out while the
-    backward runs; dQ, dK, dV follow.  The kernels are the ones `dm_attn_func` and its backward launch, in the same
-    order (the op layer is called directly, there is no autograd graph)."""
+    backward runs; dQ, dK, dV follow.  The op layer is called directly, there is no autograd graph; its backward is the
+    key-stationary one for every shape (see ops.bwd_fp8)."""
     from . import ops
     from .attn import _check_inputs
     for name, t in (("q", q), ("k", k), ("v", v), ("do", do)):

@@ -317,9 +317,11 @@ def bwd_fp8(q8, k8, v8, do8, qs, ks, vs, dos, lse, delta, causal: bool, identity
     ds32=True scales dS per (32 queries x 32 keys) instead of (128 x 32) (numerics arm "sm100-mx-ds32", see NUMERICS).
 
     Without the identity probe the two-pass form runs: the dK / dV kernel leaves the dS codes in a workspace and dQ
-    streams them (bit-identical to the recomputing kernel).  The workspace is allocated here unless
-    `workspace` (uint8, at least bwd_workspace_bytes) is given; when it would exceed DM_BWD_WORKSPACE_MB the call is
-    split over (batch, kv-head group) ranges, and when a single group exceeds it the recomputing kernel runs."""
+    streams them (bit-identical to the recomputing kernel).  The eager route of dm_attn_func has further forms for small
+    problems and for head_dim 256 (dm_attn_bwd of the C ABI; the same bits), which this op does not take.  The workspace is
+    allocated here unless `workspace` (uint8, at least bwd_workspace_bytes) is given; when it would exceed
+    DM_BWD_WORKSPACE_MB the call is split over (batch, kv-head group) ranges, and when a single group exceeds it the
+    recomputing kernel runs."""
     dev = _cuda(q8, k8, v8, do8, qs, ks, vs, dos, lse, delta)
     _enter(dev)
     B, H, N, D = q8.shape

@@ -157,7 +157,7 @@ int dm_bwd_ws(const void* q8, const void* k8, const void* v8, const void* do8,
               void* workspace, int64_t workspace_bytes, int parts, int* status, void* stream);
 
 /* Whole passes: everything a forward, or a backward, of the attention layer launches, in one call (what the native PyTorch
- * path uses).  The kernels and their results are those of the separate entry points.  The caller vouches that
+ * path uses).  The results are those of the separate entry points, bit for bit; the backward's kernels may be others.  The caller vouches that
  * the pointers are memory of the current device, which is not looked up here; NULL and misaligned pointers (16 bytes), shapes
  * and strides are refused as everywhere.
  *
@@ -170,7 +170,9 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
                 void* q8, void* k8, void* v8, float* qs, float* ks, float* vs, float* kmean, void* workspace,
                 void* o, float* lse, int* status, void* stream);
 
-/* dm_attn_bwd = dm_quant_do, dm_delta, dm_bwd_ws with parts = 3.  o == NULL: the matched delta (dm_delta, or dm_delta_sum with
+/* dm_attn_bwd: what dm_quant_do, dm_delta and dm_bwd_ws with parts = 3 compute.  Small problems take a tile-parallel form that
+ * leaves P^T and dS^T tiles in the workspace and streams dQ, dK and dV from them, other head_dim-256 calls one that streams dV
+ * beside dQ, in ranges of batches or kv groups; dm_bwd_ws has neither.  o == NULL: the matched delta (dm_delta, or dm_delta_sum with
  * DM_ATTN_DELTA_SUM); o = the forward's contiguous (B, N, H, D) output: the stale delta.  do8, dos, delta are filled here;
  * dq, dk, dv are contiguous token-major.  workspace: dm_attn_bwd_workspace_bytes, 16-byte aligned.  flags: DM_DS_BLOCK32, DM_ATTN_DELTA_SUM, DM_ATTN_DELTA_ONLY (stop behind
  * do8, dos and delta: for callers that split the rest over several dm_bwd_ws calls; dq, dk, dv and workspace are unused). */

@@ -1,5 +1,5 @@
-"""The native eager route (csrc/dm_torch.cpp) against the Python route it stands in for: the same kernels on the same inputs,
-so the same bits, over layouts, head dims, modes, arms and a bounded workspace."""
+"""The native eager route (csrc/dm_torch.cpp) against the Python route it stands in for: the same bits over layouts, head dims,
+modes, arms and a bounded workspace, although its backward may take other kernels (tests/test_small_grids_gpu.py)."""
 import pytest
 import torch
 
