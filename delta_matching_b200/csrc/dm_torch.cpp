@@ -9,13 +9,14 @@
 //
 // The module does not link against the kernel library: bind() receives the addresses of the entry points from the
 // ctypes handle, so that DM_SO decides for both which library runs.  attn() returns None whenever a call is not one it
-// serves as it stands (a violated constraint, a tensor subclass, a functorch or dispatch-mode wrapper); the caller then
+// serves as it stands (a violated constraint, a tensor subclass, a functorch or dispatch-mode wrapper, a trace); the caller then
 // takes the Python route, which raises the contract's exceptions or serves the call.
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/dynamo/compiled_autograd.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/core/PythonFallbackKernel.h>
@@ -357,6 +358,8 @@ PyObject* attn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const Tensor *qp = nullptr, *kp = nullptr, *vp = nullptr;
   if (n != 8 || !plain_cuda_bf16(args[0], qp) || !plain_cuda_bf16(args[1], kp) || !plain_cuda_bf16(args[2], vp)) Py_RETURN_NONE;
   if (c10::impl::TorchDispatchModeTLS::any_modes_set() || !PyUnicode_Check(args[5])) Py_RETURN_NONE;
+  // torch.jit.trace records the Python route's autograd function; from here it would see a tensor from nowhere, a constant
+  if (torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const Tensor &q = *qp, &k = *kp, &v = *vp;
   const bool hm = args[7] == Py_True;
   const int causal = PyObject_IsTrue(args[4]);

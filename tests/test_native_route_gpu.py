@@ -55,3 +55,19 @@ def test_second_derivative_is_refused(oracle):
     (dq,) = torch.autograd.grad(o, leaves[:1], do.requires_grad_(), create_graph=True)
     with pytest.raises(RuntimeError, match="once_differentiable"):
         dq.sum().backward()
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("mode", ["matched", "stale"])
+def test_jit_trace_records_the_call(mode, grad, oracle):
+    """A traced function gives the eager result on inputs other than those it was traced with."""
+    from delta_matching_b200 import dm_attn_func
+    f = lambda q, k, v: 2.0 * dm_attn_func(q, k, v, causal=True, mode=mode)
+    one, two = (oracle.make_inputs(1, 256, 2, 2, 128, seed=s, device="cuda") for s in (63, 64))
+    traced = torch.jit.trace(f, [t.requires_grad_(grad) for t in one[:3]], check_trace=False)
+    got, want = ([t.detach().requires_grad_(grad) for t in two[:3]] for _ in range(2))
+    a, b = traced(*got), f(*want)
+    assert torch.equal(a, b)
+    if grad:
+        for x, y in zip(torch.autograd.grad(a, got, two[3]), torch.autograd.grad(b, want, two[3])):
+            assert torch.equal(x, y)
