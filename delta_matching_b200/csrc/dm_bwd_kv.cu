@@ -1,5 +1,6 @@
-// Backward pass 1 of delta-matching fp8 attention on sm_100a: dK and dV, key-stationary, bit-deterministic (one writer per
-// output element, fixed loop order, no atomics).
+// Backward pass 1 of delta-matching fp8 attention on sm_100a with dK and dV made by different CTAs, or dV elsewhere: head_dim 256, and
+// small grids at head_dim 128 (the others: dm_bwd_pipe.cu).  Key-stationary, bit-deterministic (one writer per output element, fixed loop
+// order, no atomics).
 //
 //   CTA = (128-key tile, kv head, batch); it walks the query heads of the GQA group and their 128-query tiles:
 //   dP^T = V8 dO8^T and S^T = K8 Q8^T (kind::f8f6f4), P^T codes and dS^T codes written to TMEM, dV += P^T dO and
@@ -19,42 +20,32 @@
 namespace dm {
 
 // Eight compute warps (two per SM quarter, up to 168 registers a thread) and four that issue.  A tile of 128 keys x 128 queries
-// is a chain: S^T MMA -> exponentials and P^T codes -> dP^T -> dS, block maximum, dS^T codes -> dV and dK MMAs.  S^T and dP^T
-// have TMEM columns of their own and nothing of the next tile waits for the end of this one:
-//   - a thread holds 64 values each of P and dP (one key row, 64 queries), so that both TMEM regions are in registers early and
-//     take the tile's codes and scale words: P^T codes over S^T, the scale words and the dS^T codes over dP^T;
-//   - the dV chain is issued behind the hand-off of the P^T codes and S^T of the next tile right behind it: both run under dS and its
-//     quantisation (an MMA's accumulator writes are ordered behind the operand reads of earlier MMAs of the same thread);
-//   - the dK chain and then dP^T of the next tile run under the next tile's exponentials.  Only here a completion is waited
-//     for: dP^T lands on the scale words, and for scale-factor reads the PTX ISA promises no order.
-// With sixteen warps on 32 queries each and one 128-column region that S^T and dP^T shared (what this kernel did before), every
-// link of the chain was exposed and the fixed work of a warp per tile was done sixteen times.
+// is a chain: S^T MMA -> exponentials and P^T codes -> dP^T -> dS, block maximum, dS^T codes -> dV or dK MMAs.  S^T and dP^T
+// have TMEM columns of their own; a thread holds 64 values each of P and dP (one key row, 64 queries), so that both TMEM regions are in
+// registers early.
 //
 // Head_dim 256: one accumulator fills 256 columns.  Either a key tile is two CTAs (and so it is in small grids at head_dim 128): a
 // DV role (S^T, P^T codes, dV; the columns of dP^T are a second S^T buffer, and the words lie beside the codes) and a DK role
-// (S^T, dP^T, dS codes, dK and the dS tiles for the workspace), each with the other half of the work compiled out.  Or, PO, the DK
-// role also leaves the P^T tiles in the workspace, and dV is streamed from them beside dQ (dm_bwd_p2.cu), which saves the
-// DV role's S^T and exponentials.
-template <int D, bool DV, bool DK, bool PO = false>
+// (S^T, dP^T, dS codes, dK and the dS tiles for the workspace; the scale words and the dS^T codes over dP^T), each with the other half of
+// the work compiled out.  Or, PO, the DK role also leaves the P^T tiles in the workspace, and dV is streamed from them beside dQ
+// (dm_bwd_p2.cu), which saves the DV role's S^T and exponentials.
+// DK: the DK role, else the DV role.
+template <int D, bool DK, bool PO = false>
 struct KvCfg {
-  static_assert(!PO || (DK && !DV), "P^T tiles go out of the DK role");
-  static_assert((D == 128 || D == 256) && (DV || DK) && !(D == 256 && DV && DK), "two accumulators of 256 columns fill the TMEM");
+  static_assert((D == 128 || D == 256) && (DK || !PO), "P^T tiles go out of the DK role");
   static constexpr int kSub = D / 128;                 // 128-byte-wide sub-tiles of an operand row
   static constexpr int kTileBytes = 128 * D;           // K, V, Q, dO tile
   static constexpr int kCodeBytes = 128 * 128;         // dS^T code tile (does not depend on head_dim)
   static constexpr int kStages = (D == 128) ? 4 : 2;
-  static constexpr int kComputeWarps = 8;              // with sixteen on one block of 32 queries each, a warp's fixed work per tile is
-                                                       // done sixteen times (B=4 N=4096 H=32: 861 instead of 818 us); at head_dim 256
-                                                       // the two are equal
+  static constexpr int kComputeWarps = 8;
   static constexpr int kThreads = (kComputeWarps + 4) * 32;
   static constexpr int kTmemCols = 512;
   static constexpr int kColS = 0, kColDp = 128;        // fp32 accumulators, 128 columns each
-  // What a warp writes over the 64 columns [64 h, 64 h + 64) that it has read, relative to the region:
-  static constexpr int kColCodes = 0;        // 64 h + 8 c: codes of query block 2 h + c (P^T over S^T, dS^T over dP^T)
-  static constexpr int kColXv = 16;          // 64 h + 16: 4 columns of the dV scale word of half h (byte c = block 2 h + c)
-  static constexpr int kColXk = 20;          // 64 h + 20: likewise, dK
+  // What a warp writes over the 64 columns [64 h, 64 h + 64) that it has read, relative to the region (DV role: S^T, DK role: dP^T):
+  static constexpr int kColCodes = 0;        // 64 h + 8 c: codes of query block 2 h + c
+  static constexpr int kColWord = 16;        // 64 h + 16: 4 columns of the scale word of half h (byte c = block 2 h + c)
   static constexpr int kColOne = 24;         // 4 columns of 0x7F7F7F7F (written by h = 0)
-  static constexpr int kColDv = 256, kColDk = (DV && DK) ? 384 : 256;
+  static constexpr int kColAcc = 256;        // dV or dK
   static constexpr int kSmemK = 0;
   static constexpr int kSmemV = kTileBytes;                          // the DV role has no V tile
   static constexpr int kSmemQ = DK ? 2 * kTileBytes : kTileBytes;    // [kStages]
@@ -85,10 +76,10 @@ __device__ __forceinline__ void store_bf16_row32(const uint32_t (&r)[32], __nv_b
 
 // DS32: the dS scale is taken per (32 queries x 32 keys), which is one 32-column block of one warp, instead of the contract's
 // (128 queries x 32 keys), for which the two warps of a key quadrant exchange their maxima.
-template <int D, bool DV, bool DK, bool DS32, bool PO = false>
+template <int D, bool DK, bool DS32, bool PO = false>
 __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                                           const CUtensorMap& tm_do, const CUtensorMap& tm_ds, const CUtensorMap& tm_p, const BwdParams& p) {
-  using C = KvCfg<D, DV, DK, PO>;
+  using C = KvCfg<D, DK, PO>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemBar);
   uint64_t* bar_kv = bars + 0;       // K and V landed
@@ -287,18 +278,15 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         if (!(ok = issue_s(i + 1))) break;
       }
       if (!(ok = DK ? wait_warp(bar_p, ph, abort_flag) : wait_warp((i & 1) ? bar_p1 : bar_p, (i >> 1) & 1, abort_flag))) break;
-      if (DV) {
-        if (!DK && !(ok = landed(full_d, i))) break;
+      if (!DK) {
+        if (!(ok = landed(full_d, i))) break;
         tc_fence_after();
-        const uint32_t b_lo = do_lo(i), region = tmem + (DK ? C::kColS : 128 * (i & 1));
-        const uint32_t words = DK ? tmem + C::kColDp : region;
+        const uint32_t b_lo = do_lo(i), region = tmem + 128 * (i & 1);
         if (elect_one()) {                               // dV += P^T dO
-          chain_acc(tmem + C::kColDv, region + C::kColCodes, words + C::kColXv, words + C::kColOne, b_lo, i == 0);
-          if (!DK) {
-            tc_commit(bar_done);
-            tc_commit(empty + i % C::kStages);
-            if (i == n_it - 1) tc_commit(bar_acc);
-          }
+          chain_acc(tmem + C::kColAcc, region + C::kColCodes, region + C::kColWord, region + C::kColOne, b_lo, i == 0);
+          tc_commit(bar_done);
+          tc_commit(empty + i % C::kStages);
+          if (i == n_it - 1) tc_commit(bar_acc);
         }
       }
       if (DK) {
@@ -307,7 +295,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         tc_fence_after();
         const uint32_t b_lo = q_lo(i);
         if (elect_one()) {                               // dK += dS^T Q
-          chain_acc(tmem + C::kColDk, tmem + C::kColDp + C::kColCodes, tmem + C::kColDp + C::kColXk, tmem + C::kColDp + C::kColOne, b_lo, i == 0);
+          chain_acc(tmem + C::kColAcc, tmem + C::kColDp + C::kColCodes, tmem + C::kColDp + C::kColWord, tmem + C::kColDp + C::kColOne, b_lo, i == 0);
           tc_commit(bar_done);
           tc_commit(empty + i % C::kStages);
           if (i == n_it - 1) tc_commit(bar_acc);
@@ -367,7 +355,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         tmem_ld32(t_s, rs[0]);
         tmem_ld32(t_s + 32, rs[1]);
         tmem_wait_ld();
-        if (!DV) {                                       // S^T of the next tile may land
+        if (DK) {                                        // S^T of the next tile may land
           tc_fence_before();
           __syncwarp();
           if ((tid & 31) == 0) mbar_arrive(bar_p);
@@ -384,18 +372,18 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
           const float2 cc = splat2((ks_row * (c ? qs2.y : qs2.x)) * kLog2e);
           if (PO && c == 0 && i > 0) ok = wait_warp(po_free, ph ^ 1, abort_flag);
           const float pm = p_block(rs[c], cc, va + C::kVecLse + 128 * c, pr[c]);
-          if (DV || PO) {
+          if (!DK || PO) {
             // P^T codes: one power-of-two scale per (key row, 32 queries) = per thread and block
             const uint32_t psb = pow2_sb(pm, 0u);
             uint32_t w[8];
             codes32(pr[c], sb_to_inv(psb), w);
-            if (DV) tmem_st8(t_s + C::kColCodes + 8 * c, w);
+            if (!DK) tmem_st8(t_s + C::kColCodes + 8 * c, w);
             if (PO) stage_codes(ws_a + C::kCodeBytes, r, 2 * half + c, w);     // like the dS^T codes below
             xv |= sb_mul(psb, scale_to_sb(c ? dos2.y : dos2.x)) << (8 * c);
           }
         }
         if (!DK) {                                       // DV role: the words go beside the codes, and that is the tile
-          tmem_st4(t_s + C::kColXv, xv, xv, xv, xv);
+          tmem_st4(t_s + C::kColWord, xv, xv, xv, xv);
           if (half == 0) tmem_st4(t_s + C::kColOne, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
           tmem_wait_st();
           tc_fence_before();
@@ -417,13 +405,6 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
         tmem_ld32(t_dp + 32, rd[1]);
         tmem_wait_ld();
         if (half == 0) tmem_st4(t_dp + C::kColOne, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
-        if (DV) {                                        // P^T codes and words are complete
-          tmem_st4(t_dp + C::kColXv, xv, xv, xv, xv);
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if ((tid & 31) == 0) mbar_arrive(bar_p);
-        }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const float2 na = splat2(-(vs_row * (c ? dos2.y : dos2.x)));
@@ -457,7 +438,7 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
             if (p.ds_codes != nullptr) stage_codes(ws_row, r, 2 * half + c, w);
           }
           const uint32_t xk = sb_mul(dsb[0], scale_to_sb(qs2.x)) | (sb_mul(dsb[1], scale_to_sb(qs2.y)) << 8);
-          tmem_st4(t_dp + C::kColXk, xk, xk, xk, xk);
+          tmem_st4(t_dp + C::kColWord, xk, xk, xk, xk);
           if (p.ds_codes != nullptr) {
             fence_async_smem();
             // scale bytes of the tile for pass 2, [query block][key block]
@@ -487,23 +468,16 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
       raise_abort(abort_flag, p.status, kStatusTimeoutCompute + kInDkDv);
     } else {
       tc_fence_after();
-      // two warps per lane quadrant: each writes 64 columns of every 128-column slice of the accumulators
+      // two warps per lane quadrant: each writes 64 columns of every 128-column slice of the accumulator
 #pragma unroll 1
       for (int s = 0; s < 2 * C::kSub; ++s) {
         const int col = 128 * (s / 2) + 64 * half + 32 * (s % 2);
         uint32_t rr[32];
-        if (DV) {
-          tmem_ld32(tmem + lane_base + C::kColDv + col, rr);
-          tmem_wait_ld();
-          store_bf16_row32(rr, p.dv + static_cast<int64_t>(b) * p.dv_sb + static_cast<int64_t>(key) * p.dv_sn +
-                                   static_cast<int64_t>(hk) * p.dv_sh + col);
-        }
-        if (DK) {
-          tmem_ld32(tmem + lane_base + C::kColDk + col, rr);
-          tmem_wait_ld();
-          store_bf16_row32(rr, p.dk + static_cast<int64_t>(b) * p.dk_sb + static_cast<int64_t>(key) * p.dk_sn +
-                                   static_cast<int64_t>(hk) * p.dk_sh + col);
-        }
+        tmem_ld32(tmem + lane_base + C::kColAcc + col, rr);
+        tmem_wait_ld();
+        __nv_bfloat16* out = DK ? p.dk + static_cast<int64_t>(b) * p.dk_sb + static_cast<int64_t>(key) * p.dk_sn + static_cast<int64_t>(hk) * p.dk_sh
+                                : p.dv + static_cast<int64_t>(b) * p.dv_sb + static_cast<int64_t>(key) * p.dv_sn + static_cast<int64_t>(hk) * p.dv_sh;
+        store_bf16_row32(rr, out + col);
       }
     }
   }
@@ -512,14 +486,14 @@ __device__ __forceinline__ void dkdv_tile(const CUtensorMap& tm_q, const CUtenso
   if (warp == C::kComputeWarps) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-// How dK and dV of a key tile are made: by one CTA; by two, both kinds in one grid, the longer one (dK) first; or dK here and dV
-// from the P^T tiles that the launch leaves in the workspace.
-enum KvForm { kKvOne, kKvRoles, kKvDkAndP };
+// How dK and dV of a key tile are made: by two CTAs, both kinds in one grid, the longer one (dK) first; or dK here and dV from the P^T
+// tiles that the launch leaves in the workspace.
+enum KvForm { kKvRoles, kKvDkAndP };
 
 template <int D, int Form>
 struct KvLaunch {
-  using Dk = KvCfg<D, Form == kKvOne, true, Form == kKvDkAndP>;
-  using Dv = KvCfg<D, true, Form == kKvOne>;
+  using Dk = KvCfg<D, true, Form == kKvDkAndP>;
+  using Dv = KvCfg<D, false>;
   static constexpr int kThreads = Dk::kThreads;
   static constexpr int kSmemBytes = Dk::kSmemBytes > Dv::kSmemBytes ? Dk::kSmemBytes : Dv::kSmemBytes;
 };
@@ -529,10 +503,9 @@ __global__ void __launch_bounds__(KvLaunch<D, Form>::kThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_p, const BwdParams p) {
-  if constexpr (Form == kKvOne) dkdv_tile<D, true, true, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else if constexpr (Form == kKvDkAndP) dkdv_tile<D, false, true, DS32, true>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else if (blockIdx.z == 0) dkdv_tile<D, false, true, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
-  else dkdv_tile<D, true, false, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  if constexpr (Form == kKvDkAndP) dkdv_tile<D, true, DS32, true>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else if (blockIdx.z == 0) dkdv_tile<D, true, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
+  else dkdv_tile<D, false, DS32>(tm_q, tm_k, tm_v, tm_do, tm_ds, tm_p, p);
 }
 
 template <int D, int Form, bool DS32>
@@ -562,7 +535,7 @@ cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk,
   if (D != 128) return (p.ds32 ? launch_kv_t<256, kKvRoles, true> : launch_kv_t<256, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
   if (2ll * p.B * p.Hk * (p.N / 128) <= sm_count())
     return (p.ds32 ? launch_kv_t<128, kKvRoles, true> : launch_kv_t<128, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
-  return (p.ds32 ? launch_kv_t<128, kKvOne, true> : launch_kv_t<128, kKvOne, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
+  return launch_bwd_pipe(tq, tk, tv, tdo, tds, p, stream);
 }
 
 cudaError_t launch_bwd_dk_and_p(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
