@@ -289,19 +289,19 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
 }
 
 // Which backward dm_attn_bwd runs (same results).  The key-stationary kernel takes as long as its longest chain, (H / Hk)
-// (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.7 us a tile; the tile-parallel
-// pair takes its share of all tiles at about 3.7 us.  Forward + backward, chain / tiles per SM: 16 (N=1024 H=8 Hk=2) 92 -> 60 us;
-// 4.6 (N=8192 H=4 Hk=1) 594 -> 440; 2.3 (N=16384 H=2 Hk=1) 810 -> 758; 2.2 (N=2048 H=32 Hk=8) 222 -> 214; 2.06 (B=4 N=1024 H=16 Hk=4) 139 ->
-// 134.5; 1.95 (N=2304 H=32 Hk=8) 254.8 -> 253.8; 1.9 (B=3 N=1536 H=16 Hk=4) 192.4 -> 192.8; 1.8 (N=5120 H=16 Hk=4) 528 -> 519; 1.76 (N=2560 H=32
-// Hk=8) 289 -> 298; 1.6 (N=2816 H=32 Hk=8) 333 -> 352; 1.5 (N=6144 H=16 Hk=4) 678 -> 737; 1.3 (B=3 N=1792 H=15 Hk=5) 202 -> 235.  Head_dim 256: 2.2
-// (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152 -> 143; 1.45 (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 ->
-// 495.  The lines are drawn at 2.0, where the two meet, and at 1.6, and at 2 GiB of workspace.  The workspace is the whole square of
-// tiles, of which a causal call touches half: at its edge (N=8192 H=16 Hk=1, ratio 4.6, 2.03 GiB) it sends calls back to the
-// key-stationary kernel that the tile-parallel one would win.
+// (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.6 us a tile; the tile-parallel
+// pair takes its share of all tiles at about 3.7 us.  Forward + backward in us, key-stationary -> tile-parallel by chain / tiles per SM:
+// 4.6 (N=8192 H=4 Hk=1) 593 -> 452; 3.0 (N=6144 H=8 Hk=2) 496 -> 435; 3.0 (N=4096 H=12 Hk=3) 346 -> 308; 2.7 (B=6 N=1024 H=8 Hk=2) 122.5 ->
+// 120; 2.29 (N=16384 H=2 Hk=1) 777 -> 758; 2.28 (N=8192 H=8 Hk=2) 689 -> 691; 2.24 (N=4096 H=16 Hk=4) 371 -> 376; 2.18 (N=2048 H=32 Hk=8) 213 ->
+// 218; 2.18 (B=2 N=2048 H=16 Hk=4) 212 -> 222; 2.06 (B=4 N=1024 H=16 Hk=4) 136.8 -> 138.8; 1.95 (N=2304 H=32 Hk=8) 245 -> 254; 1.8 (N=5120 H=16
+// Hk=4) 492 -> 516; 1.5 (B=2 N=3072 H=12 Hk=4) 269 -> 316.  Head_dim 256: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152
+// -> 143; 1.45 (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 -> 495.  The lines are drawn at 2.25, where the two meet, and at
+// 1.6, and at 2 GiB of workspace.  The workspace is the whole square of tiles, of which a causal call touches half: at its edge (N=8192
+// H=16 Hk=1, ratio 4.6, 2.03 GiB) it sends calls back to the key-stationary kernel that the tile-parallel one would win.
 static bool tile_parallel(int B, int N, int H, int Hk, int D, int causal) {
   const long long n_t = N / 128, tiles = static_cast<long long>(B) * H * (causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
   const long long chain = H / Hk * n_t;
-  return 10 * chain * dm::sm_count() >= (D == 128 ? 20 : 16) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
+  return 20 * chain * dm::sm_count() >= (D == 128 ? 45 : 32) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
 }
 
 // Workspace of `units` query heads with both tile sets: dS^T tiles, P^T tiles, dS words, P words.
