@@ -23,6 +23,7 @@
 // accumulator fills the columns, and an item's first chain waits for the read-out of the previous item), warp 8 TMA, warp 9 MMA.
 // Items = (query tile, head) for dQ and (key tile, kv head) for dK and dV, in the order of stream_item.
 #include <cuda_bf16.h>
+#include "dm_bwd_math.cuh"
 #include "dm_common.cuh"
 #include "dm_kernels.h"
 #include "dm_ptx.cuh"
@@ -319,7 +320,6 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
   } else {
     // ------------------------------------------------------------------------------------------ dQ read-out
     const int quad = warp & 3;
-    const int r = quad * 32 + (tid & 31);
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     bool ok = true;
     uint32_t n_done = 0;
@@ -331,26 +331,19 @@ bwd_stream_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_consta
       const uint32_t acc = n_done % C::kAccs;
       if (!(ok = wait_warp(dq_full + acc, (n_done / C::kAccs) & 1, abort_flag))) break;
       tc_fence_after();
-      const int64_t token = itm.tile * 128 + r;
-      __nv_bfloat16* dst = p.dq + b * p.dq_sb + token * p.dq_sn + h * p.dq_sh;
-      if (Kinds != kOnlyDq && itm.kind == kDk) dst = p.dk + b * p.dk_sb + token * p.dk_sn + h * p.dk_sh;
-      if (Kinds != kOnlyDq && itm.kind == kDv) dst = p.dv + b * p.dv_sb + token * p.dv_sn + h * p.dv_sh;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t rr[32];
-        tmem_ld32(tmem + lane_base + C::kColDq + D * acc + 32 * c, rr);
-        tmem_wait_ld();
-        uint32_t w[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(rr[2 * e]) * mul,
-                                                   __uint_as_float(rr[2 * e + 1]) * mul);
-          w[e] = *reinterpret_cast<uint32_t*>(&v);
-        }
-        uint4* d4 = reinterpret_cast<uint4*>(dst + 32 * c);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) d4[e] = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+      __nv_bfloat16* dst = p.dq + b * p.dq_sb + h * p.dq_sh;
+      int64_t sn = p.dq_sn;
+      if (Kinds != kOnlyDq && itm.kind == kDk) {
+        dst = p.dk + b * p.dk_sb + h * p.dk_sh;
+        sn = p.dk_sn;
       }
+      if (Kinds != kOnlyDq && itm.kind == kDv) {
+        dst = p.dv + b * p.dv_sb + h * p.dv_sh;
+        sn = p.dv_sn;
+      }
+      dst += (static_cast<int64_t>(itm.tile) * 128 + quad * 32) * sn;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) store_rows32(tmem + lane_base + C::kColDq + D * acc + 32 * c, mul, dst + 32 * c, sn);
       tc_fence_before();
       __syncwarp();
       if ((tid & 31) == 0) mbar_arrive(dq_free + acc);

@@ -134,39 +134,12 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     auto write_out = [&](int k, int kt, int bhk) -> bool {
       if (!wait_warp(bar_acc, k & 1, abort_flag)) return false;
       tc_fence_after();
-      // A thread that held a row would write 16 bytes into each of 32 lines per instruction (3.3 us an item).  Four threads share a
-      // row instead: loaded as MMA fragments, a 4 x 4 exchange gives each of them 16 contiguous bytes of the row's 64.
-      const int lane = tid & 31, i = lane & 3;
-      const int64_t b = bhk / p.Hk, hk = bhk - b * p.Hk, key = kt * 128 + 32 * quad + (lane >> 2);
+      const int64_t b = bhk / p.Hk, hk = bhk - b * p.Hk, key = kt * 128 + 32 * quad;
 #pragma unroll 1
-      for (int x = 0; x < 4; ++x) {                      // dV, dK of lanes 0 - 15, then of lanes 16 - 31
-        uint32_t rr[16];
-        tmem_ld_frag32(tmem + lane_base + (static_cast<uint32_t>(x >> 1) << 20) + ((x & 1) ? C::kColDk : C::kColDv) + 32 * qb, rr);
-        tmem_wait_ld();
-        __nv_bfloat16* dst = (x & 1) ? p.dk + b * p.dk_sb + hk * p.dk_sh : p.dv + b * p.dv_sb + hk * p.dv_sh;
-        const int64_t sn = (x & 1) ? p.dk_sn : p.dv_sn;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {                    // rows lane / 4 and lane / 4 + 8
-          uint32_t w[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(rr[4 * j + 2 * h]), __uint_as_float(rr[4 * j + 2 * h + 1]));
-            w[j] = *reinterpret_cast<uint32_t*>(&v);     // columns 8 j + 2 i and the next
-          }
-          // 4 x 4 transposition in the group of four lanes: word j of lane i <-> word i of lane j
-#pragma unroll
-          for (int bit = 1; bit < 4; bit *= 2) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (j & bit) continue;
-              const bool up = (i & bit) != 0;
-              const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[j] : w[j | bit], bit);
-              if (up) w[j] = got; else w[j | bit] = got;
-            }
-          }
-          const int64_t row = key + 16 * (x >> 1) + 8 * h;
-          *reinterpret_cast<uint4*>(dst + row * sn + 32 * qb + 8 * i) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
+      for (int x = 0; x < 2; ++x) {
+        const int64_t sn = x ? p.dk_sn : p.dv_sn;
+        store_rows32(tmem + lane_base + (x ? C::kColDk : C::kColDv) + 32 * qb, 1.0f,
+                     (x ? p.dk + b * p.dk_sb + hk * p.dk_sh : p.dv + b * p.dv_sb + hk * p.dv_sh) + key * sn + 32 * qb, sn);
       }
       return true;
     };
