@@ -68,9 +68,14 @@ int make_code_map(CUtensorMap* m, const void* base, uint64_t rows, int D) {
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(D)};
   const cuuint32_t box[2] = {128, 128};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&]() {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  int dev = 0;
+  // A thread whose first CUDA call this is (autograd's) has no context yet; the runtime makes one current when the device is set.
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
   if (r != CUDA_SUCCESS) return fail(DM_ERR_CUDA, "delta_matching: cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return 0;
 }
@@ -360,8 +365,7 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t hd = static_cast<int64_t>(H) * D, kd = static_cast<int64_t>(Hk) * D;
   const dm::QuantParams pd = make_quant(d_o, do_sb, do_sh, do_sn, nullptr, 1.0f, o, N * hd, D, hd, B, N, H, D, do8, dos, delta);
-  cudaError_t e = dm::launch_quant(pd, st);
-  if (e != cudaSuccess) return cuda_fail(e, "quantiser launch");
+  cudaError_t e;
   CUtensorMap tq, tk, tv, td, tds;
   DM_TRY(make_code_map(&tq, q8, static_cast<uint64_t>(B) * H * N, D));
   DM_TRY(make_code_map(&tk, k8, static_cast<uint64_t>(B) * Hk * N, D));
@@ -369,8 +373,11 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
   DM_TRY(make_code_map(&td, do8, static_cast<uint64_t>(B) * H * N, D));
   if (o == nullptr) {
     const dm::DeltaParams p{qs, ks, vs, dos, lse, delta, B, H, Hk, N, causal ? 1 : 0, status, (flags & DM_ATTN_DELTA_SUM) ? 0 : 1};
-    e = dm::launch_delta(D, tq, tk, tv, td, p, st);
-    if (e != cudaSuccess) return cuda_fail(e, "matched-delta launch");
+    e = dm::launch_quant_do_delta(D, tq, tk, tv, td, p, pd, st);
+    if (e != cudaSuccess) return cuda_fail(e, "dO quantiser or matched-delta launch");
+  } else {
+    e = dm::launch_quant(pd, st);
+    if (e != cudaSuccess) return cuda_fail(e, "quantiser launch");
   }
   if (!kernels) return 0;
   dm::BwdParams p{};

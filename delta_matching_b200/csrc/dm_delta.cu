@@ -17,6 +17,7 @@
 // once, at the end, in shared memory.
 #include "dm_common.cuh"
 #include "dm_kernels.h"
+#include "dm_quant_block.cuh"
 
 namespace dm {
 
@@ -47,10 +48,14 @@ __device__ __forceinline__ void delta_item(int item, int n_qt, int bh_count, int
   bh = item % bh_count;
 }
 
-template <int D>
+// kQuant: the CTA has one item and quantises its dO tile itself (codes and scales also go to where the kernels behind expect them),
+// which takes the place of a launch of the dO producer: with at most as many items as SMs, where a step is bound by its launches.  The
+// codes come back by TMA, while the first key tiles land.  Training step in us: 69.3 -> 67.5 (N=256 H=2), 87.6 -> 85.3 (N=1024 H=8), 88.8 -> 87.9
+// (B=2 N=1024 H=16: 256 items, two launches as before, within the spread), 91.4 -> 91.1 (head_dim 256, N=1920 H=6).
+template <int D, bool kQuant>
 __global__ void __launch_bounds__(DeltaCfg<D>::kThreads, 1)
 delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const DeltaParams p) {
+             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const DeltaParams p, const QuantParams pq) {
   using C = DeltaCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -70,6 +75,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 7 + 2 * C::kStages);
   uint64_t* bar_pub = bars + 20;   // [3] parts 1-3 have published their partial sums of the item (rotating slots)
   uint64_t* bar_read = bars + 23;  // [3] part 0 has read the slot
+  uint64_t* bar_do = bars + 26;    // kQuant: the dO codes are in global memory (one arrival per compute warp)
   static_assert(7 + 2 * C::kStages < 20, "barrier block layout");
 
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -92,6 +98,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       mbar_init(bar_pub + s, (C::kGroups - 1) * 4);
       mbar_init(bar_read + s, 4);
     }
+    mbar_init(bar_do, C::kGroups * 4);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -121,11 +128,13 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         const int n_it = p.causal ? (qt + 1) : n_qt;
         if (n_done > 0 && !(ok = wait_or_abort(bar_qfree, (n_done - 1) & 1, abort_flag))) break;
         mbar_expect_tx(bar_q, 2 * C::kTileBytes);
-        for (int s = 0; s < C::kSub; ++s) {
-          tma_load_2d(sQ + s * 16384, &tm_q, bar_q, s * 128, bh * p.N + qt * 128);
-          tma_load_2d(sDo + s * 16384, &tm_do, bar_q, s * 128, bh * p.N + qt * 128);
-        }
+        for (int s = 0; s < C::kSub; ++s) tma_load_2d(sQ + s * 16384, &tm_q, bar_q, s * 128, bh * p.N + qt * 128);
         for (int it = 0; it < n_it; ++it, ++g) {
+          // dO: at once, or behind the first key tiles, when the compute warps have made it
+          if (it == (kQuant ? min(n_it, C::kStages) - 1 : 0)) {
+            if (kQuant && !(ok = wait_or_abort(bar_do, 0, abort_flag))) break;
+            for (int s = 0; s < C::kSub; ++s) tma_load_2d(sDo + s * 16384, &tm_do, bar_q, s * 128, bh * p.N + qt * 128);
+          }
           const uint32_t st = g % C::kStages;
           if (g >= C::kStages && !(ok = wait_or_abort(empty + st, ((g / C::kStages) - 1) & 1, abort_flag))) break;
           const int row = bhk * p.N + it * 128;          // key tiles in ascending order
@@ -192,6 +201,16 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     const int nblk = p.N / 32;
     uint32_t g = 0, n_done = 0;
     bool ok = true;
+    if (kQuant) {
+      // a warpgroup per 32-token block; sRed is not in use yet
+      int qt, bh;
+      delta_item(blockIdx.x, n_qt, bh_count, qt, bh);
+      quant_block<D, false, false>(pq, qt * 4 + (tid >> 7), bh, reinterpret_cast<float*>(sRed) + 4 * (tid >> 7), r, 1 + (tid >> 7));
+      fence_async_global();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(bar_do);
+      bar_sync(5, C::kGroups * 128);                     // the scales are there for all; sRed is free
+    }
     for (int k = 0, item; (item = sched_item(k, blockIdx.x, gridDim.x)) < n_items; ++k, ++n_done) {
       int qt, bh;
       delta_item(item, n_qt, bh_count, qt, bh);
@@ -295,27 +314,36 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   if (warp == 17) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-template <int D>
+template <int D, bool kQuant>
 static cudaError_t launch_delta_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                                  const CUtensorMap& tdo, const DeltaParams& p, cudaStream_t stream) {
+                                  const CUtensorMap& tdo, const DeltaParams& p, const QuantParams& pq, cudaStream_t stream) {
   using C = DeltaCfg<D>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(delta_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(delta_kernel<D, kQuant>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   const int n_items = (p.N / 128) * p.B * p.H;
   const int ctas = sm_count();
   count_launch();
-  return launch_chained(delta_kernel<D>, n_items < ctas ? n_items : ctas, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, p);
+  return launch_chained(delta_kernel<D, kQuant>, n_items < ctas ? n_items : ctas, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, p, pq);
 }
 
 cudaError_t launch_delta(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& tdo, const DeltaParams& p, cudaStream_t stream) {
-  return D == 128 ? launch_delta_t<128>(tq, tk, tv, tdo, p, stream) : launch_delta_t<256>(tq, tk, tv, tdo, p, stream);
+  return (D == 128 ? launch_delta_t<128, false> : launch_delta_t<256, false>)(tq, tk, tv, tdo, p, QuantParams{}, stream);
+}
+
+cudaError_t launch_quant_do_delta(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                  const DeltaParams& p, const QuantParams& pq, cudaStream_t stream) {
+  if ((p.N / 128) * static_cast<long long>(p.B) * p.H > sm_count()) {
+    const cudaError_t e = launch_quant(pq, stream);
+    return e != cudaSuccess ? e : launch_delta(D, tq, tk, tv, tdo, p, stream);
+  }
+  return (D == 128 ? launch_delta_t<128, true> : launch_delta_t<256, true>)(tq, tk, tv, tdo, p, pq, stream);
 }
 
 }  // namespace dm

@@ -110,6 +110,9 @@ cudaError_t launch_fwd(int D, const CUtensorMap& tq, const CUtensorMap& tk, cons
                        cudaStream_t stream);
 cudaError_t launch_delta(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& tdo, const DeltaParams& p, cudaStream_t stream);
+// The dO producer and pass 0, in one launch where each CTA of pass 0 has one item.
+cudaError_t launch_quant_do_delta(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                  const DeltaParams& p, const QuantParams& pq, cudaStream_t stream);
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const CUtensorMap& tdo, const CUtensorMap* tds_or_null, const BwdParams& p,
                             cudaStream_t stream);

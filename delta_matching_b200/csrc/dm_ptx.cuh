@@ -109,6 +109,8 @@ __device__ __forceinline__ void sts_u4(void* p, uint32_t a, uint32_t b, uint32_t
 }
 // ------------------------------------------------------------------------------------------------ fences
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Global memory written by this thread, for the async proxy (a TMA load that a signal from this thread releases).
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
