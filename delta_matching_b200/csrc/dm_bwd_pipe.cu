@@ -19,7 +19,8 @@
 //     while the last tile of the one before is worked on, and that one is written out behind the first exponentials of the next.
 //     With a CTA per item its start and end cost 8 us: 777 -> 742 us, and 474 -> 394 (B=8 N=2048 H=16 bidirectional, 16 tiles an item).
 //   - one copy of each role's loop (48 KB of code in all): at 88 KB the warps waited for instructions a fifth of the time (920 us).
-// Before (eight compute warps on one phase, one issuing warp, a CTA per item): 836, 490 and 230 us (B=1) -> 742, 394, 209.
+// Before (eight compute warps on one phase, one issuing warp, a CTA per item): 836, 490 and 230 us (B=1) -> 742, 394, 209; barriers by their
+// shared addresses and a shorter scale byte: 762 -> 756 on another GPU of the same model.
 #include <cuda_bf16.h>
 #include "dm_bwd_math.cuh"
 #include "dm_common.cuh"
@@ -122,6 +123,9 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t xch_a = smem_u32(smem + C::kSmemXch) + 16 * quad;
     const uint32_t ws_a = smem_u32(smem + C::kSmemWs) + r * 128;
     const uint32_t ws_c0 = ws_a + (((2 * qb) ^ (r & 7)) << 4);      // its neighbour is 16 bytes up or down
+    // barriers by their shared addresses
+    const uint32_t s_bar = smem_u32(bar_s), dp_bar = smem_u32(bar_dp), k_bar = smem_u32(bar_k), p_bar = smem_u32(bar_p);
+    const uint32_t vec_bar = smem_u32(vec_ok), x_bar = smem_u32(bar_x) + 8 * quad;
     const bool leader = (tid & 31) == 0;
     bool ok = true;
     float ks_row = 0.f, vs_row = 0.f;                    // scales of the item's key row
@@ -170,16 +174,16 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       --left;
       --n;
       const uint32_t va = vec_a + (g % C::kStages) * C::kVecBytes;
-      uint64_t* bx = bar_x + 4 * ((g - 1) & 1) + quad;
+      const uint32_t bx = x_bar + 32 * ((g - 1) & 1);
       // S^T, the vectors, and the maxima of the tile before, in one look
       {
         const bool need_x = !DS32 && g > 0;
-        bool seen = mbar_test_wait(bar_s, g & 1);
-        if (more) seen = mbar_test_wait(vec_ok + g % C::kStages, (g / C::kStages) & 1) && seen;
+        bool seen = mbar_test_wait(s_bar, g & 1);
+        if (more) seen = mbar_test_wait(vec_bar + 8 * (g % C::kStages), (g / C::kStages) & 1) && seen;
         if (need_x) seen = mbar_test_wait(bx, ((g - 1) >> 1) & 1) && seen;
         if (!__all_sync(0xffffffffu, seen)) {
-          seen = poll_or_abort(bar_s, g & 1, abort_flag);
-          if (more) seen = seen && poll_or_abort(vec_ok + g % C::kStages, (g / C::kStages) & 1, abort_flag);
+          seen = poll_or_abort(s_bar, g & 1, abort_flag);
+          if (more) seen = seen && poll_or_abort(vec_bar + 8 * (g % C::kStages), (g / C::kStages) & 1, abort_flag);
           if (need_x) seen = seen && poll_or_abort(bx, ((g - 1) >> 1) & 1, abort_flag);
           if (!(ok = __all_sync(0xffffffffu, seen))) break;
         }
@@ -207,7 +211,7 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (leader) mbar_arrive(bar_k);
+        if (leader) mbar_arrive(k_bar);
       }
       if (!more) break;
       const float4 rec = lds_f4(va + C::kVecRec + 16 * qb);
@@ -220,7 +224,7 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const float pm = p_block(rs, splat2(ks_row * rec.x), va + C::kVecLse + 128 * qb, pr);
       if (first && g > 0 && !(ok = write_out(k - 2, kt_done, bhk_done))) break;
       // P^T codes: one scale per (key row, 32 queries)
-      if (!(ok = wait_warp(bar_dp, g & 1, abort_flag))) break;
+      if (!(ok = wait_warp(dp_bar, g & 1, abort_flag))) break;
       tc_fence_after();
       uint32_t rd[32];
       tmem_ld32(t_dp, rd);
@@ -234,11 +238,11 @@ bwd_dkdv_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (leader) mbar_arrive(bar_p);
+      if (leader) mbar_arrive(p_bar);
       am = warp_max(neg_ds_block(rd, splat2(vs_row * rec.y), va + C::kVecDelta + 128 * qb, pr));
       if (leader) {
         sts_f(xch_a + 64 * (g & 1) + 4 * qb, am);
-        mbar_arrive(bar_x + 4 * (g & 1) + quad);
+        mbar_arrive(x_bar + 32 * (g & 1));
       }
     }
     if (ok) ok = write_out(k - 2, kt_done, bhk_done);

@@ -30,10 +30,9 @@ constexpr float kLn2 = 0.6931471805599453f;
 // inv_pow2_from_sb) and the producers' rule in delta_matching/sm100/quant.py:160-176.
 // Byte of the smallest power of two s with amax <= 448 * s; `zero_byte` is returned for amax == 0.
 __device__ __forceinline__ uint32_t pow2_sb(float amax, uint32_t zero_byte) {
-  uint32_t bits = __float_as_uint(amax);
-  int eb = static_cast<int>((bits >> 23) & 0xFF) - 8 + ((bits & 0x7FFFFF) > 0x600000 ? 1 : 0);
-  eb = max(1, min(eb, 254));
-  return amax > 0.f ? static_cast<uint32_t>(eb) : zero_byte;
+  // exponent field - 8, one more where the mantissa field exceeds 0x600000 (the addition carries into the exponent then); at most 248
+  const int eb = static_cast<int>((__float_as_uint(amax) + 0x1FFFFFu) >> 23) - 8;
+  return amax > 0.f ? static_cast<uint32_t>(max(1, eb)) : zero_byte;
 }
 __device__ __forceinline__ float sb_to_scale(uint32_t b) { return __uint_as_float(b << 23); }          // 2^(b-127), b>=1
 __device__ __forceinline__ float sb_to_inv(uint32_t b) { return __uint_as_float((254u - b) << 23); }   // 2^(127-b)
@@ -90,7 +89,8 @@ constexpr uint32_t kWaitLimitNs = 2000000000u;
 // The phase is not complete yet (or has not been looked at).  A waiting warp must not eat the issue slots of the warps it waits for:
 // after a few immediate retries it sleeps between polls, and it looks at the abort flag and the clock only every 64 polls (every
 // poll under a short limit).
-__device__ __forceinline__ bool poll_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
+template <typename Bar>
+__device__ __forceinline__ bool poll_or_abort(Bar bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
   const uint32_t t0 = global_ns_lo(), check_mask = limit_ns < 100000000u ? 0u : 63u;
 #pragma unroll 1
   for (uint32_t i = 0;; ++i) {
@@ -99,13 +99,15 @@ __device__ __forceinline__ bool poll_or_abort(uint64_t* bar, uint32_t parity, vo
     if ((i & check_mask) == check_mask && (*abort_flag != 0 || global_ns_lo() - t0 > limit_ns)) return false;
   }
 }
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
+template <typename Bar>
+__device__ __forceinline__ bool wait_or_abort(Bar bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
   if (mbar_test_wait(bar, parity)) return true;      // the common case in a pipeline that runs ahead: already complete
   return poll_or_abort(bar, parity, abort_flag, limit_ns);
 }
 // Whole-warp form for the compute warps: every lane polls, the verdict is made uniform so that the warp-wide tcgen05.ld /
 // tcgen05.st that follow are never executed by a part of the warp.
-__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+template <typename Bar>
+__device__ __forceinline__ bool wait_warp(Bar bar, uint32_t parity, volatile int* abort_flag) {
   if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity) ? 1 : 0) != 0) return true;   // ~80 cycles when complete
   return __all_sync(0xffffffffu, poll_or_abort(bar, parity, abort_flag) ? 1 : 0) != 0;
 }
