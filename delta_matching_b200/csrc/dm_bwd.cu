@@ -1,5 +1,6 @@
 // dQ of the backward without a workspace, on sm_100a: all matmuls on tcgen05 with TMEM accumulators, bit-deterministic (one
-// writer per output element, fixed loop orders, no atomics).  dK and dV: dm_bwd_kv.cu; dQ from stored dS tiles: dm_bwd_p2.cu.
+// writer per output element, fixed loop orders, no atomics).  dK and dV: dm_bwd_pipe.cu and
+// dm_bwd_kv.cu; dQ from stored dS tiles: dm_bwd_p2.cu.
 //
 //   Query-stationary: CTA = (128-query tile, query head, batch); loops over key tiles: S, dP recomputed, dS codes staged in
 //   shared memory, dQ += dS K block-scaled; dQ * softmax_scale rounded to bf16 once.  Also the form of the identity probe.

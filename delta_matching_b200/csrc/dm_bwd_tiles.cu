@@ -1,8 +1,8 @@
 // Backward of small problems, tile-parallel: every live 128 x 128 (key x query) tile on its own, its P^T and dS^T codes and
 // scale words left in a workspace, from which one streaming launch (dm_bwd_p2.cu) makes dV, dK and dQ.
 //
-// The key-stationary kernel (dm_bwd_kv.cu) walks all tiles of a key tile, the whole GQA group's, in one CTA: a chain of
-// (H / Hk) (N / 128) tiles at about 1.7 us each, however many SMs are idle.  At B=1 N=1024 H=8 Hk=2 that is 16 chains of up to
+// The key-stationary kernels (dm_bwd_pipe.cu, dm_bwd_kv.cu) walk all tiles of a key tile, the whole GQA group's, in one CTA: a chain of
+// (H / Hk) (N / 128) tiles at about 1.6 us each, however many SMs are idle.  At B=1 N=1024 H=8 Hk=2 that is 16 chains of up to
 // 32 tiles on 148 SMs.  Here the tiles are dealt out evenly, and what stays a chain is the accumulation alone, at about a
 // fifth of the time per tile.  The arithmetic, the order of every sum and so the bits are those of the key-stationary kernel.
 #include <cuda_bf16.h>
