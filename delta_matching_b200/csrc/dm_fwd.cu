@@ -11,7 +11,7 @@
 //   O = bf16(O_acc / l);  LSE = (m + log2 l) * ln2.  Key tiles are visited from the highest index down.
 //
 // Work item = one 128-query tile of one (batch, query head); a CTA walks a list of items.  Warps 0-3: softmax / epilogue
-// (thread t owns TMEM lane t = query row t).  Warp 4: TMA producer.  Warp 5: MMA issuer and TMEM owner.  Every mbarrier wait is bounded.
+// (thread t owns TMEM lane t = query row t; at head_dim 256 warps 6-9 share the rows).  Warp 4: TMA producer.  Warp 5: MMA issuer and TMEM owner.  Every mbarrier wait is bounded.
 #include <type_traits>
 #include <cuda_bf16.h>
 #include "dm_common.cuh"
@@ -29,7 +29,14 @@ struct FwdCfg {
   // S chain of key tile i + 1 runs while the softmax warps work on tile i.  At head_dim 128 two CTAs share the SM with 256
   // columns each (S 0-127, O 128-255) and take turns instead.
   static constexpr bool kDoubleS = (D == 256);
-  static constexpr int kColS = 0;                      // S accumulator, 128 fp32 columns; P codes reuse columns 0-31
+  // ... and two warps share a row (warps 6-9 take the upper 64 keys of the rows of warps 0-3): with one warp per scheduler nothing runs
+  // under the latencies of its chain.  590 -> 579 us (B=2 N=8192 H=16); what bounds it then is the MMA warp's turn per tile.
+  static constexpr int kRowWarps = (D == 256) ? 2 : 1;
+  static constexpr int kChunks = 4 / kRowWarps;        // 32-key chunks per thread and tile
+  static constexpr int kThreads = 192 + 128 * (kRowWarps - 1);
+  static constexpr int kColS = 0;                      // S accumulator, 128 fp32 columns
+  // P codes of 32 keys, 8 columns: over columns that the writing warp itself has loaded (0-31; with two warps per row 0-15 and 64-79)
+  __host__ __device__ static constexpr int code_col(int ks) { return (kRowWarps == 2 && ks >= 2) ? 64 + 8 * (ks - 2) : 8 * ks; }
   static constexpr int kColSfa = 32;                   // 4 columns, each this row's SFA word
   static constexpr int kColSfb = 36;                   // 4 columns, each the tile's V scale word
   static constexpr int kColO = kDoubleS ? 256 : 128;   // O accumulator, D fp32 columns
@@ -39,7 +46,10 @@ struct FwdCfg {
   static constexpr int kSmemV = kSmemK + kStages * kTileBytes;
   static constexpr int kSmemOut = kSmemV + kStages * kTileBytes;   // 4 warps x 32 rows x 80 bytes: O write-out staging
   static constexpr int kOutRow = 80;                               // 64 bytes of a row + 16 of padding (bank spread)
-  static constexpr int kSmemBar = kSmemOut + 4 * 32 * kOutRow;
+  // two warps per row: block exponents and sums (16 bytes) and the maximum of the upper 64 keys per row, by tile parity
+  static constexpr int kSmemXch = kSmemOut + 4 * 32 * kOutRow;
+  static constexpr int kXchBytes = 128 * 20;
+  static constexpr int kSmemBar = kSmemXch + (kRowWarps - 1) * 2 * kXchBytes;
   static constexpr int kSmemBytes = kSmemBar + 256 + 1024;   // + slack for the 1024-byte alignment of the tile base
 };
 
@@ -53,7 +63,7 @@ struct FwdCfg {
 // reference met the same question and answers it with a commit and a wait, delta_matching/sm100/dm_fwd_sm100.py:636-645).
 // kOrdered = false issues S(i + 1) straight behind PV(i) and relies on issue order alone.
 template <int D, bool kOrdered>
-__global__ void __launch_bounds__(192, (D == 128) ? 2 : 1)
+__global__ void __launch_bounds__(FwdCfg<D>::kThreads, (D == 128) ? 2 : 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
   using C = FwdCfg<D>;
@@ -75,6 +85,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   uint64_t* empty_k = bars + 8;   // [kStages] K stage free again (MMA commit behind the S chain)
   uint64_t* empty_v = bars + 14;  // [kStages] V stage free again (MMA commit behind the PV chain)
   uint64_t* bar_qfree = bars + 10; // the item's last S chain has read Q (MMA commit)
+  uint64_t* bar_x = bars + 18;    // [2][4] two warps per row: tile parity, row quarter: what the lower warp needs is written
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 13);
 
@@ -90,9 +101,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     mbar_init(bar_q, 1);
     mbar_init(bar_s, 1);
     mbar_init(bar_s1, 1);
-    mbar_init(bar_p1, 4);
+    mbar_init(bar_p1, 4 * C::kRowWarps);
     mbar_init(bar_o1, 1);
-    mbar_init(bar_p, 4);
+    mbar_init(bar_p, 4 * C::kRowWarps);
+    if (C::kRowWarps == 2)
+      for (int i = 0; i < 8; ++i) mbar_init(bar_x + i, 1);
     mbar_init(bar_o, 1);
     mbar_init(bar_qfree, 1);
     for (int s = 0; s < C::kStages; ++s) {
@@ -209,7 +222,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
             for (int s = 0; s < C::kSub; ++s) {
-              mma_mxf8_ts(tmem + C::kColO + s * 128, tmem + C::kColS + 128 * buf + ks * 8, v_lo + s * 1024 + ks * 256,
+              mma_mxf8_ts(tmem + C::kColO + s * 128, tmem + C::kColS + 128 * buf + C::code_col(ks), v_lo + s * 1024 + ks * 256,
                           idesc_mxf8(128, 128, false, true, ks, ks), tmem + C::kColSfa + 128 * buf,
                           tmem + C::kColSfb + 128 * buf, (it > 0) || (ks > 0));
             }
@@ -222,14 +235,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
   } else {
     // ------------------------------------------------------------------------------------------ softmax / epilogue
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    const int half = (C::kRowWarps == 2 && warp > 5) ? 1 : 0;               // upper 64 keys of a tile
+    const int quad = (C::kRowWarps == 2) ? (warp & 3) : warp;
+    const int trow = (C::kRowWarps == 2) ? (quad * 32 + (tid & 31)) : tid;  // row of the tile = TMEM lane
+    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t xch_a = smem_u32(smem + C::kSmemXch);
     const int nblk = p.N / 32;
     bool ok = true;
     int gt = 0;
     // scalars of an item: head, query row, first key tile; the scales of item + 1 are requested one item ahead
     auto item_qs = [&](int item) -> const float* {
       const int qt = n_qt - 1 - item / BH, bh = item % BH;
-      return p.qs + static_cast<size_t>(bh) * nblk + (qt * 128 + tid) / 32;
+      return p.qs + static_cast<size_t>(bh) * nblk + (qt * 128 + trow) / 32;
     };
     auto item_kv = [&](int item, const float* base) -> const float* {
       const int qt = n_qt - 1 - item / BH, bh = item % BH;
@@ -247,7 +264,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const int qt = n_qt - 1 - item / BH, bh = item % BH;
       const int b = bh / p.H, h = bh % p.H;
       const int n_it = p.causal ? (qt + 1) : n_qt;
-      const int row = qt * 128 + tid;                                       // query index inside the head
+      const int row = qt * 128 + trow;                                       // query index inside the head
       const float qsl = qs_next * kLog2e;
       const int item_n = sched_item(k + 1, first_item, item_step);
       const bool has_next = item_n < n_items;
@@ -259,7 +276,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       // above the query index are masked; a compile-time variant so that the other tiles carry no select per element.
       auto tile = [&](int it, auto diag_tag) -> bool {
         constexpr bool kDiag = decltype(diag_tag)::value;
-        const float cb[4] = {qsl * ks4.x, qsl * ks4.y, qsl * ks4.z, qsl * ks4.w};
+        float cb[4] = {qsl * ks4.x, qsl * ks4.y, qsl * ks4.z, qsl * ks4.w};  // of this warp's chunks
+        if (half) {
+          cb[0] = cb[2];
+          cb[1] = cb[3];
+        }
         const uint32_t sfb = pack4(scale_to_sb(vs4.x), scale_to_sb(vs4.y), scale_to_sb(vs4.z), scale_to_sb(vs4.w));
         // scales of the next key tile (of this item or of the next one): in flight while this tile is processed
         if (it + 1 < n_it) {
@@ -277,16 +298,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         tc_fence_after();
         float bsum[4], kb[4], bmax[4];
         uint32_t r[2][32];
-        tmem_ld32(tmem + lane_base + s_col, r[0]);
+        const uint32_t t_s = tmem + lane_base + s_col + 64 * half;
+        tmem_ld32(t_s, r[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < C::kChunks; ++c) {
           uint32_t (&rc)[32] = r[c & 1];
           tmem_wait_ld();
-          if (c < 3) tmem_ld32(tmem + lane_base + s_col + 32 * (c + 1), r[(c + 1) & 1]);   // next chunk in flight
+          if (c < C::kChunks - 1) tmem_ld32(t_s + 32 * (c + 1), r[(c + 1) & 1]);   // next chunk in flight
           if (kDiag) {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (32 * c + e > tid) rc[e] = 0xff800000u;       // -inf: key index above the query index
+              if (32 * c + e > trow - 64 * half) rc[e] = 0xff800000u;       // -inf: key index above the query index
           }
           float2 s2[16];
 #pragma unroll
@@ -307,7 +329,32 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           }
           sum0 = add2(sum0, sum1);
           bsum[c] = sum0.x + sum0.y;
-          tmem_st8(tmem + lane_base + s_col + 8 * c, codes);
+          tmem_st8(t_s + 8 * c, codes);
+        }
+        if constexpr (C::kRowWarps == 2) {
+          // The upper warp hands the lower one what the running maximum, the sum and the scale words need.  Its slot is free again: this
+          // tile's S was issued behind the PV chain of tile gt - 2, so behind the lower warp's arrival for that tile.
+          const uint32_t xa = xch_a + sbuf * C::kXchBytes + 16 * trow, xm = xch_a + sbuf * C::kXchBytes + 2048 + 4 * trow;
+          if (half) {
+            sts_u4(xa, __float_as_uint(kb[0]), __float_as_uint(kb[1]), __float_as_uint(bsum[0]), __float_as_uint(bsum[1]));
+            sts_f(xm, fmaxf(bmax[0], bmax[1]));
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if ((tid & 31) == 0) {
+              mbar_arrive(bar_x + 4 * sbuf + quad);
+              mbar_arrive(p_bar(gt));
+            }
+            ++gt;
+            return true;
+          }
+          if (!wait_warp(bar_x + 4 * sbuf + quad, tile_ph(gt), abort_flag)) return false;
+          const float4 up = lds_f4(xa);
+          kb[2] = up.x;
+          kb[3] = up.y;
+          bsum[2] = up.z;
+          bsum[3] = up.w;
+          bmax[2] = bmax[3] = lds_f(xm);
         }
         const float mcand = ceilf(fmaxf(fmaxf(bmax[0], bmax[1]), fmaxf(bmax[2], bmax[3])));
         float acc_scale = 1.0f;
@@ -353,6 +400,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       };
       ok = p.causal ? tile(0, std::true_type{}) : tile(0, std::false_type{});
       for (int it = 1; ok && it < n_it; ++it) ok = tile(it, std::false_type{});
+      if (ok && half) continue;                            // O is written out by the lower warps
       if (ok) ok = wait_warp(o_bar(gt - 1), tile_ph(gt - 1), abort_flag);
       if (!ok) break;
       tc_fence_after();
@@ -411,7 +459,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
   const int items = (p.N / 128) * p.B * p.H;
   const int ctas = sms * ((D == 128) ? 2 : 1);              // co-resident CTAs: 256 of the 512 TMEM columns each at D = 128
   count_launch();
-  return launch_chained(fwd_kernel<D, kOrdered>, items < ctas ? items : ctas, 192, C::kSmemBytes, stream, tq, tk, tv, p);
+  return launch_chained(fwd_kernel<D, kOrdered>, items < ctas ? items : ctas, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, p);
 }
 
 
