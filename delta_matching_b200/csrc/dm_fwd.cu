@@ -11,7 +11,8 @@
 //   O = bf16(O_acc / l);  LSE = (m + log2 l) * ln2.  Key tiles are visited from the highest index down.
 //
 // Work item = one 128-query tile of one (batch, query head); a CTA walks a list of items.  Warps 0-3: softmax / epilogue
-// (thread t owns TMEM lane t = query row t; at head_dim 256 warps 6-9 share the rows).  Warp 4: TMA producer.  Warp 5: MMA issuer and TMEM owner.  Every mbarrier wait is bounded.
+// (thread t owns TMEM lane t = query row t; at head_dim 256 warps 6-9 share the rows).  Warp 4: TMA producer.  Warp 5: MMA
+// issuer and TMEM owner.  Every mbarrier wait is bounded.
 #include <type_traits>
 #include <cuda_bf16.h>
 #include "dm_common.cuh"
@@ -30,7 +31,8 @@ struct FwdCfg {
   // columns each (S 0-127, O 128-255) and take turns instead.
   static constexpr bool kDoubleS = (D == 256);
   // ... and two warps share a row (warps 6-9 take the upper 64 keys of the rows of warps 0-3): with one warp per scheduler nothing runs
-  // under the latencies of its chain.  590 -> 579 us (B=2 N=8192 H=16); what bounds it then is the MMA warp's turn per tile.
+  // under the latencies of its chain.  590 -> 579 us (B=2 N=8192 H=16); what bounds it then is the chain S -> PV -> its
+  // completion -> next S into the same buffer (PV as four MMAs of N = 256 instead of eight of 128: equal).
   static constexpr int kRowWarps = (D == 256) ? 2 : 1;
   static constexpr int kChunks = 4 / kRowWarps;        // 32-key chunks per thread and tile
   static constexpr int kThreads = 192 + 128 * (kRowWarps - 1);
