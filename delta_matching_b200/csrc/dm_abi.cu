@@ -295,18 +295,25 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
 
 // Which backward dm_attn_bwd runs (same results).  The key-stationary kernel takes as long as its longest chain, (H / Hk)
 // (N / 128) tiles in one CTA, or as its share of all tiles per SM, whichever is more, at about 1.6 us a tile; the tile-parallel
-// pair takes its share of all tiles at about 3.7 us.  Forward + backward in us, key-stationary -> tile-parallel by chain / tiles per SM:
-// 4.6 (N=8192 H=4 Hk=1) 593 -> 452; 3.0 (N=6144 H=8 Hk=2) 496 -> 435; 3.0 (N=4096 H=12 Hk=3) 346 -> 308; 2.7 (B=6 N=1024 H=8 Hk=2) 122.5 ->
-// 120; 2.29 (N=16384 H=2 Hk=1) 777 -> 758; 2.28 (N=8192 H=8 Hk=2) 689 -> 691; 2.24 (N=4096 H=16 Hk=4) 371 -> 376; 2.18 (N=2048 H=32 Hk=8) 213 ->
-// 218; 2.18 (B=2 N=2048 H=16 Hk=4) 212 -> 222; 2.06 (B=4 N=1024 H=16 Hk=4) 136.8 -> 138.8; 1.95 (N=2304 H=32 Hk=8) 245 -> 254; 1.8 (N=5120 H=16
-// Hk=4) 492 -> 516; 1.5 (B=2 N=3072 H=12 Hk=4) 269 -> 316.  Head_dim 256: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152
-// -> 143; 1.45 (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1 (N=4096 H=16 Hk=8) 467 -> 495.  The lines are drawn at 2.25, where the two meet, and at
-// 1.6, and at 2 GiB of workspace.  The workspace is the whole square of tiles, of which a causal call touches half: at its edge (N=8192
+// pair takes its share of all tiles at about 3.7 us.  Forward + backward in us, key-stationary -> tile-parallel by chain / tiles per SM,
+// causal: 4.6 (N=8192 H=4 Hk=1) 593 -> 452; 3.0 (N=6144 H=8 Hk=2) 496 -> 435; 3.0 (N=4096 H=12 Hk=3) 346 -> 308; 2.7 (B=6 N=1024 H=8 Hk=2)
+// 122.5 -> 120; 2.29 (N=16384 H=2 Hk=1) 777 -> 758; 2.28 (N=8192 H=8 Hk=2) 689 -> 691; 2.24 (N=4096 H=16 Hk=4) 371 -> 376; 2.18 (N=2048 H=32
+// Hk=8) 213 -> 218; 2.18 (B=2 N=2048 H=16 Hk=4) 212 -> 222; 2.06 (B=4 N=1024 H=16 Hk=4) 136.8 -> 138.8; 1.95 (N=2304 H=32 Hk=8) 245 -> 254;
+// 1.8 (N=5120 H=16 Hk=4) 492 -> 516; 1.5 (B=2 N=3072 H=12 Hk=4) 269 -> 316.
+// Bidirectional calls near the line have 66 to 74 key tiles, for which the key-stationary side is the kernel of two roles (dm_bwd_kv.cu)
+// and not the pipeline; the ratio is SMs / key tiles.  2.24 (N=2816 H=12 Hk=3) 227 -> 223, (B=11 N=768 H=4 Hk=1) 79.8 -> 75.9; 2.18 (N=4352 H=16
+// Hk=2) 632 -> 607, (B=17 N=512 H=4 Hk=1) 63.5 -> 61.6, (B=34 N=256 H=4 Hk=1) 43.2 -> 43.2; 2.11 (N=8960 H=4 Hk=1) 644 -> 628, (B=5 N=1792 H=4 Hk=1)
+// 152 -> 154, (N=8960 H=1) 251 -> 259, (B=35 N=256 H=4 Hk=1) 43.4 -> 44.9; 2.06 (N=2304 H=16 Hk=4) 187 -> 192.5, (N=3072 H=12 Hk=3) 240 -> 245,
+// (N=9216 H=1) 258 -> 269, (N=1536 H=12 Hk=6) 88.2 -> 86.2; 2.0 (N=9472 H=1) 269 -> 283.
+// Head_dim 256, causal: 2.2 (B=2 N=2048 H=8 Hk=4) 173 -> 151; 1.9 (B=3 N=1536 H=8 Hk=4) 152 -> 143; 1.45 (B=3 N=2048 H=8 Hk=4) 226 -> 228; 1.1
+// (N=4096 H=16 Hk=8) 467 -> 495.
+// The lines at head_dim 128 are drawn where the two meet, at 2.25 for causal calls and 2.15 for bidirectional ones, at head_dim 256 at 1.6,
+// and all at 2 GiB of workspace.  The workspace is the whole square of tiles, of which a causal call touches half: at its edge (N=8192
 // H=16 Hk=1, ratio 4.6, 2.03 GiB) it sends calls back to the key-stationary kernel that the tile-parallel one would win.
 static bool tile_parallel(int B, int N, int H, int Hk, int D, int causal) {
   const long long n_t = N / 128, tiles = static_cast<long long>(B) * H * (causal ? n_t * (n_t + 1) / 2 : n_t * n_t);
-  const long long chain = H / Hk * n_t;
-  return 20 * chain * dm::sm_count() >= (D == 128 ? 45 : 32) * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
+  const long long chain = H / Hk * n_t, line = D == 256 ? 32 : causal ? 45 : 43;      // twentieths
+  return 20 * chain * dm::sm_count() >= line * tiles && static_cast<long long>(B) * H * n_t * n_t * (2 * 16384 + 528) <= (2ll << 30);
 }
 
 // Workspace of `units` query heads with both tile sets: dS^T tiles, P^T tiles, dS words, P words.
