@@ -530,8 +530,12 @@ cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk,
                             cudaStream_t stream) {
   const CUtensorMap& tds = (tds_or_null != nullptr) ? *tds_or_null : tq;     // unused by the kernel without a workspace
   // At head_dim 128 the roles cost a second S^T and a second exponential per element, so they are for grids that leave half of
-  // the SMs without a CTA: each role's chain per tile is the shorter one then (the same bits: the accumulators do not
-  // depend on each other).
+  // the SMs without a CTA (the same bits: the accumulators do not depend on each other).  There the dK role is a little shorter than the
+  // pipeline, per tile (1.51 against 1.53 us; 32 x 32 dS blocks 1.31 against 1.40) and by some 2 us a launch, as dV is written out elsewhere.
+  // Pipeline -> roles, us of this pass alone: 20.6 -> 18.5 (N=1024 H=2), 32.9 -> 30.8 (N=512 H=8 Hk=2), 12.4 -> 10.3 (B=36 N=256 H=1), 70.0 ->
+  // 67.8 (N=1280 H=16 Hk=4), 400 -> 394 (N=4096 H=8 Hk=1), 463 -> 456 (N=9472 H=4 Hk=1); 32 x 32 blocks: 367 -> 342 and 425 -> 396 for the
+  // last two.  (Causal calls; bidirectional ones gain the same, with 32 x 32 blocks less: 371 -> 362, 429 -> 423.)  With more key tiles some SM
+  // has two roles in a row; whole step, bidirectional: 822 -> 928 (N=9728 H=4 Hk=1, 76 key tiles), 93 -> 108 (B=18 N=512 H=8 Hk=2, 144).
   if (D != 128) return (p.ds32 ? launch_kv_t<256, kKvRoles, true> : launch_kv_t<256, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);
   if (2ll * p.B * p.Hk * (p.N / 128) <= sm_count())
     return (p.ds32 ? launch_kv_t<128, kKvRoles, true> : launch_kv_t<128, kKvRoles, false>)(tq, tk, tv, tdo, tds, tq, p, stream);

@@ -116,7 +116,7 @@ cudaError_t launch_quant_do_delta(int D, const CUtensorMap& tq, const CUtensorMa
 cudaError_t launch_bwd_dkdv(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const CUtensorMap& tdo, const CUtensorMap* tds_or_null, const BwdParams& p,
                             cudaStream_t stream);
-// The form of launch_bwd_dkdv at head_dim 128 where the key tiles fill at least half of the SMs.
+// The form of launch_bwd_dkdv at head_dim 128 where there are more key tiles than half the SMs.
 cudaError_t launch_bwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                             const CUtensorMap& tds, const BwdParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_dq(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
