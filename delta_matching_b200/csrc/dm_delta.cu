@@ -10,11 +10,10 @@
 //
 // One persistent CTA per SM; a work item is one 128-query tile of one (batch, query head).  S = Q8 K8^T and dP = dO8 V8^T run on tcgen05
 // (kind::f8f6f4) into TMEM accumulators that are double-buffered (2 x (128 + 128) columns), so the tensor pipe works on
-// key tile i+1 while the compute warps take the exponentials of tile i.  Four compute groups of four warps (warps 0-15)
-// split the 128 key columns of a tile, 32 each, i.e. one K/V scale block per group (thread t of every group = TMEM lane
-// t % 128 = query row), which puts four compute warps on every scheduler: enough to keep the MUFU pipe fed while one
-// warp waits for TMEM or an mbarrier.  Warp 16 issues TMA loads, warp 17 the MMAs.  The four partial sums of a row meet
-// once, at the end, in shared memory.
+// key tile i+1 while the compute warps take the exponentials of tile i.  Sixteen compute warps (0-15; thread t of every group of four
+// warps = TMEM lane t % 128 = query row) in two teams of eight, each on the tiles of one buffer, 64 key columns a thread: four
+// compute warps on every scheduler, enough to keep the MUFU pipe fed while others wait for TMEM or an mbarrier.  Warp 16 issues
+// TMA loads, warp 17 the MMAs.  The four partial sums of a row (tile parity x column half) meet once, at the end, in shared memory.
 #include "dm_common.cuh"
 #include "dm_kernels.h"
 #include "dm_quant_block.cuh"
@@ -31,7 +30,7 @@ struct DeltaCfg {
   static constexpr int kSmemDo = kTileBytes;
   static constexpr int kSmemK = 2 * kTileBytes;
   static constexpr int kSmemV = kSmemK + kStages * kTileBytes;
-  static constexpr int kGroups = 4;                                     // compute groups, 32 key columns each
+  static constexpr int kGroups = 4;                                     // of four compute warps: two teams x two column halves
   static constexpr int kThreads = kGroups * 128 + 64;
   static constexpr int kSmemRed = kSmemV + kStages * kTileBytes;        // 3 slots x 3 groups x 128 rows x (num, den) doubles
   static constexpr int kSmemBar = kSmemRed + 3 * 3 * 128 * 16;
@@ -50,8 +49,11 @@ __device__ __forceinline__ void delta_item(int item, int n_qt, int bh_count, int
 
 // kQuant: the CTA has one item and quantises its dO tile itself (codes and scales also go to where the kernels behind expect them),
 // which takes the place of a launch of the dO producer: with at most as many items as SMs, where a step is bound by its launches.  The
-// codes come back by TMA, while the first key tiles land.  Training step in us: 69.3 -> 67.5 (N=256 H=2), 87.6 -> 85.3 (N=1024 H=8), 88.8 -> 87.9
-// (B=2 N=1024 H=16: 256 items, two launches as before, within the spread), 91.4 -> 91.1 (head_dim 256, N=1920 H=6).
+// codes come back by TMA, while the first key tiles land.  Training step in us, two launches -> one, in turn: in a run of calls 78.5 -> 75.3
+// (N=256 H=2), 76.0 -> 73.0 (N=512 H=4), 87.2 -> 84.0 (N=1024 H=8 Hk=2), 102.4 -> 101.5 (N=2048 H=8 Hk=2), 185.8 -> 184.8 (N=4096 H=4 Hk=1); at
+// head_dim 256 84.0 -> 80.7 (N=256 H=2), 79.1 -> 76.9 (N=1024 H=8 Hk=4), 78.6 -> 75.4 (B=2 N=512 H=8), 88.1 -> 86.6 (N=1920 H=6 Hk=2).  Under graph
+// replay, where a launch is cheaper, 0 to 3 us.  With long items the two are equal
+// (N=18944 H=1: 626 -> 630, replayed 617 -> 615).
 template <int D, bool kQuant>
 __global__ void __launch_bounds__(DeltaCfg<D>::kThreads, 1)
 delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
