@@ -108,7 +108,7 @@ __device__ __forceinline__ bool wait_or_abort(Bar bar, uint32_t parity, volatile
 // tcgen05.st that follow are never executed by a part of the warp.
 template <typename Bar>
 __device__ __forceinline__ bool wait_warp(Bar bar, uint32_t parity, volatile int* abort_flag) {
-  if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity) ? 1 : 0) != 0) return true;   // ~80 cycles when complete
+  if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity) ? 1 : 0) != 0) return true;   // 67 - 71 cycles when complete
   return __all_sync(0xffffffffu, poll_or_abort(bar, parity, abort_flag) ? 1 : 0) != 0;
 }
 // The status word may live in pinned host memory that the GPU writes directly (the host then sees a give-up without a

@@ -31,7 +31,9 @@ struct FwdCfg {
   // columns each (S 0-127, O 128-255) and take turns instead.
   static constexpr bool kDoubleS = (D == 256);
   // ... and two warps share a row (warps 6-9 take the upper 64 keys of the rows of warps 0-3): with one warp per scheduler nothing runs
-  // under the latencies of its chain.  590 -> 579 us (B=2 N=8192 H=16); what bounds it then is the chain S -> PV -> its
+  // under the latencies of its chain.  One -> two warps: 2348 -> 2209 cycles a tile, with an instruction issued in 37 -> 46 % of
+  // them; us at B=2 N=8192 H=16 causal 598 -> 588 in a burst and 691 -> 650 in a run of calls at the power limit, B=4 N=2048 H=16 97.5 -> 90.6,
+  // N=4096 H=16 80.2 -> 75.5, N=1920 H=6 bidirectional 35.1 -> 33.5, N=1024 H=8 equal.  What bounds it then is the chain S -> PV -> its
   // completion -> next S into the same buffer (PV as four MMAs of N = 256 instead of eight of 128: equal).
   static constexpr int kRowWarps = (D == 256) ? 2 : 1;
   static constexpr int kChunks = 4 / kRowWarps;        // 32-key chunks per thread and tile
