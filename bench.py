@@ -49,10 +49,10 @@ WORKLOADS = {
 FP8_NOMINAL_TFLOPS = 4500.0
 SEED = 1234
 # DRAM bytes (read + written) per live 128 x 128 tile position of the dK/dV kernel: one ncu capture of one launch at B=2 N=4096
-# H=32 Hk=8 D=128 (dram__bytes_read.sum 170.9 MB + dram__bytes_write.sum 535.3 MB over 33792 tile positions; the summary is in
+# H=32 Hk=8 D=128 (dram__bytes_read.sum 173.2 MB + dram__bytes_write.sum 535.4 MB over 33792 tile positions; the summary is in
 # profiles/), scaled to a launch by its tile count (per position one 16 KiB dS tile is written for pass 2, and the Q / dO / K / V
 # tiles are read mostly from L2).
-DKDV_DRAM_BYTES_PER_TILE = 20898.0
+DKDV_DRAM_BYTES_PER_TILE = 20969.0
 
 
 def counted_flops(B, N, H, D, causal=True):
