@@ -467,9 +467,27 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 }
 
 
+// Head_dim 128: which calls the three teams of dm_fwd_teams.cu take (the same bits).  A single query tile takes them 0.6 of the time it takes here, and
+// a CTA per SM ends a call with shorter remainders than two; the change from one item to the next costs them more, which many short
+// items show.  Items are n_t = N / 128 query tiles of every head; us, two CTAs -> teams, H = 1, by items per SM.
+// Up to 1: causal 7.9 -> 8.4 (n_t 2), 10.5 -> 9.7 (4), 15.8 -> 12.5 (8), 26.6 -> 18.6 (16), 48.5 -> 31.2 (32), 91.6 -> 54.5 (64); bidirectional alike.
+// Up to 2, causal: 1.5 11.5 -> 10.9, 2 12.0 -> 12.5 (4); 15.3 -> 15.1 (6), 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32); bidirectional: 12.2 ->
+// 13.8 (4), 18.8 -> 20.2 (8), 32.5 -> 32.7 (16), 46.1 -> 44.9 (24), 59.3 -> 56.9 (32).
+// More, causal, at 3, 6 and 14: 20.4 -> 23.5, 36.9 -> 40.9, 82.5 -> 87.2 (8); 31.1 -> 33.3, 59.1 -> 60.6, 130.8 -> 132.4 (16); 43.7 -> 43.1, 80.2 -> 77.9, 175.7 -> 172.8
+// but 60.2 -> 62.0 at 4.5 (24); 55.6 -> 54.2, 102.2 -> 98.2, 75.5 -> 76.4 at 4.5 (32); 104.7 -> 95.0, 187.5 -> 172.3 (64).  Bidirectional: 19.9 -> 18.7, 30.9 -> 33.2,
+// 70.3 -> 72.5 (4); 25.8 -> 23.6, 41.7 -> 42.5, 94.5 -> 92.9 (6); 34.3 -> 35.1, 51.7 -> 51.7, 118.8 -> 113.2 (8); 60.1 -> 59.7, 114 -> 101.7, 234.5 -> 211.1 (16).
+static bool teams(const FwdParams& p) {
+  const long long n_t = p.N / 128, items = n_t * p.B * p.H, sms = sm_count();
+  if (items <= sms) return n_t >= 4;
+  const bool few = items <= 2 * sms;
+  return n_t >= (p.causal ? (few ? 6 : 32) : (few ? 24 : 6));
+}
+
 cudaError_t launch_fwd(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                        cudaStream_t stream) {
-  // One kernel for both head dims: S (128 columns) plus O (head_dim columns) per CTA, two CTAs per SM at head_dim 128.
+  // One kernel for both head dims: S (128 columns) plus O (head_dim columns) per CTA, two CTAs per SM at head_dim 128, where
+  // dm_fwd_teams.cu takes over for long chains and small grids.
+  if (D == 128 && teams(p)) return launch_fwd_teams(tq, tk, tv, p, stream);
   if (p.unordered) {
     if (D != 128) return launch_fwd_t<256, false>(tq, tk, tv, p, stream);
     return launch_fwd_t<128, false>(tq, tk, tv, p, stream);
