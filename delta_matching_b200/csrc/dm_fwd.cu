@@ -468,19 +468,21 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 
 
 // Head_dim 128: which calls the three teams of dm_fwd_teams.cu take (the same bits).  A single query tile takes them 0.6 of the time it takes here, and
-// a CTA per SM ends a call with shorter remainders than two; the change from one item to the next costs them more, which many short
-// items show.  Items are n_t = N / 128 query tiles of every head; us, two CTAs -> teams, H = 1, by items per SM.
-// Up to 1: causal 7.9 -> 8.4 (n_t 2), 10.5 -> 9.7 (4), 15.8 -> 12.5 (8), 26.6 -> 18.6 (16), 48.5 -> 31.2 (32), 91.6 -> 54.5 (64); bidirectional alike.
-// Up to 2, causal: 1.5 11.5 -> 10.9, 2 12.0 -> 12.5 (4); 15.3 -> 15.1 (6), 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32); bidirectional: 12.2 ->
-// 13.8 (4), 18.8 -> 20.2 (8), 32.5 -> 32.7 (16), 46.1 -> 44.9 (24), 59.3 -> 56.9 (32).
-// More, causal, at 3, 6 and 14: 20.4 -> 23.5, 36.9 -> 40.9, 82.5 -> 87.2 (8); 31.1 -> 33.3, 59.1 -> 60.6, 130.8 -> 132.4 (16); 43.7 -> 43.1, 80.2 -> 77.9, 175.7 -> 172.8
-// but 60.2 -> 62.0 at 4.5 (24); 55.6 -> 54.2, 102.2 -> 98.2, 75.5 -> 76.4 at 4.5 (32); 104.7 -> 95.0, 187.5 -> 172.3 (64).  Bidirectional: 19.9 -> 18.7, 30.9 -> 33.2,
-// 70.3 -> 72.5 (4); 25.8 -> 23.6, 41.7 -> 42.5, 94.5 -> 92.9 (6); 34.3 -> 35.1, 51.7 -> 51.7, 118.8 -> 113.2 (8); 60.1 -> 59.7, 114 -> 101.7, 234.5 -> 211.1 (16).
+// one CTA per SM ends a call with a shorter remainder than two; the change from one item to the next costs them more, which many short items
+// show, and they execute 14 % more instructions, which counts at the power limit.  Items are n_t = N / 128 query tiles of every head; us, two CTAs ->
+// teams, H = 1, at the items per SM named, single calls.
+// Causal.  1: 7.9 -> 8.4 (n_t 2), 10.5 -> 9.7 (4), 15.8 -> 12.5 (8), 26.6 -> 18.6 (16), 48.5 -> 31.2 (32), 91.6 -> 54.5 (64).  2: 12.0 -> 12.5 (4), 15.3 -> 15.1 (6),
+// 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32).  2.5: 25.0 -> 25.4 (12), 31.2 -> 29.5 (16), 43.9 -> 37.1 (24), 105.8 -> 84.1 (64).  3 and 6: 31.1 -> 33.3, 59.1 -> 60.6
+// (16); 55.6 -> 54.2, 102.2 -> 98.2 (32); 104.7 -> 95.0, 187.5 -> 172.3 (64).  In a run of calls 7 (N=4096 H=32 Hk=8: the step 452 -> 458) and 28
+// (B=4: 529 -> 539) items of 32 tiles lose.
+// Bidirectional, where all items are equally long: rounds of items count.  2.16 (3 rounds of single items, or 4) 200 -> 154 (64); 2.5 14.3 -> 12.7 (2), 31.7 -> 28.0 (8),
+// 56.1 -> 46.6 (16); 4.5 29.3 -> 28.1 (4), 39.8 -> 36.0 (6), 88.8 -> 74.4 (16); 14.03 181 -> 164 (12).  As many rounds: 1.5 12.3 -> 13.7 (4), 19.0 -> 20.1 (8), 32.5 -> 32.7
+// (16); 6 30.9 -> 33.2 (4), 51.7 -> 51.7 (8), 131.4 -> 124.9 (24); 13.8 (B=8 N=2048 H=16) 214 -> 200, in a run of calls the step 973 -> 965.
 static bool teams(const FwdParams& p) {
   const long long n_t = p.N / 128, items = n_t * p.B * p.H, sms = sm_count();
-  if (items <= sms) return n_t >= 4;
-  const bool few = items <= 2 * sms;
-  return n_t >= (p.causal ? (few ? 6 : 32) : (few ? 24 : 6));
+  if (p.causal) return items <= sms ? n_t >= 4 : items <= 2 * sms ? n_t >= 6 : 2 * items <= 5 * sms ? n_t >= 16 : items <= 8 * sms && n_t >= 64;
+  const long long single = (items + sms - 1) / sms, paired = 2 * ((items + 2 * sms - 1) / (2 * sms));
+  return single < paired || (single >= 8 && n_t >= 16);
 }
 
 cudaError_t launch_fwd(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
