@@ -10,9 +10,10 @@
 //
 // With many items the exponentials of a call bound neither this nor the two CTAs per SM of dm_fwd.cu: 450 us at B=4 N=4096 H=32 Hk=8 causal become
 // 378 without any exponential and 279 without three quarters of the softmax; MUFU 55 %, issue slots 55 %.  What the teams gain there
-// is the end of a call.  us, before -> now: B=8 N=2048 H=16 bidirectional 214 -> 200, N=16384 H=16 Hk=2 causal 753 -> 720, B=4 N=4096 H=32 Hk=8
-// 426 -> 421, N=1024 H=8 Hk=2 16.4 -> 12.8 (dm_fwd.cu says which calls come here).
-// Slower: K and V by a producer warp each (441 -> 448), a staging row for each team instead of Q and four stages (200 -> 216).
+// is the end of a call.  us, two CTAs per SM -> teams, single calls: N=1024 H=8 Hk=2 causal 16.4 -> 12.8, N=4096 H=9 56.5 -> 34.9, N=8192 H=6 105.8 -> 84.1;
+// bidirectional N=2048 H=42 88.8 -> 74.4, B=8 N=2048 H=16 214 -> 200 (dm_fwd.cu says which calls come here, and what the others would take).
+// Slower: K and V by a producer warp each (441 -> 448 at B=4 N=4096 H=32), a staging row for each team in the place of a second Q tile and the fourth
+// stages (200 -> 216 at B=8 N=2048 H=16).
 #include <type_traits>
 #include <cuda_bf16.h>
 #include "dm_common.cuh"
