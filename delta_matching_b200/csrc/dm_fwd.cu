@@ -469,7 +469,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 
 // Head_dim 128: which calls the three teams of dm_fwd_teams.cu take (the same bits).  A single query tile takes them 0.6 of the time it takes here, and
 // one CTA per SM ends a call with a shorter remainder than two; the change from one item to the next costs them more, which many short items
-// show, and they execute 14 % more instructions, which counts at the power limit.  Items are n_t = N / 128 query tiles of every head; us, two CTAs ->
+// show, and they execute 12 % more instructions, which counts at the power limit.  Items are n_t = N / 128 query tiles of every head; us, two CTAs ->
 // teams, H = 1, at the items per SM named, single calls.
 // Causal.  1: 7.9 -> 8.4 (n_t 2), 10.5 -> 9.7 (4), 15.8 -> 12.5 (8), 26.6 -> 18.6 (16), 48.5 -> 31.2 (32), 91.6 -> 54.5 (64).  2: 12.0 -> 12.5 (4), 15.3 -> 15.1 (6),
 // 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32).  2.5: 25.0 -> 25.4 (12), 31.2 -> 29.5 (16), 43.9 -> 37.1 (24), 105.8 -> 84.1 (64).  3 and 6: 31.1 -> 33.3, 59.1 -> 60.6
