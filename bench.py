@@ -354,7 +354,8 @@ def kernel_breakdown(job, steps, first_units=None):
     parts = {
         "producers_qkv": lambda: ops.quant_qkv(qh, kh, vh),
         "forward": lambda: ops.fwd_fp8(q8, k8, v8, qs, ks, vs, causal),
-        # the same kernel without the wait that orders S(i + 1) behind the scale-word reads of PV(i): what the ordering costs
+        # two CTAs per SM without the wait that orders S(i + 1) behind the scale-word reads of PV(i): what the ordering costs where
+        # `forward` is that kernel too (causal calls of many tiles; head_dim 256)
         "forward_unordered_hook": lambda: ops.fwd_fp8(q8, k8, v8, qs, ks, vs, causal, unordered=True),
         "producer_do": (lambda: ops.quant_do(doh, None)) if matched else (lambda: ops.quant_do(doh, o.permute(0, 2, 1, 3))),
         "bwd_dkdv": lambda: ops.bwd_fp8(q8, k8, v8, do8, qs, ks, vs, dos, lse, delta, causal, parts=1, workspace=ws),

@@ -479,6 +479,15 @@ int dm_dbg_fwd_unordered(const void* q8, const void* k8, const void* v8, const f
   return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream, 1);
 }
 
+int dm_dbg_fwd_kernel(int B, int N, int H, int Hk, int D, int causal, int unordered) {
+  DM_TRY(check_shape(B, N, H, Hk, D));
+  dm::FwdParams p{};
+  p.B = B; p.H = H; p.Hk = Hk; p.N = N;
+  p.causal = causal ? 1 : 0;
+  p.unordered = unordered ? 1 : 0;
+  return dm::fwd_takes_teams(D, p) ? 1 : 0;
+}
+
 static int delta_impl(const void* q8, const void* k8, const void* v8, const void* do8,
                       const float* qs, const float* ks, const float* vs, const float* dos, const float* lse,
                       int B, int N, int H, int Hk, int D, int causal, float* delta, int* status, void* stream, int norm) {

@@ -51,11 +51,10 @@ struct FwdTeamsCfg {
 // Persistent: the grid is the SM count; CTA j processes the work items sched_item(0, j), sched_item(1, j), ... of a list ordered by
 // decreasing number of key tiles (item -> query tile n_qt - 1 - item / (B H), head item % (B H)).  The CTA's tiles are counted through
 // all its items; tile g belongs to team g % 3 and its S accumulator, as number g / 3 of every barrier of that team.
-// kOrdered: S of tile g + 3 waits for the completion of the PV chain of tile g.  It overwrites the TMEM columns from which that chain reads
-// its scale-factor words; the PTX ISA orders a later MMA's accumulator writes behind an earlier MMA's operand reads, but does not say so for
-// scale-factor reads (the reference met the same question and answers it with a commit and a wait,
-// delta_matching/sm100/dm_fwd_sm100.py:636-645).  kOrdered = false issues it behind the issue of that chain and relies on issue order.
-template <bool kOrdered>
+// S of tile g + 3 waits for the completion of the PV chain of tile g.  It overwrites the TMEM columns from which that chain reads its codes and
+// scale-factor words, and two threads issue the two: nothing but completion orders them (dm_fwd.cu's kOrdered asks what issue order gives within
+// one thread).  The softmax warps' parity waits for a PV chain rest on the same wait: with S of a tile landed, the PV chain before it in that
+// accumulator is complete, so a barrier of PV chains is never more than one phase away from the one that is tested.
 __global__ void __launch_bounds__(FwdTeamsCfg::kThreads, 1)
 fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -70,8 +69,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint64_t* bar_s = bars + 0;                // [T] S accumulator ready (MMA commit)
   uint64_t* bar_p = bar_s + T;               // [T] P codes + scale words written (one arrival per softmax warp)
   uint64_t* bar_o = bar_p + T;               // [T] PV chain done (MMA commit)
-  uint64_t* bar_i = bar_o + T;               // [T] PV chain issued (kOrdered = false)
-  uint64_t* bar_ml = bar_i + T;              // [T][4] running maximum and sum of a row quarter behind the tile are written
+  uint64_t* bar_ml = bar_o + T;              // [T][4] running maximum and sum of a row quarter behind the tile are written
   uint64_t* full_k = bar_ml + 4 * T;         // [kStages]
   uint64_t* full_v = full_k + C::kStages;    // [kStages] V and the scales
   uint64_t* empty_k = full_v + C::kStages;   // [kStages] K stage free again (MMA commit behind the S chain)
@@ -82,7 +80,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint64_t* bar_out = bar_ofree + 1;         // ... and has left its rows in shared memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_out + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_out + 2);
-  static_assert((8 * T + 4 * C::kStages + 8) * 8 <= 512, "barrier block");
+  static_assert((7 * T + 4 * C::kStages + 8) * 8 <= 512, "barrier block");
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // a warp-uniform value, also to the compiler
@@ -93,7 +91,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int first_item = static_cast<int>(blockIdx.x), item_step = static_cast<int>(gridDim.x);
 
   if (tid == 0) {
-    for (int s = 0; s < 8 * T + 4 * C::kStages + 6; ++s) mbar_init(bars + s, (bars + s >= bar_p && bars + s < bar_o) || bars + s >= bar_ofree ? 4 : 1);
+    for (int s = 0; s < 7 * T + 4 * C::kStages + 6; ++s) mbar_init(bars + s, (bars + s >= bar_p && bars + s < bar_o) || bars + s >= bar_ofree ? 4 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -162,7 +160,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (!pv) {
               // S = Q K^T: both operands K-major, k-step of 32 bytes inside the 128-byte swizzle row
               if (!(ok = wait_or_abort(full_k + st, st_ph, abort_flag))) break;
-              if (again && !(ok = wait_or_abort((kOrdered ? bar_o : bar_i) + team, ph ^ 1, abort_flag))) break;
+              if (again && !(ok = wait_or_abort(bar_o + team, ph ^ 1, abort_flag))) break;
               tc_fence_after();
               const uint32_t k_lo = k_lo0 + st * (C::kTileBytes >> 4);
 #pragma unroll
@@ -184,7 +182,6 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             s_col + C::kColSfb, (it > 0) || (ks > 0));
               tc_commit(bar_o + team);
               tc_commit(empty_v + st);
-              if (!kOrdered) mbar_arrive(bar_i + team);
             }
             if (++st == C::kStages) {
               st = 0;
@@ -379,8 +376,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp == C::kSoftmaxWarps) tmem_dealloc(tmem, C::kTmemCols);
 }
 
-template <bool kOrdered>
-static cudaError_t launch_teams_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
+cudaError_t launch_fwd_teams(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
   using C = FwdTeamsCfg;
   static bool done[64] = {};
   int dev = 0;
@@ -388,20 +384,16 @@ static cudaError_t launch_teams_t(const CUtensorMap& tq, const CUtensorMap& tk, 
   if (dev >= 0 && dev < 64 && !done[dev]) {
     // the register split draws on what the launch has: with fewer the softmax warps would wait for ever
     cudaFuncAttributes attr;
-    cudaError_t e = cudaFuncGetAttributes(&attr, fwd_teams_kernel<kOrdered>);
+    cudaError_t e = cudaFuncGetAttributes(&attr, fwd_teams_kernel);
     if (e != cudaSuccess) return e;
     if (attr.numRegs * C::kThreads < C::kSoftmaxWarps * 32 * C::kRegsSoftmax + 128 * C::kRegsIssue) return cudaErrorLaunchOutOfResources;
-    e = cudaFuncSetAttribute(fwd_teams_kernel<kOrdered>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    e = cudaFuncSetAttribute(fwd_teams_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     done[dev] = true;
   }
   const int items = p.B * p.H * (p.N / 128), sms = sm_count();
   count_launch();
-  return launch_chained(fwd_teams_kernel<kOrdered>, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, p);
-}
-
-cudaError_t launch_fwd_teams(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
-  return (p.unordered ? launch_teams_t<false> : launch_teams_t<true>)(tq, tk, tv, p, stream);
+  return launch_chained(fwd_teams_kernel, items < sms ? items : sms, C::kThreads, C::kSmemBytes, stream, tq, tk, tv, p);
 }
 
 }  // namespace dm

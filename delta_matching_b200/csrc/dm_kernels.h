@@ -106,6 +106,8 @@ int sm_count();
 void count_launch(int n = 1);
 long long launch_count();
 
+// Whether launch_fwd takes the three teams of dm_fwd_teams.cu.
+bool fwd_takes_teams(int D, const FwdParams& p);
 cudaError_t launch_fwd_teams(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream);
 cudaError_t launch_fwd(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                        cudaStream_t stream);

@@ -221,7 +221,8 @@ def _check_codes(B, H, Hk, N, D, q8, k8, v8, qs, ks, vs, do8=None, dos=None):
 
 def fwd_fp8(q8, k8, v8, qs, ks, vs, causal: bool, unordered: bool = False):
     """-> (O (B, N, H, D) bf16 contiguous, LSE (B, H, N) fp32 natural log).  Replaces the fwd_fp8 op.  unordered=True is
-    the test hook dm_dbg_fwd_unordered (same results, one ordering wait per key tile fewer)."""
+    the test hook dm_dbg_fwd_unordered (same results; at head_dim 128 always the two CTAs per SM, one ordering wait per key tile
+    fewer)."""
     dev = _cuda(q8, k8, v8, qs, ks, vs)
     _enter(dev)
     _require(q8.dim() == 4 and k8.dim() == 4, "codes must be 4-D")

@@ -87,10 +87,15 @@ int dm_fwd(const void* q8, const void* k8, const void* v8, const float* qs, cons
  * commit-and-wait that dm_fwd puts between them (the next S overwrites the TMEM columns the PV chain reads its scale
  * words from; the reference documents the hazard and orders the two, delta_matching/sm100/dm_fwd_sm100.py:636-645).
  * Test hook: the unit tests demand bitwise equal O and LSE from both forms and the benchmark reports what the ordering
- * costs.  Not a production entry point. */
+ * costs.  It is the kernel of one thread issuing both chains whatever the shape: at head_dim 128 the two CTAs per SM, also where
+ * dm_fwd takes the three teams.  Not a production entry point. */
 int dm_dbg_fwd_unordered(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
                          int B, int N, int H, int Hk, int D, int causal,
                          void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream);
+
+/* Which kernel dm_fwd (unordered = 0) or dm_dbg_fwd_unordered (unordered = 1) launches for a shape on the current device (148 SMs without
+ * one): 1 = head_dim 128 in three teams, 0 = the kernel beside it, negative = the shape is refused.  Host only. */
+int dm_dbg_fwd_kernel(int B, int N, int H, int Hk, int D, int causal, int unordered);
 
 /* Matched delta (pass 0): delta_i = sum_j P_ij dP_ij / sum_j P_ij from the backward's own P / dP recompute.
  * Replaces the delta_fp8 op (csrc/delta_matching_api.cpp:470-609). */

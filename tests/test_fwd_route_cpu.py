@@ -1,0 +1,26 @@
+"""Which of the two forwards of head_dim 128 a shape takes (host only: B200's 148 SMs, which the library also assumes without a GPU)."""
+import pytest
+
+# (B, N, H, Hk, D, causal), whether dm_fwd takes the three teams
+CALLS = [((1, 1024, 8, 2, 128, True), True), ((1, 4096, 9, 9, 128, True), True), ((1, 8192, 6, 1, 128, True), True),
+         ((8, 2048, 16, 16, 128, False), True), ((4, 4096, 32, 8, 128, True), False), ((1, 2048, 6, 2, 256, True), False)]
+
+
+def _route(shape, unordered=0):
+    from delta_matching_b200 import _lib
+    return _lib.lib().dm_dbg_fwd_kernel(*(int(x) for x in shape), unordered)
+
+
+@pytest.mark.parametrize("shape,teams", CALLS)
+def test_route(shape, teams):
+    assert _route(shape) == int(teams)
+
+
+@pytest.mark.parametrize("shape", [c[0] for c in CALLS])
+def test_the_form_without_the_ordering_wait_never_takes_the_teams(shape):
+    """Two threads issue the teams' S and PV chains: there is no issue order between them to rely on."""
+    assert _route(shape, unordered=1) == 0
+
+
+def test_route_of_a_refused_shape():
+    assert _route((1, 100, 1, 1, 128, True)) < 0
