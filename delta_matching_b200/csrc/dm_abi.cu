@@ -288,7 +288,7 @@ int dm_attn_fwd(const void* q, int64_t q_sb, int64_t q_sh, int64_t q_sn,
   DM_TRY(make_code_map(&tk, k8, static_cast<uint64_t>(B) * Hk * N, D));
   DM_TRY(make_code_map(&tv, v8, static_cast<uint64_t>(B) * Hk * N, D));
   const dm::FwdParams p{qs, ks, vs, static_cast<__nv_bfloat16*>(o), static_cast<int64_t>(N) * H * D, static_cast<int64_t>(H) * D, D,
-                        lse, B, H, Hk, N, causal ? 1 : 0, status, 0};
+                        lse, B, H, Hk, N, causal ? 1 : 0, status, dm::kFwdByRule};
   e = dm::launch_fwd(D, tq, tk, tv, p, st);
   return e == cudaSuccess ? 0 : cuda_fail(e, "forward launch");
 }
@@ -450,7 +450,7 @@ int dm_attn_bwd(const void* d_o, int64_t do_sb, int64_t do_sh, int64_t do_sn, co
 static int fwd_impl(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
                     int B, int N, int H, int Hk, int D, int causal,
                     void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream,
-                    int unordered) {
+                    int form) {
   DM_TRY(check_shape(B, N, H, Hk, D));
   DM_TRY(check_sm100());
   DM_TRY(check_device_ptr(q8, "q8")); DM_TRY(check_device_ptr(k8, "k8")); DM_TRY(check_device_ptr(v8, "v8"));
@@ -461,8 +461,7 @@ static int fwd_impl(const void* q8, const void* k8, const void* v8, const float*
   DM_TRY(make_code_map(&tq, q8, static_cast<uint64_t>(B) * H * N, D));
   DM_TRY(make_code_map(&tk, k8, static_cast<uint64_t>(B) * Hk * N, D));
   DM_TRY(make_code_map(&tv, v8, static_cast<uint64_t>(B) * Hk * N, D));
-  dm::FwdParams p{qs, ks, vs, static_cast<__nv_bfloat16*>(o), o_sb, o_sn, o_sh, lse, B, H, Hk, N, causal ? 1 : 0, status,
-                  unordered};
+  dm::FwdParams p{qs, ks, vs, static_cast<__nv_bfloat16*>(o), o_sb, o_sn, o_sh, lse, B, H, Hk, N, causal ? 1 : 0, status, form};
   cudaError_t e = dm::launch_fwd(D, tq, tk, tv, p, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? 0 : cuda_fail(e, "forward launch");
 }
@@ -470,13 +469,21 @@ static int fwd_impl(const void* q8, const void* k8, const void* v8, const float*
 int dm_fwd(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
            int B, int N, int H, int Hk, int D, int causal,
            void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream) {
-  return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream, 0);
+  return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream, dm::kFwdByRule);
 }
 
 int dm_dbg_fwd_unordered(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
                          int B, int N, int H, int Hk, int D, int causal,
                          void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream) {
-  return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream, 1);
+  return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream, dm::kFwdUnordered);
+}
+
+int dm_dbg_fwd_forced(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
+                      int B, int N, int H, int Hk, int D, int causal,
+                      void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream, int kernel) {
+  if (kernel != 0 && !(kernel == 1 && D == 128)) return fail(DM_ERR_ARG, "delta_matching: no forward kernel %d at head_dim %d", kernel, D);
+  return fwd_impl(q8, k8, v8, qs, ks, vs, B, N, H, Hk, D, causal, o, o_sb, o_sn, o_sh, lse, status, stream,
+                  kernel == 1 ? dm::kFwdTeams : dm::kFwdPairs);
 }
 
 int dm_dbg_fwd_kernel(int B, int N, int H, int Hk, int D, int causal, int unordered) {
@@ -484,7 +491,7 @@ int dm_dbg_fwd_kernel(int B, int N, int H, int Hk, int D, int causal, int unorde
   dm::FwdParams p{};
   p.B = B; p.H = H; p.Hk = Hk; p.N = N;
   p.causal = causal ? 1 : 0;
-  p.unordered = unordered ? 1 : 0;
+  p.form = unordered ? dm::kFwdUnordered : dm::kFwdByRule;
   return dm::fwd_takes_teams(D, p) ? 1 : 0;
 }
 

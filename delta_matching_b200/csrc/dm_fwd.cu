@@ -485,15 +485,15 @@ static bool teams(const FwdParams& p) {
   return single < paired || (single >= 8 && n_t >= 16);
 }
 
-// The form without the ordering wait exists where one thread issues S and PV, so in the kernel of this file alone.
-bool fwd_takes_teams(int D, const FwdParams& p) { return D == 128 && !p.unordered && teams(p); }
+bool fwd_takes_teams(int D, const FwdParams& p) { return D == 128 && (p.form == kFwdTeams || (p.form == kFwdByRule && teams(p))); }
 
 cudaError_t launch_fwd(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                        cudaStream_t stream) {
   // One kernel for both head dims: S (128 columns) plus O (head_dim columns) per CTA, two CTAs per SM at head_dim 128, where
-  // dm_fwd_teams.cu takes over for long chains and small grids.
+  // dm_fwd_teams.cu takes over for long chains and small grids.  The form without the ordering wait exists here alone, where one thread issues
+  // both chains.
   if (fwd_takes_teams(D, p)) return launch_fwd_teams(tq, tk, tv, p, stream);
-  if (p.unordered) {
+  if (p.form == kFwdUnordered) {
     if (D != 128) return launch_fwd_t<256, false>(tq, tk, tv, p, stream);
     return launch_fwd_t<128, false>(tq, tk, tv, p, stream);
   }

@@ -8,6 +8,14 @@
 namespace dm {
 
 // Codes are e4m3 bytes in (B, H, N, D) order, dense; scales fp32 powers of two in (B, H, N / 32) order.
+// What launch_fwd chooses: the rule of dm_fwd.cu, or (test hooks) what is named.
+enum FwdForm : int {
+  kFwdByRule = 0,
+  kFwdPairs = 1,               // fwd_kernel: two CTAs per SM at head_dim 128
+  kFwdTeams = 2,               // fwd_teams_kernel, head_dim 128
+  kFwdUnordered = 3,           // fwd_kernel, S of the next tile issued without waiting for the PV chain (see its kOrdered)
+};
+
 struct FwdParams {
   const float* qs;
   const float* ks;
@@ -18,7 +26,7 @@ struct FwdParams {
   int B, H, Hk, N;
   int causal;
   int* status;
-  int unordered;               // S of the next tile issued without waiting for the PV chain (see fwd_kernel's kOrdered)
+  int form;                    // FwdForm
 };
 
 struct DeltaParams {

@@ -93,8 +93,14 @@ int dm_dbg_fwd_unordered(const void* q8, const void* k8, const void* v8, const f
                          int B, int N, int H, int Hk, int D, int causal,
                          void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream);
 
+/* dm_fwd on a named kernel: 1 = head_dim 128 in three teams, 0 = two CTAs per SM (at head_dim 256 its only kernel); anything else is
+ * refused.  Test hook: the unit tests demand the same bits of O and LSE from both. */
+int dm_dbg_fwd_forced(const void* q8, const void* k8, const void* v8, const float* qs, const float* ks, const float* vs,
+                      int B, int N, int H, int Hk, int D, int causal,
+                      void* o, int64_t o_sb, int64_t o_sn, int64_t o_sh, float* lse, int* status, void* stream, int kernel);
+
 /* Which kernel dm_fwd (unordered = 0) or dm_dbg_fwd_unordered (unordered = 1) launches for a shape on the current device (148 SMs without
- * one): 1 = head_dim 128 in three teams, 0 = the kernel beside it, negative = the shape is refused.  Host only. */
+ * one): 1 or 0 as in dm_dbg_fwd_forced, negative = the shape is refused.  Host only. */
 int dm_dbg_fwd_kernel(int B, int N, int H, int Hk, int D, int causal, int unordered);
 
 /* Matched delta (pass 0): delta_i = sum_j P_ij dP_ij / sum_j P_ij from the backward's own P / dP recompute.

@@ -24,3 +24,10 @@ def test_the_form_without_the_ordering_wait_never_takes_the_teams(shape):
 
 def test_route_of_a_refused_shape():
     assert _route((1, 100, 1, 1, 128, True)) < 0
+
+
+@pytest.mark.parametrize("D,kernel", [(256, 1), (128, 2), (128, -1)])
+def test_no_such_kernel(D, kernel):
+    from delta_matching_b200 import _lib
+    rc = _lib.lib().dm_dbg_fwd_forced(None, None, None, None, None, None, 1, 256, 1, 1, D, 1, None, 0, 0, 0, None, None, None, kernel)
+    assert rc < 0 and "no forward kernel" in _lib.last_error()
