@@ -56,10 +56,12 @@ def fwd_forced(codes, causal, kernel, o=None):
     """dm_fwd on a named kernel (0: two CTAs per SM, 1: three teams) -> (O, LSE).  codes = (q8, k8, v8, qs, ks, vs); o: a (B, N, H, D)
     view to write to."""
     from delta_matching_b200 import _lib, ops
-    q8, k8 = codes[:2]
+    q8, k8, v8, qs, ks, vs = codes
     B, H, N, D = q8.shape
+    ops._check_codes(B, H, k8.shape[1], N, D, q8, k8, v8, qs, ks, vs)       # the raw entry cannot see sizes
     if o is None:
         o = torch.empty(B, N, H, D, device=q8.device, dtype=torch.bfloat16)
+    assert tuple(o.shape) == (B, N, H, D) and o.dtype == torch.bfloat16 and o.stride(3) == 1
     lse = torch.empty(B, H, N, device=q8.device, dtype=torch.float32)
     _lib.check(_lib.lib().dm_dbg_fwd_forced(*(t.data_ptr() for t in codes), B, N, H, k8.shape[1], D, int(causal), o.data_ptr(),
                                             o.stride(0), o.stride(1), o.stride(2), lse.data_ptr(), ops.status_word(q8.device).data_ptr(),
