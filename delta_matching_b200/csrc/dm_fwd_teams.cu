@@ -103,7 +103,11 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   constexpr uint32_t tmem = 0;                         // 512 columns are all there are: the allocation starts at column 0
-  grid_dep_wait();
+  // The next kernel does not start its set-up under this one.  Its CTAs would come onto each SM straight behind the one here and keep the
+  // division of that SM's 256 KB that 199 KB of shared memory call for, so that the producers of the next call run with the smallest L1 (with a
+  // carve-out of their own they did not).  us, producers and forward in a run, two CTAs per SM -> teams with that start -> without, bidirectional, H = 1:
+  // 14.5 -> 13.7 -> 11.5 (N=256, 71 heads), 64.8 -> 68.4 -> 62.0 (N=768, 122), 236 -> 250 -> 227 (N=512, 775), 507 -> 554 -> 509 (N=768, 1010).
+  grid_dep_wait_alone();
 
   if (warp >= C::kSoftmaxWarps) {
     reg_dec<C::kRegsIssue>();

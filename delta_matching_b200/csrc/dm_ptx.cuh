@@ -31,6 +31,9 @@ __device__ __forceinline__ void grid_dep_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The wait alone: the next kernel starts when this one has ended.
+__device__ __forceinline__ void grid_dep_wait_alone() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------------------------ register split
 // Executed by every warp of a warpgroup.  The pool is what the CTA was launched with (threads x registers a thread at launch): the
 // shares of the warpgroups must not add up to more, or the request waits for ever.
