@@ -475,13 +475,19 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 // 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32).  2.5: 25.0 -> 25.4 (12), 31.2 -> 29.5 (16), 43.9 -> 37.1 (24), 105.8 -> 84.1 (64).  3 and 6: 31.1 -> 33.3, 59.1 -> 60.6
 // (16); 55.6 -> 54.2, 102.2 -> 98.2 (32); 104.7 -> 95.0, 187.5 -> 172.3 (64).  In a run of calls 7 (N=4096 H=32 Hk=8: the step 452 -> 458) and 28
 // (B=4: 529 -> 539) items of 32 tiles lose.
-// Bidirectional, where all items are equally long: rounds of items count.  2.16 (3 rounds of single items, or 4) 200 -> 154 (64); 2.5 14.3 -> 12.7 (2), 31.7 -> 28.0 (8),
-// 56.1 -> 46.6 (16); 4.5 29.3 -> 28.1 (4), 39.8 -> 36.0 (6), 88.8 -> 74.4 (16); 14.03 181 -> 164 (12).  As many rounds: 1.5 12.3 -> 13.7 (4), 19.0 -> 20.1 (8), 32.5 -> 32.7
-// (16); 6 30.9 -> 33.2 (4), 51.7 -> 51.7 (8), 131.4 -> 124.9 (24); 13.8 (B=8 N=2048 H=16) 214 -> 200, in a run of calls the step 973 -> 965.
+// Bidirectional, where all items are equally long: rounds of items count; us for producers and forward in a run of calls.  One round less: 14.4 -> 11.8 (n_t 2,
+// at 0.97 items per SM), 18.1 -> 15.5 (4), 25.2 -> 19.2 (8); 27.3 -> 26.1 (2, 2.99), 37.1 -> 34.6 (4), 49.0 -> 41.8 (8); 46.1 -> 44.6 (2, 4.99), 61.1 -> 57.8 (4), 118 -> 104 (16); 131 -> 119
+// (2, 15), 247 -> 234 (4, 21), 526 -> 517 (6, 41), 627 -> 599 (8, 41).  Single key tiles have no chain to overlap: 7.0 -> 8.1 (at 0.11), 10.0 -> 10.2 (0.59), 12.2 -> 11.0 (0.98, but the
+// forward alone 4.9 -> 6.8), 22.2 -> 23.4 (2.99), 38.8 -> 39.5 (4.99), 52.8 -> 53.1 (6.99); 66.1 -> 64.8 (8.99), 291 -> 266 (41).  Three leave each team one tile of an item and the
+// write-out always to the same one: 15.5 -> 13.2 (0.97), 34.2 -> 33.2 (2.98), 49.5 -> 51.1 (4.2), 56.5 -> 56.7 (4.99), 76.5 -> 76.3 (6.97, the forward alone 32.0 -> 33.4); 95.8 -> 95.4
+// (8.98), 438 -> 419 (41).
+// As many rounds: 15.0 -> 16.5 (2, 1.5), 27.2 -> 28.7 (8), 34.0 -> 35.1 (12); 45.3 -> 46.9 (4, 3.97), 54.8 -> 55.2 (8); 88.6 -> 87.4 (4, 7.97), 96.4 -> 97.2 (6), 111 -> 110 (8), 140.5 -> 137 (12), 176 -> 171 (16, 8),
+// 316 -> 299 (16, 13.95), 740 -> 677 (16, 30).  (Below 16 tiles the teams would gain 1 - 7 % from 14 rounds on: 199 -> 191 (8, 13.95); that is not used.)
 static bool teams(const FwdParams& p) {
   const long long n_t = p.N / 128, items = n_t * p.B * p.H, sms = sm_count();
   if (p.causal) return items <= sms ? n_t >= 4 : items <= 2 * sms ? n_t >= 6 : 2 * items <= 5 * sms ? n_t >= 16 : items <= 8 * sms && n_t >= 64;
   const long long single = (items + sms - 1) / sms, paired = 2 * ((items + 2 * sms - 1) / (2 * sms));
+  if (n_t == 1 || n_t == 3) return single < paired && (single >= 9 || (n_t == 3 && single <= 3));
   return single < paired || (single >= 8 && n_t >= 16);
 }
 

@@ -31,3 +31,10 @@ def test_no_such_kernel(D, kernel):
     from delta_matching_b200 import _lib
     rc = _lib.lib().dm_dbg_fwd_forced(None, None, None, None, None, None, 1, 256, 1, 1, D, 1, None, 0, 0, 0, None, None, None, kernel)
     assert rc < 0 and "no forward kernel" in _lib.last_error()
+
+
+# Bidirectional chains of one and three key tiles, whose few rounds of items measured slower in the teams
+@pytest.mark.parametrize("N,heads,teams", [(128, 16, False), (128, 148, False), (128, 441, False), (128, 1033, False), (128, 1329, True), (384, 49, True),
+                                           (384, 147, True), (384, 207, False), (384, 246, False), (384, 443, True), (256, 71, True), (512, 184, True)])
+def test_route_of_short_bidirectional_chains(N, heads, teams):
+    assert _route((1, N, heads, heads, 128, False)) == int(teams)
