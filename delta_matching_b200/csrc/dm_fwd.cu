@@ -467,15 +467,16 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 }
 
 
-// Head_dim 128: which calls the three teams of dm_fwd_teams.cu take (the same bits).  A single query tile takes them 0.6 of the time it takes here, and
-// one CTA per SM ends a call with a shorter remainder than two; the change from one item to the next costs them more, which many short items
-// show, and they execute 12 % more instructions, which counts at the power limit.  Items are n_t = N / 128 query tiles of every head; us, two CTAs ->
-// teams, H = 1, at the items per SM named, single calls.
-// Causal.  1: 7.9 -> 8.4 (n_t 2), 10.5 -> 9.7 (4), 15.8 -> 12.5 (8), 26.6 -> 18.6 (16), 48.5 -> 31.2 (32), 91.6 -> 54.5 (64).  2: 12.0 -> 12.5 (4), 15.3 -> 15.1 (6),
-// 18.3 -> 16.4 (8), 31.5 -> 23.1 (16), 56.5 -> 34.9 (32).  2.5: 25.0 -> 25.4 (12), 31.2 -> 29.5 (16), 43.9 -> 37.1 (24), 105.8 -> 84.1 (64).  3 and 6: 31.1 -> 33.3, 59.1 -> 60.6
-// (16); 55.6 -> 54.2, 102.2 -> 98.2 (32); 104.7 -> 95.0, 187.5 -> 172.3 (64).  In a run of calls 7 (N=4096 H=32 Hk=8: the step 452 -> 458) and 28
-// (B=4: 529 -> 539) items of 32 tiles lose.
-// Bidirectional, where all items are equally long: rounds of items count; us for producers and forward in a run of calls.  One round less: 14.4 -> 11.8 (n_t 2,
+// Head_dim 128: which calls the three teams of dm_fwd_teams.cu take (the same bits).  A query tile that has its SM to itself takes them 0.6 of the time it takes
+// here from 32 key tiles on, 0.7 at 16, 0.8 at 8 and 0.93 at 4, and one CTA per SM ends a call with a shorter remainder than two; the change from one item to the
+// next costs them more, which many short items show, and they execute 12 % more instructions, which counts at the power limit.  Items are n_t = N / 128
+// query tiles of every head; us, two CTAs -> teams, for producers and forward in a run of calls, at the items per SM named.
+// Causal.  Up to 1: 14.1 -> 13.1 (n_t 2, but the forward alone 7.3 -> 8.4), 16.7 -> 15.9 (4), 22.5 -> 17.7 (6), 24.9 -> 19.9 (8), 31.0 -> 23.0 (12).  Up to 2: 18.6 -> 18.8 (4, 1.59), 20.4 -> 21.8
+// (4, 1.97), 23.2 -> 21.5 (6, 1.46), 23.7 -> 23.6 (6, 1.70), 24.6 -> 25.6 (6, 1.95), 26.1 -> 25.9 (7, 1.89), 27.7 -> 26.9 (8, 1.95), 34.0 -> 30.3 (12, 1.95).  Up to 2.5: 36.3 -> 37.3 (12, 2.43),
+// 39.9 -> 40.1 (14, 2.46), 43.1 -> 41.0 (16, 2.38), 50.1 -> 46.0 (20, 2.43).  More: 45.2 -> 47.9 (16, 2.92), 71.2 -> 74.1 (24, 3.89), 94.5 -> 98.5 (32, 4.32), 134 -> 139 (32, 6.92), 124.4 -> 124.3 (48, 4.22),
+// 200 -> 202 (48, 6.81); 147 -> 144 (64, 3.89), 163.1 -> 162.4 (64, 4.32), 219 -> 207 (64, 5.62), 261.0 -> 260.5 (64, 6.92), 297 -> 290 (128, 4.32).  Beyond 8 the teams gain 1 - 2 % in such runs (310 ->
+// 306 (64, 8.2), 465 -> 457 (64, 13.8), 535 -> 530 (32, 27.7)) and less than the spread in a training step (1731 -> 1725 (32, 27.7)): the two CTAs keep them.
+// Bidirectional, where all items are equally long: rounds of items count.  One round less: 14.4 -> 11.8 (n_t 2,
 // at 0.97 items per SM), 18.1 -> 15.5 (4), 25.2 -> 19.2 (8); 27.3 -> 26.1 (2, 2.99), 37.1 -> 34.6 (4), 49.0 -> 41.8 (8); 46.1 -> 44.6 (2, 4.99), 61.1 -> 57.8 (4), 118 -> 104 (16); 131 -> 119
 // (2, 15), 247 -> 234 (4, 21), 526 -> 517 (6, 41), 627 -> 599 (8, 41).  Single key tiles have no chain to overlap: 7.0 -> 8.1 (at 0.11), 10.0 -> 10.2 (0.59), 12.2 -> 11.0 (0.98, but the
 // forward alone 4.9 -> 6.8), 22.2 -> 23.4 (2.99), 38.8 -> 39.5 (4.99), 52.8 -> 53.1 (6.99); 66.1 -> 64.8 (8.99), 291 -> 266 (41).  Three leave each team one tile of an item and the
@@ -485,7 +486,11 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 // 316 -> 299 (16, 13.95), 740 -> 677 (16, 30).  (Below 16 tiles the teams would gain 1 - 7 % from 14 rounds on: 199 -> 191 (8, 13.95); that is not used.)
 static bool teams(const FwdParams& p) {
   const long long n_t = p.N / 128, items = n_t * p.B * p.H, sms = sm_count();
-  if (p.causal) return items <= sms ? n_t >= 4 : items <= 2 * sms ? n_t >= 6 : 2 * items <= 5 * sms ? n_t >= 16 : items <= 8 * sms && n_t >= 64;
+  if (p.causal) {
+    if (items <= sms) return n_t >= 4;
+    if (items <= 2 * sms) return n_t >= (4 * items <= 7 * sms ? 6 : 7);
+    return 2 * items <= 5 * sms ? n_t >= 16 : items <= 8 * sms && n_t >= 64;
+  }
   const long long single = (items + sms - 1) / sms, paired = 2 * ((items + 2 * sms - 1) / (2 * sms));
   if (n_t == 1 || n_t == 3) return single < paired && (single >= 9 || (n_t == 3 && single <= 3));
   return single < paired || (single >= 8 && n_t >= 16);

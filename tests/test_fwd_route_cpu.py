@@ -38,3 +38,9 @@ def test_no_such_kernel(D, kernel):
                                            (384, 147, True), (384, 207, False), (384, 246, False), (384, 443, True), (256, 71, True), (512, 184, True)])
 def test_route_of_short_bidirectional_chains(N, heads, teams):
     assert _route((1, N, heads, heads, 128, False)) == int(teams)
+
+
+# Causal calls of short chains close to two items per SM: six key tiles measured slower in the teams there, seven did not
+@pytest.mark.parametrize("N,heads,teams", [(768, 36, True), (768, 42, True), (768, 48, False), (768, 49, False), (896, 40, True), (1024, 36, True)])
+def test_route_of_short_causal_chains(N, heads, teams):
+    assert _route((1, N, heads, heads, 128, True)) == int(teams)
