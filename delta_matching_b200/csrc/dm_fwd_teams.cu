@@ -10,7 +10,7 @@
 //
 // With many items the exponentials of a call bound neither this nor the two CTAs per SM of dm_fwd.cu: 450 us at B=4 N=4096 H=32 Hk=8 causal become
 // 378 without any exponential and 279 without three quarters of the softmax; MUFU 55 %, issue slots 55 %.  What the teams gain there
-// is the end of a call.  us, two CTAs per SM -> teams, single calls: N=1024 H=8 Hk=2 causal 16.4 -> 12.8, N=4096 H=9 56.5 -> 34.9, N=8192 H=6 105.8 -> 84.1;
+// is the end of a call.  us, two CTAs per SM -> teams, the forward alone in single calls: N=1024 H=8 Hk=2 causal 16.4 -> 12.8, N=4096 H=9 56.5 -> 34.9, N=8192 H=6 105.8 -> 84.1;
 // bidirectional N=2048 H=42 88.8 -> 74.4, B=8 N=2048 H=16 214 -> 200 (dm_fwd.cu says which calls come here, and what the others would take).
 // Slower: K and V by a producer warp each (441 -> 448 at B=4 N=4096 H=32), a staging row for each team in the place of a second Q tile and the fourth
 // stages (200 -> 216 at B=8 N=2048 H=16).
@@ -105,7 +105,7 @@ fwd_teams_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   constexpr uint32_t tmem = 0;                         // 512 columns are all there are: the allocation starts at column 0
   // The next kernel does not start its set-up under this one.  Its CTAs would come onto each SM straight behind the one here and keep the
   // division of that SM's 256 KB that 199 KB of shared memory call for, so that the producers of the next call run with the smallest L1 (with a
-  // carve-out of their own they did not).  us, producers and forward in a run, two CTAs per SM -> teams with that start -> without, bidirectional, H = 1:
+  // carve-out of their own they did not).  us, producers and forward in a run, two CTAs per SM -> teams with that start -> without, bidirectional:
   // 14.5 -> 13.7 -> 11.5 (N=256, 71 heads), 64.8 -> 68.4 -> 62.0 (N=768, 122), 236 -> 250 -> 227 (N=512, 775), 507 -> 554 -> 509 (N=768, 1010).
   grid_dep_wait_alone();
 
